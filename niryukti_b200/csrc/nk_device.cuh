@@ -65,6 +65,7 @@ struct Control {
     int pending;        // 1 while pending_w must still be applied
     unsigned arrive;    // last-CTA detection in dual_kernel
     int flags;          // bit 0 adaptive, bit 1 halpern, bit 2 residual restarts
+    int fault;          // a CTA of resident_kernel gave up waiting
 };
 
 struct Vecs {
@@ -384,22 +385,25 @@ __global__ void __launch_bounds__(kFusedThreads, kFusedMinBlocks)
 }
 
 // ------------------------------------------------------------------ dual + decide
-__device__ inline void decide(Vecs &v, double p, double d, double c) {
-    Control &s = *v.ctl;
-    const bool adaptive = s.flags & 1, halpern = s.flags & 2, residual_restarts = s.flags & 4;
-    if (s.restart != 0) { // a requested Halpern restart freezes the chunk (src/cuda.cu:298-301)
+// The decision of a trial: energy = p / tau + d / sigma of the trial's steps, c = sum
+// dy * delta, weight = factor / (mass + factor), and (accepted + 2) to the powers
+// -.3 and -.6 (read when adaptive).  HALPERN false leaves that form's code out
+// for a caller that knows its engine is not Halpern's.
+template <bool HALPERN = true>
+__device__ inline void decide(Control &s, double energy, double c, double weight, double pow03,
+                              double pow06) {
+    const bool adaptive = s.flags & 1, halpern = HALPERN && (s.flags & 2),
+               residual_restarts = s.flags & 4;
+    if (HALPERN && s.restart != 0) { // a requested restart freezes the chunk (src/cuda.cu:298-301)
         s.accept = 0;
         return;
     }
     double factor = s.factor;
-    double tau = s.tau * factor, sigma = s.sigma * factor;
-    double energy = p / tau + d / sigma;
     double limit = fabs(c) > 0 ? energy / (2 * fabs(c)) : INFINITY;
     bool finite = isfinite(energy) && isfinite(c);
     bool accept = finite && (!adaptive || limit >= 1);
     if (adaptive) {
-        double k = s.accepted + 2;
-        double mult = fmin((1 - pow(k, -.3)) * limit, 1 + pow(k, -.6));
+        double mult = fmin((1 - pow03) * limit, 1 + pow06);
         if (!finite || !isfinite(mult) || mult <= 0)
             mult = .5;
         s.factor = clampd(factor * mult, 1e-12, 1e12);
@@ -409,7 +413,7 @@ __device__ inline void decide(Vecs &v, double p, double d, double c) {
     if (accept) {
         s.mass += factor;
         s.accepted += 1;
-        s.weight = factor / s.mass;
+        s.weight = weight;
         if (halpern) {
             double residual = sqrt(fmax(0., energy - 2 * c));
             if (s.epoch == 0)
@@ -431,6 +435,25 @@ __device__ inline void decide(Vecs &v, double p, double d, double c) {
         }
     } else
         s.rejected += 1;
+}
+
+// Everything of `s` but the launch state (flags, fault).
+__device__ inline void store_control(Control *ctl, const Control &s) {
+    ctl->factor = s.factor;
+    ctl->mass = s.mass;
+    ctl->accepted = s.accepted;
+    ctl->rejected = s.rejected;
+    ctl->accept = s.accept;
+    ctl->weight = s.weight;
+    ctl->epoch = s.epoch;
+    ctl->init_res = s.init_res;
+    ctl->prev_res = s.prev_res;
+    ctl->restart = s.restart;
+    ctl->lambda = s.lambda;
+    ctl->pending_w = s.pending_w;
+    ctl->cur = s.cur;
+    ctl->pending = s.pending;
+    ctl->arrive = s.arrive;
 }
 
 // PANEL: A's long rows (engine rows [0, v.panel_rows)) come from panel_kernel
@@ -607,7 +630,12 @@ __global__ void __launch_bounds__(kFusedThreads, kFusedMinBlocks)
     double r3[3] = {p, d, c};
     cta_sum<3, kFusedWarps>(r3, red);
     if (threadIdx.x == 0) {
-        decide(v, r3[0], r3[1], r3[2]);
+        Control &s = *v.ctl;
+        const double k = s.accepted + 2;
+        const bool adaptive = s.flags & 1;
+        decide(s, r3[0] / (s.tau * s.factor) + r3[1] / (s.sigma * s.factor), r3[2],
+               s.factor / (s.mass + s.factor), adaptive ? pow(k, -.3) : 0.,
+               adaptive ? pow(k, -.6) : 0.);
         v.ctl->arrive = 0;
     }
 }

@@ -10,6 +10,7 @@
 #include "nk_common.cuh"
 #include "nk_device.cuh"
 #include "nk_panel.cuh"
+#include "nk_resident.cuh"
 #include "nk_host.hpp"
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
@@ -68,6 +69,7 @@ struct SellMatrix {
     std::vector<int32_t> chunk_len; // host: padded length of each chunk
     DevBuf<int64_t> coff, clist;    // the fused kernels' per-CTA chunk lists
     int max_cta_items = 0;          // longest of those lists
+    std::vector<int64_t> hoff, hlist; // the lists on the host (the resident kernel's slots)
 
     // The view the fused trial kernels use: with the per-CTA chunk lists
     // (built for their persistent grid).
@@ -167,6 +169,18 @@ struct PanelMatrix {
         return cptr.bytes() + uoff.bytes() + roff.bytes() + units.bytes() + lidx.bytes() +
                val64.bytes() + partial.bytes() + val32.bytes() + claim.bytes();
     }
+};
+
+// The resident kernel's plan for a model (nk_resident.cuh).
+struct ResidentPlan {
+    bool on = false;
+    int grid = 0;
+    unsigned tag = 1;
+    size_t smem = 0;
+    ResidentView view{};
+    DevBuf<int> lists;   // own_t, own_a, slot_t, slot_a, sync of the view
+    DevBuf<double> work; // sum_p, sum_d, word, last_x, last_y
+    size_t device_bytes() const { return lists.bytes() + work.bytes(); }
 };
 
 // Stable order of items by decreasing length (counting sort): result[k] is the
@@ -448,6 +462,14 @@ template <class Acc, class V, class I> PrimalFn<V, I> primal_kernel_for(bool spa
     return split ? primal_kernel<Acc, V, I, false, F, true> : primal_kernel<Acc, V, I, false, F, false>;
 }
 
+template <class V> const void *resident_kernel_of(bool split, bool halpern) {
+    if (halpern)
+        return split ? (const void *)resident_kernel<V, true, true>
+                     : (const void *)resident_kernel<V, false, true>;
+    return split ? (const void *)resident_kernel<V, true, false>
+                 : (const void *)resident_kernel<V, false, false>;
+}
+
 // ------------------------------------------------------------------ engine
 struct Engine {
     int64_t n = 0, m = 0;
@@ -474,6 +496,7 @@ struct Engine {
     int64_t accepted = 0, rejected = 0, trials = 0;
     int empty_chunks = 0;
     bool request_restart = false;
+    ResidentPlan resident; // small and medium models: whole chunks of trials in one launch
     cudaGraphExec_t graph_exec[8] = {};
     double cscale = 1;
     // engine order: engine column j is the caller's column col_perm[j], engine
@@ -603,6 +626,33 @@ struct Engine {
         }
     }
 
+    // trials of one resident launch (bounds its run time and its barrier count)
+    static constexpr int kResidentTrials = 4096;
+    void launch_resident(int count) {
+        if (precision == NK_PRECISION_FP64)
+            launch_resident_t<double>(count);
+        else
+            launch_resident_t<float>(count);
+    }
+    const void *resident_function() const {
+        const bool split = A.nsv + At.nsv > 0;
+        return precision == NK_PRECISION_FP64 ? resident_kernel_of<double>(split, halpern)
+                                              : resident_kernel_of<float>(split, halpern);
+    }
+    template <class V> void launch_resident_t(int count) {
+        auto at = At.view<V, int32_t>();
+        auto a = A.view<V, int32_t>();
+        Vecs v = vecs();
+        // the decision messages' tags: the next one is never what the words still hold
+        unsigned tag = resident.tag;
+        resident.tag += unsigned(count);
+        void *args[] = {&at, &a, &v, &resident.view, &count, &tag};
+        cuda_check(cudaLaunchCooperativeKernel(resident_function(), dim3(resident.grid),
+                                               dim3(kResThreads), args, resident.smem, stream),
+                   "trial launch");
+    }
+    int vbits() const { return precision == NK_PRECISION_FP64 ? 64 : 32; }
+
     template <class V, class I>
     void spmv_t(const SellMatrix &M, const double *xin, double *out) {
         if (M.nv == 0)
@@ -709,7 +759,10 @@ struct Engine {
             push_ctl();
         }
         int left = count;
-        if (graphs) {
+        if (resident.on) {
+            for (; left > 0; left -= kResidentTrials)
+                launch_resident(std::min(left, kResidentTrials));
+        } else if (graphs) {
             for (int k = 7; k >= 0 && left > 0; --k)
                 while (left >= (1 << k)) {
                     cuda_check(cudaGraphLaunch(graph_for(k), stream), "graph launch");
@@ -722,6 +775,13 @@ struct Engine {
         cuda_check(cudaGetLastError(), "trial launch");
         trials += count;
         sync_ctl();
+        if (host_ctl->fault) {
+            host_ctl->fault = 0;
+            push_ctl();
+            cuda_check(cudaMemsetAsync(resident.view.sync, 0, 2 * sizeof(unsigned), stream),
+                       "trial counters");
+            throw Error(NK_ERR_CUDA, "a wait inside the trial kernel was given up");
+        }
         int64_t now = int64_t(host_ctl->accepted);
         int progress = int(now - accepted);
         accepted = now;
@@ -1099,7 +1159,8 @@ struct Engine {
     }
 
     size_t device_bytes() const {
-        size_t b = A.device_bytes() + At.device_bytes() + Q.device_bytes() + pan.device_bytes();
+        size_t b = A.device_bytes() + At.device_bytes() + Q.device_bytes() + pan.device_bytes() +
+                   resident.device_bytes();
         for (auto *d : {&c, &q, &lb, &ub, &rl, &ru, &x[0], &x[1], &y[0], &y[1], &ax[0], &ax[1],
                         &xa, &ya, &dx, &anchor_x, &anchor_y, &anchor_ax, &part_p, &part_d,
                         &scratch_n, &scratch_m})
@@ -1149,10 +1210,9 @@ std::vector<int64_t> lpt_assign(const std::vector<int64_t> &items, const std::ve
 // The schedule of `ids` (item k is ids[k], with memory work work[k]) onto
 // `ctas` persistent CTAs: longest-first list scheduling by memory work, then
 // each CTA's items costliest first (its warps claim them in that order).
-// Uploads the per-CTA lists (off, list); returns the longest list.
-int schedule_items(const std::vector<int64_t> &ids, const std::vector<int64_t> &work,
-                   int64_t ctas, DevBuf<int64_t> &off_d, DevBuf<int64_t> &list_d,
-                   cudaStream_t s) {
+// Keeps and uploads M's per-CTA lists.
+void schedule_items(const std::vector<int64_t> &ids, const std::vector<int64_t> &work,
+                    int64_t ctas, SellMatrix &M, cudaStream_t s) {
     const int64_t nit = int64_t(ids.size());
     ctas = std::max<int64_t>(1, ctas);
     std::vector<int64_t> all(static_cast<size_t>(nit)), cta(static_cast<size_t>(nit));
@@ -1180,9 +1240,11 @@ int schedule_items(const std::vector<int64_t> &ids, const std::vector<int64_t> &
         if (got != want)
             throw Error(NK_ERR_INVALID, "internal: chunk schedule is not a permutation");
     }
-    upload_vector(off_d, off, s);
-    upload_vector(list_d, list, s);
-    return longest;
+    upload_vector(M.coff, off, s);
+    upload_vector(M.clist, list, s);
+    M.max_cta_items = longest;
+    M.hoff = std::move(off);
+    M.hlist = std::move(list);
 }
 
 // Memory work of a SELL chunk of padded length L (see above).
@@ -1196,7 +1258,7 @@ void build_schedule(SellMatrix &M, int64_t ctas, cudaStream_t s) {
         ids[size_t(c)] = c;
         work[size_t(c)] = chunk_work(M.chunk_len[size_t(c)], c < split_chunks);
     }
-    M.max_cta_items = schedule_items(ids, work, ctas, M.coff, M.clist, s);
+    schedule_items(ids, work, ctas, M, s);
 }
 
 // The dual kernel's schedule when A's long rows take the panel path: the
@@ -1221,7 +1283,7 @@ void build_dual_panel_schedule(SellMatrix &M, int64_t long_rows, const std::vect
         ids.push_back(c);
         work.push_back(chunk_work(M.chunk_len[size_t(c)], false));
     }
-    M.max_cta_items = schedule_items(ids, work, ctas, M.coff, M.clist, s);
+    schedule_items(ids, work, ctas, M, s);
 }
 
 // Persistent grid: as many CTAs as fit on the device at once, at most one warp
@@ -1520,6 +1582,133 @@ template <class Acc, class V, class I> void attach_slots(Engine &E) {
     }
 }
 
+// Contiguous ranges of chunks for `parts` CTAs, the largest cost as small as it
+// can be (a chunk costs its padded length and a few steps of its own).
+std::vector<int> own_ranges(const std::vector<int32_t> &chunk_len, int parts) {
+    const int n = int(chunk_len.size());
+    auto cost = [&](int c) { return int64_t(chunk_len[size_t(c)]) + 4; };
+    int64_t lo = 0, hi = 0;
+    for (int c = 0; c < n; ++c) {
+        lo = std::max(lo, cost(c));
+        hi += cost(c);
+    }
+    std::vector<int> own;
+    auto fits = [&](int64_t cap) {
+        own.assign(1, 0);
+        int64_t load = 0;
+        for (int c = 0; c < n; ++c) {
+            if (load + cost(c) > cap) {
+                own.push_back(c);
+                load = 0;
+            }
+            load += cost(c);
+        }
+        own.push_back(n);
+        return int(own.size()) <= parts + 1;
+    };
+    while (lo < hi) {
+        const int64_t mid = lo + (hi - lo) / 2;
+        if (fits(mid))
+            hi = mid;
+        else
+            lo = mid + 1;
+    }
+    fits(hi);
+    own.resize(size_t(parts + 1), n);
+    return own;
+}
+
+// Turns the resident kernel on (nk_resident.cuh) for a model that it can run as the
+// two-kernel path does, bit for bit: 32-bit indices, FP64 sums, no column panels,
+// no sparse Q, no row split across chunks; and that fits: a CTA's products of
+// either matrix and its rows' state in shared memory (up to about 1.5 M entries).
+// Up to there it is the faster path, measured in us a trial on LPs with 6 entries
+// per column (FP64, adaptive), resident against two kernels: 5.5 / 14.6 at 4 k
+// entries, 6.6 / 16.6 at 54 k, 8.0 / 20.6 at 360 k, 12.6 / 22.6 at 720 k,
+// 18.7 / 26.7 at 1.2 M.
+void plan_resident(Engine &E, cudaStream_t s) {
+    ResidentPlan &P = E.resident;
+    ResidentView &R = P.view;
+    if (E.wide || E.precision == NK_PRECISION_FP32 || E.panels || E.sparse_q || E.A.ncounters ||
+        E.At.ncounters || E.A.nv == 0 || E.At.nv == 0)
+        return;
+    const void *k = E.resident_function();
+    int dev = 0, sms = 148, coop = 0, per = 0;
+    cuda_check(cudaGetDevice(&dev), "device");
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+    R.lists_p = E.grid_p;
+    R.lists_d = E.grid_d;
+    if (!coop || std::max(R.lists_p, R.lists_d) > kResMaxLists)
+        return;
+    P.grid = std::min(sms, 1 + int(std::max(E.At.chunk_len.size(), E.A.chunk_len.size())));
+    std::vector<int> ot = own_ranges(E.At.chunk_len, P.grid - 1),
+                     oa = own_ranges(E.A.chunk_len, P.grid - 1);
+    ot.push_back(ot.back());
+    oa.push_back(oa.back());
+    // the largest CTA's entries and virtual rows
+    auto most = [&](const std::vector<int> &own, const std::vector<int32_t> &len, int &rows) {
+        int64_t top = 0;
+        for (int b = 0; b < P.grid; ++b) {
+            int64_t steps = 0;
+            for (int c = own[size_t(b)]; c < own[size_t(b + 1)]; ++c)
+                steps += len[size_t(c)];
+            top = std::max(top, steps);
+            rows = std::max(rows, 32 * (own[size_t(b + 1)] - own[size_t(b)]));
+        }
+        rows = (rows + 63) / 64 * 64;
+        return int(std::min<int64_t>(32 * top, 1 << 24));
+    };
+    R.entries_t = most(ot, E.At.chunk_len, R.cols);
+    R.entries_a = most(oa, E.A.chunk_len, R.rows);
+    R.products = std::max(R.entries_t, R.entries_a);
+    const size_t value = size_t(E.vbits() / 8), budget = smem_budget(k, 1);
+    R.stage = 2;
+    while (R.stage > 0 && resident_shared_bytes(R, value) > budget)
+        --R.stage;
+    P.smem = resident_shared_bytes(R, value);
+    if (P.smem > budget)
+        return;
+    // the limit is the kernel's, not this engine's: another engine may need more
+    cuda_check(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(budget)),
+               "resident shared memory");
+    cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, kResThreads, P.smem),
+               "resident occupancy");
+    if (int64_t(per) * sms < P.grid)
+        return;
+    // each chunk's slot: its list of the two-kernel schedule and its place there
+    auto slots = [&](const SellMatrix &M, int lists, int &width) {
+        width = std::max(32, (M.max_cta_items + 31) / 32 * 32);
+        std::vector<int> slot(M.chunk_len.size(), 0);
+        for (int q = 0; q < lists; ++q)
+            for (int64_t k = M.hoff[size_t(q)]; k < M.hoff[size_t(q + 1)]; ++k)
+                slot[size_t(M.hlist[size_t(k)])] = q * width + int(k - M.hoff[size_t(q)]);
+        return slot;
+    };
+    const std::vector<int> st = slots(E.At, R.lists_p, R.width_p),
+                           sa = slots(E.A, R.lists_d, R.width_d);
+    std::vector<int> lists;
+    for (const std::vector<int> &part : {ot, oa, st, sa})
+        lists.insert(lists.end(), part.begin(), part.end());
+    lists.resize(lists.size() + 2, 0);
+    upload_vector(P.lists, lists, s);
+    R.own_t = P.lists.p;
+    R.own_a = R.own_t + ot.size();
+    R.slot_t = R.own_a + oa.size();
+    R.slot_a = R.slot_t + st.size();
+    R.sync = reinterpret_cast<unsigned *>(P.lists.p + lists.size() - 2);
+    const size_t np = size_t(R.lists_p) * R.width_p, nd = size_t(2) * R.lists_d * R.width_d;
+    P.work.alloc(np + nd + kResWords + (E.halpern ? size_t(E.n + E.m) : 0));
+    cuda_check(cudaMemsetAsync(P.work.p, 0, P.work.bytes(), s), "resident buffers");
+    R.sum_p = P.work.p;
+    R.sum_d = R.sum_p + np;
+    R.word = reinterpret_cast<unsigned long long *>(R.sum_d + nd);
+    R.last_x = R.sum_d + nd + kResWords;
+    R.last_y = R.last_x + E.n;
+    cuda_check(cudaStreamSynchronize(s), "resident plan"); // `lists` leaves scope
+    P.on = true;
+}
+
 Engine *create_engine(const nk_csr *Ah, const nk_csr *Qh, const double *hc, const double *hq,
                       const double *hlb, const double *hub, const double *hrl, const double *hru,
                       const double *hx0, const double *hy0, const nk_pdhg_options *o) {
@@ -1770,6 +1959,7 @@ Engine *create_engine(const nk_csr *Ah, const nk_csr *Qh, const double *hc, cons
         E->wide ? attach_slots<double, float, int64_t>(*E) : attach_slots<double, float, int32_t>(*E);
     else
         E->wide ? attach_slots<float, float, int64_t>(*E) : attach_slots<float, float, int32_t>(*E);
+    plan_resident(*E, s);
     E->split_p.alloc(size_t(std::max(1, E->At.ncounters)));
     E->split_d.alloc(size_t(2 * std::max(1, E->A.ncounters)));
     cuda_check(cudaMemsetAsync(E->split_p.p, 0, E->split_p.bytes(), s), "split slots");

@@ -497,3 +497,61 @@ def test_profiled_trials_are_ordinary_trials(gpu, graphs):
     b.advance(30, tau, sigma)
     for u, w in zip(a.candidates(), b.candidates()):
         assert np.array_equal(u, w)
+
+
+def resident_model(kind):
+    if kind == "one row":
+        m = tiny(3, 1, [(0, 0, 1.0), (0, 1, -2.0), (0, 2, 0.5)])
+        m.c[:] = [1.0, -1.0, 0.5]
+        m.rl[:] = m.ru[:] = 3
+        return m
+    if kind == "empty rows and columns":
+        m = synth.random_lp(m=70, n=131, per_col=2, seed=5)
+        keep = (m.idx % 7 != 0) & (np.repeat(np.arange(m.m), np.diff(m.ptr)) % 5 != 0)
+        counts = np.add.reduceat(np.r_[keep, 0].astype(np.int64), m.ptr[:-1]) * (np.diff(m.ptr) > 0)
+        m.ptr = np.concatenate([[0], np.cumsum(counts)])
+        m.idx, m.val = m.idx[keep], m.val[keep]
+        return m
+    if kind == "dense column":  # 400 entries: a split row of A^T
+        rows, cols = 400, 97
+        rng = np.random.default_rng(6)
+        entries = sorted({(i, 3) for i in range(rows)} |
+                         {(i, int(j)) for i in range(rows) for j in rng.integers(0, cols, 3)})
+        m = tiny(cols, rows, [(i, j, float(rng.standard_normal())) for i, j in entries])
+        m.c[:] = rng.standard_normal(cols)
+        m.rl[:] = m.ru[:] = rng.standard_normal(rows)
+        return m
+    shapes = {"chunk": (32, 64), "chunk and one": (33, 65), "small": (2000, 5000),
+              "unstaged entries": (60000, 130001), "unstaged": (100003, 200001)}
+    m, n = shapes[kind]
+    return synth.random_lp(m=m, n=n, per_col=5, seed=7)
+
+
+@pytest.mark.parametrize("method", ["adaptive", "rejecting", "fixed", "halpern", "quadratic",
+                                    "mixed"])
+@pytest.mark.parametrize("kind", ["one row", "empty rows and columns", "dense column", "chunk",
+                                  "chunk and one", "small", "unstaged entries", "unstaged"])
+def test_resident_trials_match_the_kernel_path(gpu, kind, method):
+    """advance() of a small or medium model runs its trials in one launch; the
+    profiled trials run as kernels of their own.  Both add every sum in the same
+    order, so the points agree bit for bit, over several calls, with rejected
+    trials, Halpern commits, a diagonal quadratic term and FP32 values."""
+    m = resident_model(kind)
+    if method == "quadratic":
+        m.q = np.random.default_rng(8).uniform(0.1, 1.0, m.n)
+    tau, sigma = step_sizes(m)
+    if method == "rejecting":
+        tau, sigma = 40 * tau, 40 * sigma
+    options = dict(adaptive=method not in ("fixed", "halpern"), graphs=True,
+                   precision="mixed" if method == "mixed" else "fp64")
+    if method == "halpern":
+        options.update(halpern=True, reflection=0.5, residual_restarts=True)
+    a, b = gpu.PdhgBackend(m, **options), gpu.PdhgBackend(m, **options)
+    for count in (1, 2, 30):
+        a.advance(count, tau, sigma)
+        b.profile_kernels(count, tau, sigma)
+        for u, w in zip(a.candidates(), b.candidates()):
+            assert np.array_equal(u, w)
+    assert a.rejected_steps() == b.rejected_steps()
+    if method == "rejecting" and kind == "small":
+        assert a.rejected_steps() > 0
