@@ -1812,8 +1812,10 @@ Engine *create_engine(const nk_csr *Ah, const nk_csr *Qh, const double *hc, cons
                 width >= 16 && long_entries >= NK_PANEL_MIN_RUN * np * E->A.nsr;
             if (long_runs && np * E->A.nsr <= (int64_t(1) << 25)) {
                 const size_t smem = size_t(width * xsize);
+                // the limit is the kernel's, not this engine's: an engine with wider
+                // panels may be alive
                 cuda_check(cudaFuncSetAttribute(pk, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                int(smem)),
+                                                int(smem_budget(pk, kPanelMinBlocks))),
                            "panel shared memory");
                 int dev = 0, sms = 148, per = 0;
                 cuda_check(cudaGetDevice(&dev), "device");

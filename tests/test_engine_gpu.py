@@ -555,3 +555,16 @@ def test_resident_trials_match_the_kernel_path(gpu, kind, method):
     assert a.rejected_steps() == b.rejected_steps()
     if method == "rejecting" and kind == "small":
         assert a.rejected_steps() > 0
+
+
+def test_panel_engines_of_different_widths_coexist(gpu):
+    """Two engines whose panels differ in width: the kernel's shared-memory limit
+    belongs to both, so the wider one still runs after the narrower was built."""
+    wide = synth.power_law_lp(m=20000, n=100000, nnz=500000, seed=3, len_hi=5000)
+    narrow = synth.power_law_lp(m=3000, n=6000, nnz=60000, seed=4, len_hi=3000)
+    a = gpu.PdhgBackend(wide)
+    b = gpu.PdhgBackend(narrow)
+    assert a.layout_info()["panel_width"] > b.layout_info()["panel_width"] > 0
+    for g, m in ((a, wide), (b, narrow)):
+        tau, sigma = step_sizes(m)
+        assert g.advance(5, tau, sigma) == 5
