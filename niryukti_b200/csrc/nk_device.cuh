@@ -1,6 +1,7 @@
 // Kernels of the B200 PDHG engine (host side: nk_engine.cu).
 //
 // One PDHG trial is two kernels over SELL-32 matrices (nk_sell.cuh):
+//   (q_rows_kernel Q x of the current iterate, for a sparse Q)
 //   primal_kernel  g = c + A^T y (+ Q x + q.x)   -- one lane per row of A^T
 //                  trial x = clamp((x - tau g)/(1 + tau q), lb, ub), dx, sum dx^2
 //                  (restates primal_trial, src/cuda.cu:240-260, and the CPU loop
@@ -71,6 +72,8 @@ struct Control {
 struct Vecs {
     const double *c, *q, *lb, *ub, *rl, *ru;
     double *x0, *x1, *y0, *y1, *ax0, *ax1, *xa, *ya;
+    double *qx0, *qx1;    // sparse Q: Q x of x0, x1 (the current one's, with the resident
+                          // kernel also the trial's)
     double *dx;           // primal displacement (FP64 gather source)
     float *dx32;          // FP32 gather source (precision FP32)
     float *y32_0, *y32_1; // FP32 copies of y (precision FP32)
@@ -279,7 +282,7 @@ __device__ __forceinline__ void ordered_slots(const double *slots, int count, do
 // order, so it too lands in the sums the same way every time.
 template <class Acc, class V, class I, bool SPARSE_Q, bool FP32G, bool SPLIT>
 __global__ void __launch_bounds__(kFusedThreads, kFusedMinBlocks)
-    primal_kernel(Sell<V, I> At, QCsr<V, I> Q, Vecs v) {
+    primal_kernel(Sell<V, I> At, Vecs v) {
     __shared__ double wpart[SPLIT ? kFusedWarps : 1][32];
     __shared__ unsigned claim;
     extern __shared__ __align__(16) unsigned char dyn_smem[];
@@ -300,13 +303,14 @@ __global__ void __launch_bounds__(kFusedThreads, kFusedMinBlocks)
         double *xt = cur ? v.x0 : v.x1;
         const double *y = cur ? v.y1 : v.y0;
         const float *y32 = cur ? v.y32_1 : v.y32_0;
+        const double *qx = cur ? v.qx1 : v.qx0;
         // epilogue of column j; g = c_j + (A^T y)_j; returns dx_j^2 (inf if not finite)
         auto finish = [&](int64_t j, double g, double xj, double qj, double lj, double uj,
                           double aj) -> double {
             if (pending)
                 v.xa[j] = aj + (xj - aj) * pw;
             if constexpr (SPARSE_Q)
-                g = g + (double(q_dot<Acc>(Q, j, x)) + qj * xj);
+                g = g + (qx[j] + qj * xj);
             double t = (xj - tau * g) / (1 + tau * (SPARSE_Q ? 0. : qj));
             t = clampd(t, lj, uj);
             xt[j] = t;
@@ -713,11 +717,22 @@ __global__ void __launch_bounds__(kThreads) spmv_kernel(Sell<V, I> M, const doub
         }
     }
 }
+// Q x on the rows of Q that have entries: into qx0 from x0, or, by the control's
+// index, into qx1 from x1.
 template <class V, class I>
-__global__ void q_spmv_kernel(int64_t n, QCsr<V, I> Q, const double *x, double *out) {
-    int64_t stride = int64_t(gridDim.x) * blockDim.x;
-    for (int64_t r = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; r < n; r += stride)
-        out[r] = q_dot<double>(Q, r, x);
+__global__ void __launch_bounds__(kThreads) q_rows_kernel(QCsr<V, I> Q, const double *x0,
+                                                          const double *x1, double *qx0,
+                                                          double *qx1, const Control *ctl) {
+    const bool second = ctl && ctl->cur;
+    const double *x = second ? x1 : x0;
+    double *out = second ? qx1 : qx0;
+    const int per = kThreads / Q.lanes;
+    for (int r = blockIdx.x * per + threadIdx.x / Q.lanes; r - int(threadIdx.x) / Q.lanes < Q.nrows;
+         r += gridDim.x * per) { // the same turns for every warp of the CTA
+        const double s = q_row(Q, r, Q.nrows, x);
+        if (r < Q.nrows && (threadIdx.x & (Q.lanes - 1)) == 0)
+            out[Q.rows[r]] = s;
+    }
 }
 
 // ------------------------------------------------------------------ monitor

@@ -112,10 +112,12 @@ struct QMatrix {
     int64_t n = 0, nnz = 0;
     bool wide = false;
     int vbits = 64;
+    int nrows = 0, lanes = 1; // rows with entries, and the lanes that share one (QCsr)
     DevBuf<int64_t> ptr, idx64;
-    DevBuf<int32_t> idx32;
+    DevBuf<int32_t> idx32, rows;
     DevBuf<double> val64;
     DevBuf<float> val32;
+    std::vector<int32_t> hlen; // entries of each of those rows
     template <class V, class I> QCsr<V, I> view() const {
         QCsr<V, I> q;
         q.ptr = ptr.p;
@@ -127,10 +129,14 @@ struct QMatrix {
             q.val = reinterpret_cast<const V *>(val64.p);
         else
             q.val = reinterpret_cast<const V *>(val32.p);
+        q.rows = rows.p;
+        q.nrows = nrows;
+        q.lanes = lanes;
         return q;
     }
     size_t device_bytes() const {
-        return ptr.bytes() + idx64.bytes() + idx32.bytes() + val64.bytes() + val32.bytes();
+        return ptr.bytes() + idx64.bytes() + idx32.bytes() + rows.bytes() + val64.bytes() +
+               val32.bytes();
     }
 };
 
@@ -178,7 +184,7 @@ struct ResidentPlan {
     unsigned tag = 1;
     size_t smem = 0;
     ResidentView view{};
-    DevBuf<int> lists;   // own_t, own_a, slot_t, slot_a, sync of the view
+    DevBuf<int> lists;   // own_t, own_a, slot_t, slot_a, own_q, sync of the view
     DevBuf<double> work; // sum_p, sum_d, word, last_x, last_y
     size_t device_bytes() const { return lists.bytes() + work.bytes(); }
 };
@@ -453,7 +459,7 @@ void upload_raw(const nk_csr *H, int vbits, cudaStream_t stream, DevBuf<int64_t>
 
 // The primal kernel instance for a model: sparse Q or not, split rows of A^T
 // or not (each leaves unused paths out of the build).
-template <class V, class I> using PrimalFn = void (*)(Sell<V, I>, QCsr<V, I>, Vecs);
+template <class V, class I> using PrimalFn = void (*)(Sell<V, I>, Vecs);
 template <class Acc, class V, class I> PrimalFn<V, I> primal_kernel_for(bool sparse_q, bool split) {
     constexpr bool F = sizeof(Acc) == 4;
     if (sparse_q)
@@ -462,12 +468,12 @@ template <class Acc, class V, class I> PrimalFn<V, I> primal_kernel_for(bool spa
     return split ? primal_kernel<Acc, V, I, false, F, true> : primal_kernel<Acc, V, I, false, F, false>;
 }
 
-template <class V> const void *resident_kernel_of(bool split, bool halpern) {
+template <class V, bool QP> const void *resident_kernel_of(bool split, bool halpern) {
     if (halpern)
-        return split ? (const void *)resident_kernel<V, true, true>
-                     : (const void *)resident_kernel<V, false, true>;
-    return split ? (const void *)resident_kernel<V, true, false>
-                 : (const void *)resident_kernel<V, false, false>;
+        return split ? (const void *)resident_kernel<V, true, true, QP>
+                     : (const void *)resident_kernel<V, false, true, QP>;
+    return split ? (const void *)resident_kernel<V, true, false, QP>
+                 : (const void *)resident_kernel<V, false, false, QP>;
 }
 
 // ------------------------------------------------------------------ engine
@@ -483,8 +489,8 @@ struct Engine {
     QMatrix Q;
     PanelMatrix pan; // A's long rows by column panel (the dual SpMV), when panels
     bool panels = false;
-    DevBuf<double> c, q, lb, ub, rl, ru, x[2], y[2], ax[2], xa, ya, dx, anchor_x, anchor_y,
-        anchor_ax, part_p, part_d, mon_ax, mon_aty, mon_qx, mon_part, mon_out;
+    DevBuf<double> c, q, lb, ub, rl, ru, x[2], y[2], ax[2], xa, ya, qx[2], dx, anchor_x,
+        anchor_y, anchor_ax, part_p, part_d, mon_ax, mon_aty, mon_qx, mon_part, mon_out;
     DevBuf<float> dx32, y32[2];
     DevBuf<Control> ctl;
     DevBuf<unsigned> mon_arrive;
@@ -536,6 +542,8 @@ struct Engine {
         v.ax1 = ax[1].p;
         v.xa = xa.p;
         v.ya = ya.p;
+        v.qx0 = qx[0].p;
+        v.qx1 = qx[1].p;
         v.dx = dx.p;
         v.dx32 = dx32.p;
         v.y32_0 = y32[0].p;
@@ -573,11 +581,12 @@ struct Engine {
         constexpr bool F32 = sizeof(Acc) == 4;
         auto at = At.fused_view<V, I>();
         auto a = A.fused_view<V, I>();
-        auto qm = Q.view<V, I>();
         if (ev[0])
             mark(0);
+        if (sparse_q)
+            q_rows(x[0].p, x[1].p, qx[0].p, qx[1].p, ctl.p);
         primal_kernel_for<Acc, V, I>(sparse_q, At.nsv > 0)<<<grid_p, kFusedThreads, smem_p(),
-                                                              stream>>>(at, qm, v);
+                                                              stream>>>(at, v);
         if (ev[1])
             mark(1);
         if (panels) {
@@ -636,17 +645,21 @@ struct Engine {
     }
     const void *resident_function() const {
         const bool split = A.nsv + At.nsv > 0;
-        return precision == NK_PRECISION_FP64 ? resident_kernel_of<double>(split, halpern)
-                                              : resident_kernel_of<float>(split, halpern);
+        return sparse_q                         ? resident_kernel_of<double, true>(split, halpern)
+               : precision == NK_PRECISION_FP64 ? resident_kernel_of<double, false>(split, halpern)
+                                                : resident_kernel_of<float, false>(split, halpern);
     }
     template <class V> void launch_resident_t(int count) {
         auto at = At.view<V, int32_t>();
         auto a = A.view<V, int32_t>();
+        auto q = Q.view<V, int32_t>();
         Vecs v = vecs();
+        if (sparse_q) // of the current iterate; the kernel forms the trials'
+            q_rows(x[0].p, x[1].p, qx[0].p, qx[1].p, ctl.p);
         // the decision messages' tags: the next one is never what the words still hold
         unsigned tag = resident.tag;
         resident.tag += unsigned(count);
-        void *args[] = {&at, &a, &v, &resident.view, &count, &tag};
+        void *args[] = {&at, &a, &q, &v, &resident.view, &count, &tag};
         cuda_check(cudaLaunchCooperativeKernel(resident_function(), dim3(resident.grid),
                                                dim3(kResThreads), args, resident.smem, stream),
                    "trial launch");
@@ -675,20 +688,31 @@ struct Engine {
         }
         cuda_check(cudaGetLastError(), "spmv launch");
     }
+    // out = Q xin (FP64 sums)
     void q_spmv(const double *xin, double *out) {
-        int g = grid_for(n);
+        cuda_check(cudaMemsetAsync(out, 0, size_t(n) * 8, stream), "Q rows without entries");
+        q_rows(xin, xin, out, out, nullptr);
+    }
+    void q_rows(const double *x0, const double *x1, double *out0, double *out1,
+                const Control *c) {
         if (Q.vbits == 64) {
             if (Q.wide)
-                q_spmv_kernel<double, int64_t><<<g, kThreads, 0, stream>>>(n, Q.view<double, int64_t>(), xin, out);
+                q_rows_t<double, int64_t>(x0, x1, out0, out1, c);
             else
-                q_spmv_kernel<double, int32_t><<<g, kThreads, 0, stream>>>(n, Q.view<double, int32_t>(), xin, out);
+                q_rows_t<double, int32_t>(x0, x1, out0, out1, c);
         } else {
             if (Q.wide)
-                q_spmv_kernel<float, int64_t><<<g, kThreads, 0, stream>>>(n, Q.view<float, int64_t>(), xin, out);
+                q_rows_t<float, int64_t>(x0, x1, out0, out1, c);
             else
-                q_spmv_kernel<float, int32_t><<<g, kThreads, 0, stream>>>(n, Q.view<float, int32_t>(), xin, out);
+                q_rows_t<float, int32_t>(x0, x1, out0, out1, c);
         }
-        cuda_check(cudaGetLastError(), "Q spmv launch");
+        cuda_check(cudaGetLastError(), "Q product");
+    }
+    template <class V, class I>
+    void q_rows_t(const double *x0, const double *x1, double *out0, double *out1,
+                  const Control *c) {
+        q_rows_kernel<V, I><<<grid_for(int64_t(Q.nrows) * Q.lanes), kThreads, 0, stream>>>(
+            Q.view<V, I>(), x0, x1, out0, out1, c);
     }
 
     void sync_ctl() {
@@ -1162,7 +1186,7 @@ struct Engine {
         size_t b = A.device_bytes() + At.device_bytes() + Q.device_bytes() + pan.device_bytes() +
                    resident.device_bytes();
         for (auto *d : {&c, &q, &lb, &ub, &rl, &ru, &x[0], &x[1], &y[0], &y[1], &ax[0], &ax[1],
-                        &xa, &ya, &dx, &anchor_x, &anchor_y, &anchor_ax, &part_p, &part_d,
+                        &xa, &ya, &qx[0], &qx[1], &dx, &anchor_x, &anchor_y, &anchor_ax, &part_p, &part_d,
                         &scratch_n, &scratch_m})
             b += d->bytes();
         b += dx32.bytes() + y32[0].bytes() + y32[1].bytes() + col_perm.bytes() + row_perm.bytes();
@@ -1620,7 +1644,7 @@ std::vector<int> own_ranges(const std::vector<int32_t> &chunk_len, int parts) {
 
 // Turns the resident kernel on (nk_resident.cuh) for a model that it can run as the
 // two-kernel path does, bit for bit: 32-bit indices, FP64 sums, no column panels,
-// no sparse Q, no row split across chunks; and that fits: a CTA's products of
+// no row split across chunks; and that fits: a CTA's products of
 // either matrix and its rows' state in shared memory (up to about 1.5 M entries).
 // Up to there it is the faster path, measured in us a trial on LPs with 6 entries
 // per column (FP64, adaptive), resident against two kernels: 5.5 / 14.6 at 4 k
@@ -1629,7 +1653,7 @@ std::vector<int> own_ranges(const std::vector<int32_t> &chunk_len, int parts) {
 void plan_resident(Engine &E, cudaStream_t s) {
     ResidentPlan &P = E.resident;
     ResidentView &R = P.view;
-    if (E.wide || E.precision == NK_PRECISION_FP32 || E.panels || E.sparse_q || E.A.ncounters ||
+    if (E.wide || E.precision == NK_PRECISION_FP32 || E.panels || E.A.ncounters ||
         E.At.ncounters || E.A.nv == 0 || E.At.nv == 0)
         return;
     const void *k = E.resident_function();
@@ -1688,7 +1712,22 @@ void plan_resident(Engine &E, cudaStream_t s) {
     const std::vector<int> st = slots(E.At, R.lists_p, R.width_p),
                            sa = slots(E.A, R.lists_d, R.width_d);
     std::vector<int> lists;
-    for (const std::vector<int> &part : {ot, oa, st, sa})
+    // Q's rows with entries, in ranges of about equal work
+    std::vector<int> oq(size_t(P.grid) + 1, E.Q.nrows);
+    {
+        int64_t total = 0, before = 0;
+        for (int32_t l : E.Q.hlen)
+            total += l + 32;
+        int b = 0;
+        for (int r = 0; r < E.Q.nrows; ++r) {
+            for (; b < P.grid - 1 && before * (P.grid - 1) >= total * b; ++b)
+                oq[size_t(b)] = r;
+            before += E.Q.hlen[size_t(r)] + 32;
+        }
+        if (E.Q.nrows == 0)
+            oq.assign(oq.size(), 0);
+    }
+    for (const std::vector<int> &part : {ot, oa, st, sa, oq})
         lists.insert(lists.end(), part.begin(), part.end());
     lists.resize(lists.size() + 2, 0);
     upload_vector(P.lists, lists, s);
@@ -1696,6 +1735,7 @@ void plan_resident(Engine &E, cudaStream_t s) {
     R.own_a = R.own_t + ot.size();
     R.slot_t = R.own_a + oa.size();
     R.slot_a = R.slot_t + st.size();
+    R.own_q = R.slot_a + sa.size();
     R.sync = reinterpret_cast<unsigned *>(P.lists.p + lists.size() - 2);
     const size_t np = size_t(R.lists_p) * R.width_p, nd = size_t(2) * R.lists_d * R.width_d;
     P.work.alloc(np + nd + kResWords + (E.halpern ? size_t(E.n + E.m) : 0));
@@ -1868,6 +1908,21 @@ Engine *create_engine(const nk_csr *Ah, const nk_csr *Qh, const double *hc, cons
         else
             convert_csr<float, int32_t><<<g, kThreads, 0, s>>>(qnnz, pi.p, pv.p, E->Q.idx32.p, E->Q.val32.p);
         cuda_check(cudaGetLastError(), "Q convert");
+        std::vector<int32_t> qrows;
+        for (int64_t j = 0; j < n; ++j)
+            if (pptr[size_t(j + 1)] > pptr[size_t(j)]) {
+                qrows.push_back(int32_t(j));
+                E->Q.hlen.push_back(int32_t(std::min<int64_t>(INT32_MAX, pptr[size_t(j + 1)] - pptr[size_t(j)])));
+            }
+        E->Q.nrows = int(qrows.size());
+        const int64_t mean = qnnz / std::max(1, E->Q.nrows);
+        while (E->Q.lanes < 32 && 4 * E->Q.lanes < mean)
+            E->Q.lanes *= 2;
+        upload_vector(E->Q.rows, qrows, s);
+        for (auto &d : E->qx) {
+            d.alloc(size_t(n));
+            cuda_check(cudaMemsetAsync(d.p, 0, d.bytes(), s), "Q product");
+        }
         cuda_check(cudaStreamSynchronize(s), "Q build");
         // norms for the QP step safety (src/cpu.cpp:25-42, src/model.cpp:257-267)
         std::vector<double> cols(static_cast<size_t>(n), 0.0);

@@ -54,6 +54,7 @@ constexpr int kResMaxPolls = 4 << 20; // seconds: the barrier's bound
 struct ResidentView {
     const int *own_t, *own_a;   // CTA b owns chunks [own[b], own[b+1]); the last CTA none
     const int *slot_t, *slot_a; // chunk -> its place (list * width + position)
+    const int *own_q;           // sparse Q: CTA b owns its rows [own_q[b], own_q[b+1])
     int lists_p, lists_d;       // CTA lists of the two-kernel schedule
     int width_p, width_d;       // their lengths, padded to a multiple of 32 (zero slots)
     double *sum_p;              // dx^2 per chunk
@@ -299,10 +300,12 @@ __device__ __forceinline__ void resident_leave(const ResidentView &R) {
     }
 }
 
-template <class V, bool SPLIT, bool HALPERN>
+// QP: with a sparse Q, whose product with the trial x is formed in the dual part,
+// beside A dx, and is the next trial's Q x unless the trial is rejected.
+template <class V, bool SPLIT, bool HALPERN, bool QP>
 __global__ void __launch_bounds__(kResThreads, 1)
-    resident_kernel(Sell<V, int32_t> At, Sell<V, int32_t> A, Vecs v, ResidentView R, int trials,
-                    unsigned tag) {
+    resident_kernel(Sell<V, int32_t> At, Sell<V, int32_t> A, QCsr<V, int32_t> Q, Vecs v,
+                    ResidentView R, int trials, unsigned tag) {
     extern __shared__ __align__(16) unsigned char dyn_smem[];
     __shared__ double wpart[SPLIT ? kResWarps : 1][32];
     __shared__ Control c;
@@ -423,10 +426,15 @@ __global__ void __launch_bounds__(kResThreads, 1)
         {
             const double tau = c.tau * c.factor;
             const int co = cur ? R.cols : 0, to = cur ? 0 : R.cols;
+            const double *qx = cur ? v.qx1 : v.qx0;
+            double *gxt = cur ? v.x0 : v.x1;
             auto finish = [&](int l, int j, double g) -> double {
                 const int o = staged ? l : j - first_t;
                 const double xj = sx[co + l], lj = blb[o], uj = bub[o], aj = sxa[l];
-                const double den = 1 + tau * (bq ? bq[o] : 0.);
+                const double qj = bq ? bq[o] : 0.;
+                if constexpr (QP)
+                    g = g + (__ldcg(qx + j) + qj * xj);
+                const double den = QP ? 1. : 1 + tau * qj;
                 double T = xj - tau * g;
                 if (den != 1) // x / 1 is x
                     T = T / den;
@@ -443,6 +451,8 @@ __global__ void __launch_bounds__(kResThreads, 1)
                     xn = lam * v.anchor_x[j] + (1 - lam) * ((1 + r) * T - r * xj);
                 }
                 sx[to + l] = xn;
+                if constexpr (QP)
+                    __stcg(gxt + j, xn);
                 return isfinite(T) ? d * d : INFINITY;
             };
             for (int k = warp; k < nt; k += kResWarps) {
@@ -468,6 +478,17 @@ __global__ void __launch_bounds__(kResThreads, 1)
         if (!grid_barrier(R.sync, ++barrier, v.ctl, &ok)) // dx is complete
             return;
         // -------------------------------------------------- dual part
+        if constexpr (QP) {
+            const double *xt = cur ? v.x0 : v.x1;
+            double *qxt = cur ? v.qx0 : v.qx1;
+            const int per = kResThreads / Q.lanes, end = R.own_q[blockIdx.x + 1];
+            for (int k = R.own_q[blockIdx.x]; k < end; k += per) {
+                const int row = k + int(threadIdx.x) / Q.lanes;
+                const double s = q_row(Q, row, end, xt);
+                if (row < end && (threadIdx.x & (Q.lanes - 1)) == 0)
+                    __stcg(qxt + Q.rows[row], s);
+            }
+        }
         flat_products(ip_a, vp_a, acount, v.dx, prod);
         double *gyt = cur ? v.y0 : v.y1;
         {

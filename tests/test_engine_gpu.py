@@ -568,3 +568,45 @@ def test_panel_engines_of_different_widths_coexist(gpu):
     for g, m in ((a, wide), (b, narrow)):
         tau, sigma = step_sizes(m)
         assert g.advance(5, tau, sigma) == 5
+
+
+def sparse_q(n, kind):
+    """Symmetric CSR of a positive semidefinite Q: a few rows of a rank-four term,
+    a tridiagonal matrix, or one dense row and column."""
+    rng = np.random.default_rng(9)
+    if kind == "low rank":
+        return synth.sparse_qp_terms(rng, n)[:3]
+    dense = np.zeros((n, n))
+    k = np.arange(n)
+    if kind == "tridiagonal":
+        dense[k, k] = 2.0
+        dense[k[1:], k[:-1]] = dense[k[:-1], k[1:]] = -1.0
+    else:
+        dense[5, :] = dense[:, 5] = 0.01
+        dense[k, k] = 1.0
+    ptr = np.r_[0, np.cumsum(np.count_nonzero(dense, axis=1))].astype(np.int64)
+    r, c = np.nonzero(dense)
+    return ptr, c.astype(np.int64), dense[r, c]
+
+
+@pytest.mark.parametrize("halpern", [False, True])
+@pytest.mark.parametrize("kind", ["low rank", "tridiagonal", "dense row"])
+def test_sparse_q_rows_shared_by_lanes(gpu, oracle, kind, halpern):
+    """Q x by groups of lanes: the resident trials and the kernel path agree bit for
+    bit, and both with the oracle's sequential row sums to 1e-11 (a row of up to
+    600 terms of one size rounds within 600 ulp, 1.4e-13, per trial)."""
+    m = synth.random_lp(m=300, n=600, per_col=4, seed=10)
+    m.qptr, m.qidx, m.qval = sparse_q(m.n, kind)
+    tau, sigma = step_sizes(m)
+    options = dict(halpern=halpern, reflection=0.5 if halpern else 0.0)
+    a, b = gpu.PdhgBackend(m, graphs=True, **options), gpu.PdhgBackend(m, graphs=True, **options)
+    cpu = oracle.model(m).backend(np.zeros(m.n), np.zeros(m.m), **options)
+    # the step sizes a QP's advance would reduce its own to are the caller's here
+    scale = 0.01
+    for count in (1, 30):
+        a.advance(count, scale * tau, scale * sigma)
+        b.profile_kernels(count, scale * tau, scale * sigma)
+        cpu.advance(count, scale * tau, scale * sigma)
+        for u, w, z in zip(a.candidates(), b.candidates(), cpu.candidates()):
+            assert np.array_equal(u, w)
+            near(u, z)
