@@ -677,21 +677,86 @@ __global__ void halpern_commit(int64_t n, int64_t m, Vecs v, bool fp32g) {
     }
 }
 
-// Fold a pending averaging step into xa / ya (commit of the last accepted trial).
-__global__ void flush_average(int64_t n, int64_t m, Vecs v) {
-    const Control &s = *v.ctl;
-    if (!s.pending)
-        return;
-    double w = s.pending_w;
-    const double *x = s.cur ? v.x1 : v.x0;
-    const double *y = s.cur ? v.y1 : v.y0;
-    int64_t stride = int64_t(gridDim.x) * blockDim.x;
-    for (int64_t j = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; j < n; j += stride)
-        v.xa[j] = v.xa[j] + (x[j] - v.xa[j]) * w;
-    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < m; i += stride)
-        v.ya[i] = v.ya[i] + (y[i] - v.ya[i]) * w;
+// ------------------------------------------------------------------ between intervals
+// What happens between two runs of trials, each in one launch: the host knows
+// which buffer holds the iterate and what average is pending.
+
+// Fold a pending averaging step (weight w) into xa / ya (commit of the last
+// accepted trial).
+__global__ void flush_average(int64_t n, int64_t m, const double *x, const double *y, double *xa,
+                              double *ya, double w, Control *ctl) {
+    const int64_t stride = int64_t(gridDim.x) * blockDim.x;
+    const int64_t first = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    for (int64_t j = first; j < n; j += stride)
+        xa[j] = xa[j] + (x[j] - xa[j]) * w;
+    for (int64_t i = first; i < m; i += stride)
+        ya[i] = ya[i] + (y[i] - ya[i]) * w;
+    if (first == 0)
+        ctl->pending = 0;
 }
-__global__ void clear_pending(Control *s) { s->pending = 0; }
+// The current and averaged points in the caller's order (a null one is skipped),
+// with flush_average's step when `pending`.
+__global__ void collect_points(int64_t n, int64_t m, const int64_t *col_perm,
+                               const int64_t *row_perm, const double *x, const double *y,
+                               double *xa, double *ya, int pending, double w, double *ox,
+                               double *oy, double *oxa, double *oya, Control *ctl) {
+    const int64_t stride = int64_t(gridDim.x) * blockDim.x;
+    const int64_t first = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    auto collect = [&](int64_t len, const int64_t *perm, const double *cur, double *avg,
+                       double *ocur, double *oavg) {
+        for (int64_t k = first; k < len; k += stride) {
+            const int64_t to = perm[k];
+            const double c = cur[k];
+            double a = avg[k];
+            if (pending) {
+                a = a + (c - a) * w;
+                avg[k] = a;
+            }
+            if (ocur)
+                ocur[to] = c;
+            if (oavg)
+                oavg[to] = a;
+        }
+    };
+    collect(n, col_perm, x, xa, ox, oxa);
+    collect(m, row_perm, y, ya, oy, oya);
+    if (pending && first == 0)
+        ctl->pending = 0;
+}
+// Restart from a new point: sx, sy in the caller's order (col_perm, row_perm), or
+// with perms null in engine order, or with sx null the iterate as it stands.
+// Averages and their mass start again, and a Halpern engine's epoch.
+__global__ void restart_point(int64_t n, int64_t m, const int64_t *col_perm,
+                              const int64_t *row_perm, const double *sx, const double *sy,
+                              double *x, double *y, float *y32, double *xa, double *ya,
+                              Control *ctl, int cur) {
+    const int64_t stride = int64_t(gridDim.x) * blockDim.x;
+    const int64_t first = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    for (int64_t j = first; j < n; j += stride) {
+        if (sx)
+            x[j] = sx[col_perm ? col_perm[j] : j];
+        xa[j] = 0;
+    }
+    for (int64_t i = first; i < m; i += stride) {
+        if (sy)
+            y[i] = sy[row_perm ? row_perm[i] : i];
+        if (y32)
+            y32[i] = float(y[i]);
+        ya[i] = 0;
+    }
+    if (first == 0) {
+        ctl->cur = cur;
+        ctl->pending = 0;
+        ctl->mass = 0;
+        if (ctl->flags & 2) {
+            ctl->epoch = 0;
+            ctl->init_res = INFINITY;
+            ctl->prev_res = INFINITY;
+            ctl->restart = 0;
+            ctl->lambda = 0;
+        }
+    }
+}
 
 // ------------------------------------------------------------------ plain SpMV
 // out = M x (engine order on both sides, FP64 accumulation): activity rebasing

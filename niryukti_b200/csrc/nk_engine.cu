@@ -495,6 +495,7 @@ struct Engine {
     DevBuf<Control> ctl;
     DevBuf<unsigned> mon_arrive;
     Control *host_ctl = nullptr; // pinned mirror
+    bool ctl_known = false;      // it equals the device's (stream order)
     int grid_p = 1, grid_d = 1, grid_s = 148;
     // rows split across chunks: each one's step-rule contributions (A^T: dx^2;
     // A: dy^2, dy * delta)
@@ -715,11 +716,16 @@ struct Engine {
             Q.view<V, I>(), x0, x1, out0, out1, c);
     }
 
+    // The host's copy of the control state: read back only when trials have run
+    // since it was last known.
     void sync_ctl() {
+        if (ctl_known)
+            return;
         cuda_check(cudaMemcpyAsync(host_ctl, ctl.p, sizeof(Control), cudaMemcpyDeviceToHost,
                                    stream),
                    "control download");
         cuda_check(cudaStreamSynchronize(stream), "control sync");
+        ctl_known = true;
     }
     void push_ctl() {
         cuda_check(cudaMemcpyAsync(ctl.p, host_ctl, sizeof(Control), cudaMemcpyHostToDevice,
@@ -727,10 +733,14 @@ struct Engine {
                    "control upload");
     }
     void flush() {
-        Vecs v = vecs();
-        flush_average<<<grid_for(std::max(n, m)), kThreads, 0, stream>>>(n, m, v);
-        clear_pending<<<1, 1, 0, stream>>>(ctl.p);
+        sync_ctl();
+        if (!host_ctl->pending)
+            return;
+        const int cur = host_ctl->cur;
+        flush_average<<<grid_for(std::max(n, m)), kThreads, 0, stream>>>(
+            n, m, x[cur].p, y[cur].p, xa.p, ya.p, host_ctl->pending_w, ctl.p);
         cuda_check(cudaGetLastError(), "flush");
+        host_ctl->pending = 0;
     }
     // Recompute the resident activity A*x of the current iterate.
     void refresh_activity(int cur) {
@@ -783,6 +793,7 @@ struct Engine {
             push_ctl();
         }
         int left = count;
+        ctl_known = false;
         if (resident.on) {
             for (; left > 0; left -= kResidentTrials)
                 launch_resident(std::min(left, kResidentTrials));
@@ -802,6 +813,7 @@ struct Engine {
         if (host_ctl->fault) {
             host_ctl->fault = 0;
             push_ctl();
+            ctl_known = false;
             cuda_check(cudaMemsetAsync(resident.view.sync, 0, 2 * sizeof(unsigned), stream),
                        "trial counters");
             throw Error(NK_ERR_CUDA, "a wait inside the trial kernel was given up");
@@ -859,27 +871,37 @@ struct Engine {
     void upload_y(double *d, const double *h) { upload_perm(d, h, m, row_perm, scratch_m); }
 
     void candidates(double *hx, double *hy, double *hxa, double *hya) {
-        flush();
         sync_ctl();
-        int cur = host_ctl->cur;
-        // four stream-ordered transfers, one synchronisation
-        download_perm(hx, x[cur].p, n, col_perm, scratch_n, false);
-        download_perm(hy, y[cur].p, m, row_perm, scratch_m, false);
-        download_perm(hxa, xa.p, n, col_perm, scratch_n, false);
-        download_perm(hya, ya.p, m, row_perm, scratch_m, false);
+        const int cur = host_ctl->cur;
+        // all four points in one launch, four stream-ordered transfers, one
+        // synchronisation
+        double *ox = scratch_n.p, *oxa = ox + n, *oy = scratch_m.p, *oya = oy + m;
+        collect_points<<<grid_for(std::max(n, m)), kThreads, 0, stream>>>(
+            n, m, col_perm.p, row_perm.p, x[cur].p, y[cur].p, xa.p, ya.p, host_ctl->pending,
+            host_ctl->pending_w, hx ? ox : nullptr, hy ? oy : nullptr, hxa ? oxa : nullptr,
+            hya ? oya : nullptr, ctl.p);
+        cuda_check(cudaGetLastError(), "candidates");
+        host_ctl->pending = 0;
+        download(hx, ox, n);
+        download(hy, oy, m);
+        download(hxa, oxa, n);
+        download(hya, oya, m);
         refresh_activity(cur); // rebase A*x like the reference (src/cuda.cu:874-891)
         cuda_check(cudaStreamSynchronize(stream), "candidates");
     }
 
-    void zero_average() {
-        if (n)
-            cuda_check(cudaMemsetAsync(xa.p, 0, size_t(n) * 8, stream), "zero xa");
-        if (m)
-            cuda_check(cudaMemsetAsync(ya.p, 0, size_t(m) * 8, stream), "zero ya");
-    }
-
-    void restart_state(int cur) {
-        // common tail of reset / reset_candidate (src/cuda.cu:911-930,941-948)
+    // Restart from (sx, sy) -- device vectors in the caller's order with perms,
+    // in engine order without, null for the iterate as it stands -- in the
+    // buffer that holds the iterate (the common tail of reset and
+    // reset_candidate, src/cuda.cu:911-930,941-948).
+    void restart_state(const double *sx, const double *sy, bool permuted) {
+        const int cur = host_ctl->cur;
+        restart_point<<<grid_for(std::max(n, m)), kThreads, 0, stream>>>(
+            n, m, permuted ? col_perm.p : nullptr, permuted ? row_perm.p : nullptr, sx, sy,
+            x[cur].p, y[cur].p, precision == NK_PRECISION_FP32 ? y32[cur].p : nullptr, xa.p, ya.p,
+            ctl.p, cur);
+        cuda_check(cudaGetLastError(), "restart");
+        refresh_activity(cur);
         if (halpern) {
             if (n)
                 cuda_check(cudaMemcpyAsync(anchor_x.p, x[cur].p, size_t(n) * 8,
@@ -891,9 +913,6 @@ struct Engine {
                                            cudaMemcpyDeviceToDevice, stream), "anchor ax");
             }
         }
-        zero_average();
-        sync_ctl();
-        host_ctl->cur = cur;
         host_ctl->pending = 0;
         host_ctl->mass = 0;
         if (halpern) {
@@ -904,35 +923,19 @@ struct Engine {
             host_ctl->lambda = 0;
             request_restart = false;
         }
-        push_ctl();
-        cuda_check(cudaStreamSynchronize(stream), "restart");
     }
 
     void reset_candidate(bool average) {
         flush();
-        sync_ctl();
-        int cur = host_ctl->cur;
-        if (average) {
-            if (n)
-                cuda_check(cudaMemcpyAsync(x[cur].p, xa.p, size_t(n) * 8, cudaMemcpyDeviceToDevice,
-                                           stream), "restart x");
-            if (m)
-                cuda_check(cudaMemcpyAsync(y[cur].p, ya.p, size_t(m) * 8, cudaMemcpyDeviceToDevice,
-                                           stream), "restart y");
-        }
-        refresh_y32(cur);
-        refresh_activity(cur);
-        restart_state(cur);
+        restart_state(average ? xa.p : nullptr, average ? ya.p : nullptr, false);
+        cuda_check(cudaStreamSynchronize(stream), "restart");
     }
 
     void reset(const double *hx, const double *hy) {
         sync_ctl();
-        int cur = host_ctl->cur;
-        upload_perm(x[cur].p, hx, n, col_perm, scratch_n, false);
-        upload_perm(y[cur].p, hy, m, row_perm, scratch_m, false);
-        refresh_y32(cur);
-        refresh_activity(cur);
-        restart_state(cur);
+        upload(scratch_n.p, hx, n);
+        upload(scratch_m.p, hy, m);
+        restart_state(scratch_n.p, scratch_m.p, true);
         cuda_check(cudaStreamSynchronize(stream), "reset"); // the caller may reuse hx, hy
     }
 
@@ -942,7 +945,7 @@ struct Engine {
             mon_aty.alloc(std::max<int64_t>(1, n));
             mon_qx.alloc(std::max<int64_t>(1, n));
             mon_part.alloc(size_t(5 * 148 * 8));
-            mon_out.alloc(1);
+            mon_out.alloc(2);
             mon_arrive.alloc(1);
             cuda_check(cudaMemsetAsync(mon_arrive.p, 0, sizeof(unsigned), stream), "monitor");
             std::vector<double> hc(static_cast<size_t>(n));
@@ -955,7 +958,8 @@ struct Engine {
         flush();
         sync_ctl();
         int cur = host_ctl->cur;
-        double best = INFINITY;
+        if (std::max(n, m) == 0)
+            return 0;
         for (int which = 0; which < 2; ++which) {
             const double *px = which ? xa.p : x[cur].p;
             const double *py = which ? ya.p : y[cur].p;
@@ -965,20 +969,17 @@ struct Engine {
                 spmv(At, py, mon_aty.p);
             if (sparse_q)
                 q_spmv(px, mon_qx.p);
-            if (std::max(n, m) == 0)
-                return 0;
             int g = grid_for(std::max(n, m));
             monitor_kernel<<<g, kThreads, 0, stream>>>(
                 n, m, px, py, mon_ax.p, mon_aty.p, sparse_q ? mon_qx.p : nullptr, c.p, q.p, lb.p,
-                ub.p, rl.p, ru.p, cscale, mon_part.p, mon_arrive.p, mon_out.p);
+                ub.p, rl.p, ru.p, cscale, mon_part.p, mon_arrive.p, mon_out.p + which);
             cuda_check(cudaGetLastError(), "monitor");
-            double r = 0;
-            cuda_check(cudaMemcpyAsync(&r, mon_out.p, 8, cudaMemcpyDeviceToHost, stream),
-                       "monitor result");
-            cuda_check(cudaStreamSynchronize(stream), "monitor sync");
-            best = std::min(best, r);
         }
-        return best;
+        double r[2] = {0, 0};
+        cuda_check(cudaMemcpyAsync(r, mon_out.p, 16, cudaMemcpyDeviceToHost, stream),
+                   "monitor result");
+        cuda_check(cudaStreamSynchronize(stream), "monitor sync");
+        return std::min(std::min(double(INFINITY), r[0]), r[1]);
     }
 
     // snapshot parts: x, y, xa, ya, ax, anchor_x, anchor_y, anchor_ax, control(11),
@@ -1084,6 +1085,7 @@ struct Engine {
         host_ctl->tau = tau;
         host_ctl->sigma = sigma;
         push_ctl();
+        ctl_known = false;
         for (auto &e : ev)
             cuda_check(cudaEventCreate(&e), "event");
         double tp = 0, td = 0, tk = 0;
@@ -1977,8 +1979,8 @@ Engine *create_engine(const nk_csr *Ah, const nk_csr *Qh, const double *hc, cons
     vec(E->ya, nullptr, m, rperm);
     vec(E->ax[0], nullptr, m, rperm);
     vec(E->ax[1], nullptr, m, rperm);
-    E->scratch_n.alloc(size_t(std::max<int64_t>(1, n)));
-    E->scratch_m.alloc(size_t(std::max<int64_t>(1, m)));
+    E->scratch_n.alloc(size_t(std::max<int64_t>(1, 2 * n)));
+    E->scratch_m.alloc(size_t(std::max<int64_t>(1, 2 * m)));
     if (o->precision == NK_PRECISION_FP32) {
         E->dx32.alloc(std::max<int64_t>(1, n));
         E->y32[0].alloc(std::max<int64_t>(1, m));
@@ -2032,6 +2034,7 @@ Engine *create_engine(const nk_csr *Ah, const nk_csr *Qh, const double *hc, cons
     init.flags = (E->adaptive ? 1 : 0) | (E->halpern ? 2 : 0) | (E->residual_restarts ? 4 : 0);
     *E->host_ctl = init;
     E->push_ctl();
+    E->ctl_known = true;
     E->refresh_y32(0);
     E->refresh_activity(0);
     if (E->halpern && m)
