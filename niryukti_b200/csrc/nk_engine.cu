@@ -69,7 +69,6 @@ struct SellMatrix {
     std::vector<int32_t> chunk_len; // host: padded length of each chunk
     DevBuf<int64_t> coff, clist;    // the fused kernels' per-CTA chunk lists
     int max_cta_items = 0;          // longest of those lists
-    std::vector<int64_t> hoff, hlist; // the lists on the host (the resident kernel's slots)
 
     // The view the fused trial kernels use: with the per-CTA chunk lists
     // (built for their persistent grid).
@@ -180,7 +179,7 @@ struct PanelMatrix {
 // The resident kernel's plan for a model (nk_resident.cuh).
 struct ResidentPlan {
     bool on = false;
-    int grid = 0;
+    int grid = 0, carveout = 100; // carveout: percent of the SM's shared memory
     unsigned tag = 1;
     size_t smem = 0;
     ResidentView view{};
@@ -311,7 +310,7 @@ void build_sell(SellMatrix &M, int64_t rows, int64_t cols, const std::vector<int
         cuda_check(cudaMemsetAsync(M.idx64.p, 0, M.idx64.bytes(), s), "sell idx");
     } else {
         M.idx32.alloc(total);
-        cuda_check(cudaMemsetAsync(M.idx32.p, 0, M.idx32.bytes(), s), "sell idx");
+        cuda_check(cudaMemsetAsync(M.idx32.p, 0xff, M.idx32.bytes(), s), "sell idx"); // -1: padding
     }
     if (vbits == 64) {
         M.val64.alloc(total);
@@ -661,9 +660,21 @@ struct Engine {
         unsigned tag = resident.tag;
         resident.tag += unsigned(count);
         void *args[] = {&at, &a, &q, &v, &resident.view, &count, &tag};
-        cuda_check(cudaLaunchCooperativeKernel(resident_function(), dim3(resident.grid),
-                                               dim3(kResThreads), args, resident.smem, stream),
-                   "trial launch");
+        // the shared memory that this model needs and no more: L1 holds what is not
+        // staged (the kernel's own limit is the largest model's)
+        cudaLaunchAttribute attr[2] = {};
+        attr[0].id = cudaLaunchAttributeCooperative;
+        attr[0].val.cooperative = 1;
+        attr[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+        attr[1].val.sharedMemCarveout = resident.carveout;
+        cudaLaunchConfig_t config = {};
+        config.gridDim = dim3(unsigned(resident.grid));
+        config.blockDim = dim3(kResThreads);
+        config.dynamicSmemBytes = resident.smem;
+        config.stream = stream;
+        config.attrs = attr;
+        config.numAttrs = 2;
+        cuda_check(cudaLaunchKernelExC(&config, resident_function(), args), "trial launch");
     }
     int vbits() const { return precision == NK_PRECISION_FP64 ? 64 : 32; }
 
@@ -1086,6 +1097,34 @@ struct Engine {
         host_ctl->sigma = sigma;
         push_ctl();
         ctl_known = false;
+        // where advance() runs resident trials, which add a long row's segments and
+        // not its panels' runs, the timed kernels work on a state that is put back
+        const bool replay = resident.on && panels;
+        std::vector<std::pair<double *, int64_t>> state;
+        DevBuf<double> kept;
+        DevBuf<Control> kept_ctl;
+        auto copy_state = [&](bool back) {
+            int64_t at = 0;
+            for (auto &[p, len] : state) {
+                if (len)
+                    cuda_check(cudaMemcpyAsync(back ? p : kept.p + at, back ? kept.p + at : p,
+                                               size_t(len) * 8, cudaMemcpyDeviceToDevice, stream),
+                               "profile state");
+                at += len;
+            }
+            cuda_check(cudaMemcpyAsync(back ? ctl.p : kept_ctl.p, back ? kept_ctl.p : ctl.p,
+                                       sizeof(Control), cudaMemcpyDeviceToDevice, stream),
+                       "profile state");
+        };
+        if (replay) {
+            for (auto *d : {&x[0], &x[1], &xa})
+                state.push_back({d->p, n});
+            for (auto *d : {&y[0], &y[1], &ax[0], &ax[1], &ya})
+                state.push_back({d->p, m});
+            kept.alloc(size_t(3 * n + 5 * m));
+            kept_ctl.alloc(1);
+            copy_state(false);
+        }
         for (auto &e : ev)
             cuda_check(cudaEventCreate(&e), "event");
         double tp = 0, td = 0, tk = 0;
@@ -1142,6 +1181,11 @@ struct Engine {
         for (auto &e : ev) {
             cudaEventDestroy(e);
             e = nullptr;
+        }
+        if (replay) {
+            copy_state(true);
+            for (int left = count; left > 0; left -= kResidentTrials)
+                launch_resident(std::min(left, kResidentTrials));
         }
         trials += count;
         sync_ctl();
@@ -1235,48 +1279,54 @@ std::vector<int64_t> lpt_assign(const std::vector<int64_t> &items, const std::ve
 
 // The schedule of `ids` (item k is ids[k], with memory work work[k]) onto
 // `ctas` persistent CTAs: longest-first list scheduling by memory work, then
-// each CTA's items costliest first (its warps claim them in that order).
-// Keeps and uploads M's per-CTA lists.
-void schedule_items(const std::vector<int64_t> &ids, const std::vector<int64_t> &work,
-                    int64_t ctas, SellMatrix &M, cudaStream_t s) {
+// each CTA's items costliest first (its warps claim them in that order).  CTA
+// b's items are list[off[b] .. off[b+1]).
+struct CtaLists {
+    std::vector<int64_t> off, list;
+    int longest = 0;
+};
+CtaLists schedule_items(const std::vector<int64_t> &ids, const std::vector<int64_t> &work,
+                        int64_t ctas) {
+    CtaLists S;
     const int64_t nit = int64_t(ids.size());
     ctas = std::max<int64_t>(1, ctas);
     std::vector<int64_t> all(static_cast<size_t>(nit)), cta(static_cast<size_t>(nit));
     for (int64_t k = 0; k < nit; ++k)
         all[size_t(k)] = k;
     const std::vector<int64_t> order = lpt_assign(all, work, ctas, cta); // costliest first
-    std::vector<int64_t> off(static_cast<size_t>(ctas + 1), 0);
+    S.off.assign(static_cast<size_t>(ctas + 1), 0);
     for (int64_t k = 0; k < nit; ++k)
-        ++off[size_t(cta[size_t(k)] + 1)];
-    int longest = 0;
+        ++S.off[size_t(cta[size_t(k)] + 1)];
     for (int64_t b = 0; b < ctas; ++b) {
-        longest = std::max(longest, int(off[size_t(b + 1)]));
-        off[size_t(b + 1)] += off[size_t(b)];
+        S.longest = std::max(S.longest, int(S.off[size_t(b + 1)]));
+        S.off[size_t(b + 1)] += S.off[size_t(b)];
     }
-    std::vector<int64_t> list(static_cast<size_t>(std::max<int64_t>(1, nit)), 0);
+    S.list.assign(static_cast<size_t>(std::max<int64_t>(1, nit)), 0);
     {
-        std::vector<int64_t> pos(off.begin(), off.end() - 1);
+        std::vector<int64_t> pos(S.off.begin(), S.off.end() - 1);
         for (int64_t k : order)
-            list[size_t(pos[size_t(cta[size_t(k)])]++)] = ids[size_t(k)];
+            S.list[size_t(pos[size_t(cta[size_t(k)])]++)] = ids[size_t(k)];
     }
     {   // every item exactly once
-        std::vector<int64_t> got(list.begin(), list.begin() + nit), want(ids);
+        std::vector<int64_t> got(S.list.begin(), S.list.begin() + nit), want(ids);
         std::sort(got.begin(), got.end());
         std::sort(want.begin(), want.end());
         if (got != want)
             throw Error(NK_ERR_INVALID, "internal: chunk schedule is not a permutation");
     }
-    upload_vector(M.coff, off, s);
-    upload_vector(M.clist, list, s);
-    M.max_cta_items = longest;
-    M.hoff = std::move(off);
-    M.hlist = std::move(list);
+    return S;
+}
+void use_schedule(SellMatrix &M, CtaLists S, cudaStream_t s) {
+    upload_vector(M.coff, S.off, s);
+    upload_vector(M.clist, S.list, s);
+    cuda_check(cudaStreamSynchronize(s), "schedule"); // S leaves scope
+    M.max_cta_items = S.longest;
 }
 
 // Memory work of a SELL chunk of padded length L (see above).
 int64_t chunk_work(int64_t L, bool split) { return 44 * L + (split ? 100 : 70); }
 
-void build_schedule(SellMatrix &M, int64_t ctas, cudaStream_t s) {
+CtaLists chunk_schedule(const SellMatrix &M, int64_t ctas) {
     const int64_t nch = int64_t(M.chunk_len.size());
     const int64_t split_chunks = M.nsv / 32;
     std::vector<int64_t> ids(static_cast<size_t>(nch)), work(ids.size());
@@ -1284,7 +1334,7 @@ void build_schedule(SellMatrix &M, int64_t ctas, cudaStream_t s) {
         ids[size_t(c)] = c;
         work[size_t(c)] = chunk_work(M.chunk_len[size_t(c)], c < split_chunks);
     }
-    schedule_items(ids, work, ctas, M, s);
+    return schedule_items(ids, work, ctas);
 }
 
 // The dual kernel's schedule when A's long rows take the panel path: the
@@ -1292,8 +1342,8 @@ void build_schedule(SellMatrix &M, int64_t ctas, cudaStream_t s) {
 // (encoded -k-1), whose lanes each read their row's run sums (roff: row i's
 // slots [roff[i], roff[i+1]); the warp waits for its row with the most) and
 // run the row epilogue.
-void build_dual_panel_schedule(SellMatrix &M, int64_t long_rows, const std::vector<int64_t> &roff,
-                               int64_t ctas, cudaStream_t s) {
+CtaLists dual_panel_schedule(const SellMatrix &M, int64_t long_rows,
+                             const std::vector<int64_t> &roff, int64_t ctas) {
     const int64_t nch = int64_t(M.chunk_len.size());
     const int64_t split_chunks = M.nsv / 32;
     const int64_t combine = (long_rows + 31) / 32;
@@ -1309,7 +1359,7 @@ void build_dual_panel_schedule(SellMatrix &M, int64_t long_rows, const std::vect
         ids.push_back(c);
         work.push_back(chunk_work(M.chunk_len[size_t(c)], false));
     }
-    schedule_items(ids, work, ctas, M, s);
+    return schedule_items(ids, work, ctas);
 }
 
 // Persistent grid: as many CTAs as fit on the device at once, at most one warp
@@ -1645,18 +1695,19 @@ std::vector<int> own_ranges(const std::vector<int32_t> &chunk_len, int parts) {
 }
 
 // Turns the resident kernel on (nk_resident.cuh) for a model that it can run as the
-// two-kernel path does, bit for bit: 32-bit indices, FP64 sums, no column panels,
-// no row split across chunks; and that fits: a CTA's products of
-// either matrix and its rows' state in shared memory (up to about 1.5 M entries).
-// Up to there it is the faster path, measured in us a trial on LPs with 6 entries
-// per column (FP64, adaptive), resident against two kernels: 5.5 / 14.6 at 4 k
-// entries, 6.6 / 16.6 at 54 k, 8.0 / 20.6 at 360 k, 12.6 / 22.6 at 720 k,
-// 18.7 / 26.7 at 1.2 M.
-void plan_resident(Engine &E, cudaStream_t s) {
+// kernel path does, bit for bit (with column panels, up to the rounding of the
+// long rows' sums): 32-bit indices, FP64 sums, no row split across chunks; and
+// that fits: a CTA's products of either matrix and its rows' state in shared
+// memory (up to about 1.5 M entries).  Up to there it is the faster path,
+// measured in us a trial on LPs with 6 entries per column (FP64, adaptive),
+// resident against two kernels: 5.5 / 14.6 at 4 k entries, 6.6 / 16.6 at 54 k,
+// 8.0 / 20.6 at 360 k, 12.6 / 22.6 at 720 k, 18.7 / 26.7 at 1.2 M.
+void plan_resident(Engine &E, const CtaLists &lists_t, const CtaLists &lists_a,
+                   const std::vector<int64_t> &rlen, cudaStream_t s) {
     ResidentPlan &P = E.resident;
     ResidentView &R = P.view;
-    if (E.wide || E.precision == NK_PRECISION_FP32 || E.panels || E.A.ncounters ||
-        E.At.ncounters || E.A.nv == 0 || E.At.nv == 0)
+    if (E.wide || E.precision == NK_PRECISION_FP32 || E.A.ncounters || E.At.ncounters ||
+        E.A.nv == 0 || E.At.nv == 0)
         return;
     const void *k = E.resident_function();
     int dev = 0, sms = 148, coop = 0, per = 0;
@@ -1689,6 +1740,25 @@ void plan_resident(Engine &E, cudaStream_t s) {
     R.entries_a = most(oa, E.A.chunk_len, R.rows);
     R.products = std::max(R.entries_t, R.entries_a);
     const size_t value = size_t(E.vbits() / 8), budget = smem_budget(k, 1);
+    int per_sm = 0;
+    cuda_check(cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev),
+               "shared memory per SM");
+    const size_t full = size_t(per_sm);
+    // y's hot entries: rows that every CTA's part of A^T names about once or more
+    // (32 entries spread over 147 CTAs pay for the copy of one), where together
+    // they hold a tenth of the entries; up to 4,096 (32 KB)
+    R.stage = 0;
+    R.hot = 0;
+    int64_t held = 0;
+    for (int64_t i = 0; i < std::min<int64_t>(E.m, 4096) && rlen[size_t(i)] >= 32; ++i) {
+        held += rlen[size_t(i)];
+        R.hot = int(i / 32 + 1) * 32;
+    }
+    R.hot = int(std::min<int64_t>(R.hot, E.m / 32 * 32));
+    if (10 * held < E.A.nnz)
+        R.hot = 0;
+    while (R.hot > 0 && resident_shared_bytes(R, value) > budget)
+        R.hot -= 32;
     R.stage = 2;
     while (R.stage > 0 && resident_shared_bytes(R, value) > budget)
         --R.stage;
@@ -1702,17 +1772,18 @@ void plan_resident(Engine &E, cudaStream_t s) {
                "resident occupancy");
     if (int64_t(per) * sms < P.grid)
         return;
+    P.carveout = int(std::min<size_t>(100, (100 * (P.smem + full - budget) + full - 1) / full));
     // each chunk's slot: its list of the two-kernel schedule and its place there
-    auto slots = [&](const SellMatrix &M, int lists, int &width) {
-        width = std::max(32, (M.max_cta_items + 31) / 32 * 32);
+    auto slots = [&](const SellMatrix &M, const CtaLists &S, int lists, int &width) {
+        width = std::max(32, (S.longest + 31) / 32 * 32);
         std::vector<int> slot(M.chunk_len.size(), 0);
         for (int q = 0; q < lists; ++q)
-            for (int64_t k = M.hoff[size_t(q)]; k < M.hoff[size_t(q + 1)]; ++k)
-                slot[size_t(M.hlist[size_t(k)])] = q * width + int(k - M.hoff[size_t(q)]);
+            for (int64_t k = S.off[size_t(q)]; k < S.off[size_t(q + 1)]; ++k)
+                slot[size_t(S.list[size_t(k)])] = q * width + int(k - S.off[size_t(q)]);
         return slot;
     };
-    const std::vector<int> st = slots(E.At, R.lists_p, R.width_p),
-                           sa = slots(E.A, R.lists_d, R.width_d);
+    const std::vector<int> st = slots(E.At, lists_t, R.lists_p, R.width_p),
+                           sa = slots(E.A, lists_a, R.lists_d, R.width_d);
     std::vector<int> lists;
     // Q's rows with entries, in ranges of about equal work
     std::vector<int> oq(size_t(P.grid) + 1, E.Q.nrows);
@@ -2007,18 +2078,23 @@ Engine *create_engine(const nk_csr *Ah, const nk_csr *Qh, const double *hc, cons
         E->wide ? configure<double, float, int64_t>(*E) : configure<double, float, int32_t>(*E);
     else
         E->wide ? configure<float, float, int64_t>(*E) : configure<float, float, int32_t>(*E);
-    build_schedule(E->At, E->grid_p, s);
-    if (E->panels)
-        build_dual_panel_schedule(E->A, E->pan.rows, E->pan.hroff, E->grid_d, s);
-    else
-        build_schedule(E->A, E->grid_d, s);
+    const CtaLists lists_t = chunk_schedule(E->At, E->grid_p),
+                   lists_a = chunk_schedule(E->A, E->grid_d);
+    use_schedule(E->At, lists_t, s);
+    use_schedule(E->A, E->panels ? dual_panel_schedule(E->A, E->pan.rows, E->pan.hroff, E->grid_d)
+                                 : lists_a, s);
     if (o->precision == NK_PRECISION_FP64)
         E->wide ? attach_slots<double, double, int64_t>(*E) : attach_slots<double, double, int32_t>(*E);
     else if (o->precision == NK_PRECISION_MIXED)
         E->wide ? attach_slots<double, float, int64_t>(*E) : attach_slots<double, float, int32_t>(*E);
     else
         E->wide ? attach_slots<float, float, int64_t>(*E) : attach_slots<float, float, int32_t>(*E);
-    plan_resident(*E, s);
+    {
+        std::vector<int64_t> engine_rlen(static_cast<size_t>(m)); // longest first
+        for (int64_t i = 0; i < m; ++i)
+            engine_rlen[size_t(i)] = rlen[size_t(rperm[size_t(i)])];
+        plan_resident(*E, lists_t, lists_a, engine_rlen, s);
+    }
     E->split_p.alloc(size_t(std::max(1, E->At.ncounters)));
     E->split_d.alloc(size_t(2 * std::max(1, E->A.ncounters)));
     cuda_check(cudaMemsetAsync(E->split_p.p, 0, E->split_p.bytes(), s), "split slots");

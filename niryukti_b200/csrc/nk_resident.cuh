@@ -14,6 +14,10 @@
 //     gathers in flight at once (through L2: other SMs write the vectors), and
 //     land in shared memory; then a lane adds its row's products in CSR order,
 //     so a row's sum is the sequential sum of the two-kernel path bit for bit;
+//   - y's leading entries -- the longest rows', which the entries of A^T name over
+//     and over -- are copied to shared memory once a trial: gathers of a few
+//     hot lines by every SM queue up in L2 (a 40,200 x 80,000 block-angular LP
+//     with 200 rows of 4,000 entries took 55 us a trial without the copy);
 //   - two grid barriers replace the launches of a trial: after the primal part
 //     (dx is complete) and after the dual part (y and the step rule's terms are);
 //   - the last CTA holds no rows.  It adds the step rule's terms in the order of
@@ -64,17 +68,18 @@ struct ResidentView {
     // shared memory: entries of the products, of A^T and of A, virtual columns
     // and rows (each the largest CTA's; columns and rows are multiples of 64)
     int products, entries_t, entries_a, cols, rows;
+    int hot;   // leading entries of y that a CTA copies for its gathers (a multiple of 32)
     int stage; // what is copied to shared memory: 0 the state, 1 also the bounds, 2 also the entries
     unsigned *sync; // [0] barrier arrivals, [1] CTAs done; zero between launches
 };
 
-// A CTA's dynamic shared memory: the products; per virtual column x twice, its
+// A CTA's dynamic shared memory: the products; y's hot entries; per virtual column x twice, its
 // average and (stage 1) c, lb, ub, q, per virtual row y twice, A x twice, y's
 // average and (stage 1) rl, ru, and their lengths; two ints per chunk; the
 // entries (stage 2).
 inline size_t resident_shared_bytes(const ResidentView &R, size_t value_bytes) {
     const size_t cols = size_t(R.cols), rows = size_t(R.rows);
-    return (size_t(R.products) + (R.stage ? 7 : 3) * cols + (R.stage ? 7 : 5) * rows) * 8 +
+    return (size_t(R.products) + size_t(R.hot) + (R.stage ? 7 : 3) * cols + (R.stage ? 7 : 5) * rows) * 8 +
            (cols + rows) * 4 + (cols + rows) / 32 * 8 +
            (R.stage == 2 ? (size_t(R.entries_t) + size_t(R.entries_a)) * (value_bytes + 4) : 0);
 }
@@ -109,22 +114,52 @@ __device__ __forceinline__ bool grid_barrier(unsigned *counter, unsigned k, Cont
     return wait_arrivals(counter, k * (gridDim.x - 1), ctl, ok);
 }
 
-// prod[e] = value * src[column] of the CTA's `count` entries (padding entries
-// give a product that no row reads).  ip and vp point to shared or global memory.
-template <class V>
+// src[j], from the copy of its first `hot` entries where it lies there, else
+// through L2.
+__device__ __forceinline__ double gather_hot(const double *src, unsigned copy, int j, int hot) {
+    double v;
+    asm("{\n\t"
+        ".reg .pred p;\n\t"
+        "setp.lt.s32 p, %3, %4;\n\t"
+        "@p ld.shared.f64 %0, [%1];\n\t"
+        "@!p ld.global.cg.f64 %0, [%2];\n\t"
+        "}"
+        : "=d"(v)
+        : "r"(copy + 8u * unsigned(j)), "l"(src + j), "r"(j), "r"(hot)
+        : "memory");
+    return v;
+}
+
+// prod[e] = value * src[column] of the CTA's `count` entries (column -1: padding,
+// which no row reads).  ip and vp point to shared or global memory.  HOT: src's
+// first `hot` entries are in shared memory at `copy`.
+template <bool HOT, class V>
 __device__ __forceinline__ void flat_products(const int32_t *ip, const V *vp, int count,
-                                              const double *src, double *prod) {
+                                              const double *src, double *prod, const double *copy,
+                                              int hot) {
     constexpr int U = 6, T = kResThreads;
+    const unsigned at = HOT ? unsigned(__cvta_generic_to_shared(copy)) : 0u;
     for (int e = threadIdx.x; e < count; e += U * T) {
+        int j[U]; // all columns before the first gather, all gathers before the first product
+        V w[U];
         double g[U];
 #pragma unroll
         for (int u = 0; u < U; ++u)
-            if (e + u * T < count)
-                g[u] = __ldcg(src + ip[e + u * T]);
+            if (e + u * T < count) {
+                j[u] = ip[e + u * T];
+                w[u] = vp[e + u * T];
+            } else
+                j[u] = -1;
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if constexpr (HOT)
+                g[u] = gather_hot(src, at, j[u] >= 0 ? j[u] : 0, hot);
+            else
+                g[u] = j[u] >= 0 ? __ldcg(src + j[u]) : 0.;
 #pragma unroll
         for (int u = 0; u < U; ++u)
             if (e + u * T < count)
-                prod[e + u * T] = double(vp[e + u * T]) * g[u];
+                prod[e + u * T] = double(w[u]) * g[u];
     }
 }
 
@@ -330,7 +365,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
     const int first_a = a0 * 32 - int(A.nsv) + int(A.nsr);
     // columns: x twice (the iterate's buffer by cur), its average; rows: y twice,
     // A x twice, y's average
-    double *sx = prod + R.products, *sxa = sx + 2 * R.cols, *sy = sxa + R.cols,
+    double *hot = prod + R.products, *sx = hot + R.hot, *sxa = sx + 2 * R.cols, *sy = sxa + R.cols,
            *sax = sy + 2 * R.rows, *sya = sax + 2 * R.rows, *bounds = sya + R.rows;
     // the bounds by local row, or (unstaged) from the global arrays by j - first_t
     // and i - first_a, which is the local row outside the split region
@@ -366,6 +401,17 @@ __global__ void __launch_bounds__(kResThreads, 1)
     }
     __syncthreads(); // the staged entries
     const double r = v.reflection;
+    // the products of A^T with y
+    auto products_t = [&](const double *y) {
+        if (R.hot == 0) {
+            flat_products<false>(ip_t, vp_t, tcount, y, prod, nullptr, 0);
+            return;
+        }
+        for (int k = threadIdx.x; k < R.hot; k += kResThreads)
+            hot[k] = __ldcg(y + k);
+        __syncthreads();
+        flat_products<true>(ip_t, vp_t, tcount, y, prod, hot, R.hot);
+    };
     {
         const double *x = c.cur ? v.x1 : v.x0, *y = c.cur ? v.y1 : v.y0,
                      *ax = c.cur ? v.ax1 : v.ax0;
@@ -405,7 +451,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
             at_a[k] = int(A.cptr[a0 + k] - abase);
             slot_a[k] = R.slot_a[a0 + k];
         }
-        flat_products(ip_t, vp_t, tcount, y, prod);
+        products_t(y);
     }
     // the sum of column l's products (a split region's segment), from c_l
     auto row_sum = [&](int k) {
@@ -430,6 +476,9 @@ __global__ void __launch_bounds__(kResThreads, 1)
             double *gxt = cur ? v.x0 : v.x1;
             auto finish = [&](int l, int j, double g) -> double {
                 const int o = staged ? l : j - first_t;
+                // Halpern's vectors are in global memory: both loads go out first
+                const double last = HALPERN && unsaved ? R.last_x[j] : 0.,
+                             anchor = HALPERN ? v.anchor_x[j] : 0.;
                 const double xj = sx[co + l], lj = blb[o], uj = bub[o], aj = sxa[l];
                 const double qj = bq ? bq[o] : 0.;
                 if constexpr (QP)
@@ -446,9 +495,9 @@ __global__ void __launch_bounds__(kResThreads, 1)
                 double xn = T;
                 if (HALPERN) {
                     if (unsaved)
-                        sxa[l] = R.last_x[j];
+                        sxa[l] = last;
                     R.last_x[j] = T;
-                    xn = lam * v.anchor_x[j] + (1 - lam) * ((1 + r) * T - r * xj);
+                    xn = lam * anchor + (1 - lam) * ((1 + r) * T - r * xj);
                 }
                 sx[to + l] = xn;
                 if constexpr (QP)
@@ -489,13 +538,16 @@ __global__ void __launch_bounds__(kResThreads, 1)
                     __stcg(qxt + Q.rows[row], s);
             }
         }
-        flat_products(ip_a, vp_a, acount, v.dx, prod);
+        flat_products<false>(ip_a, vp_a, acount, v.dx, prod, nullptr, 0);
         double *gyt = cur ? v.y0 : v.y1;
         {
             const double sigma = c.sigma * c.factor;
             const int co = cur ? R.rows : 0, to = cur ? 0 : R.rows;
             auto finish = [&](int l, int i, double delta, double &dy2, double &cpl) {
                 const int o = staged ? l : i - first_a;
+                const double last = HALPERN && unsaved ? R.last_y[i] : 0.,
+                             anchor = HALPERN ? v.anchor_y[i] : 0.,
+                             anchor_ax = HALPERN ? v.anchor_ax[i] : 0.;
                 const double yi = sy[co + l], axi = sax[co + l], rli = brl[o], rui = bru[o],
                              ai = sya[l];
                 const double bar = axi + 2 * delta;
@@ -506,10 +558,10 @@ __global__ void __launch_bounds__(kResThreads, 1)
                     sya[l] = ai + (yi - ai) * pw;
                 if (HALPERN) {
                     if (unsaved)
-                        sya[l] = R.last_y[i];
+                        sya[l] = last;
                     R.last_y[i] = T;
-                    yn = lam * v.anchor_y[i] + (1 - lam) * ((1 + r) * T - r * yi);
-                    axn = lam * v.anchor_ax[i] + (1 - lam) * ((1 + r) * axn - r * axi);
+                    yn = lam * anchor + (1 - lam) * ((1 + r) * T - r * yi);
+                    axn = lam * anchor_ax + (1 - lam) * ((1 + r) * axn - r * axi);
                 }
                 __stcg(gyt + i, yn);
                 sy[to + l] = yn;
@@ -551,7 +603,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
         // -------------------------------------------------- decision
         const bool more = t + 1 < trials;
         if (more) { // the next trial's products and sums, should this one be accepted
-            flat_products(ip_t, vp_t, tcount, gyt, prod);
+            products_t(gyt);
             __syncthreads();
             g0 = warp < nt ? row_sum(warp) : 0.;
         }
@@ -595,7 +647,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
             return;
         unsaved = HALPERN && c.accept != 0;
         if (more && c.accept == 0) { // rejected: the products with the unchanged y
-            flat_products(ip_t, vp_t, tcount, cur ? v.y1 : v.y0, prod);
+            products_t(cur ? v.y1 : v.y0);
             __syncthreads();
             g0 = warp < nt ? row_sum(warp) : 0.;
         }
