@@ -90,4 +90,18 @@ template <class T> struct DevBuf {
     size_t bytes() const { return n * sizeof(T); }
 };
 
+// One device allocation cut into 256-byte aligned parts, for the entry points that
+// allocate on every call: first add() every part, then alloc(), then at().
+struct DevParts {
+    DevBuf<unsigned char> mem;
+    size_t total = 0;
+    template <class T> size_t add(size_t count) {
+        const size_t here = total;
+        total += (count * sizeof(T) + 255) & ~size_t(255);
+        return here;
+    }
+    void alloc() { mem.alloc(total); }
+    template <class T> T *at(size_t offset) const { return reinterpret_cast<T *>(mem.p + offset); }
+};
+
 } // namespace nk

@@ -2,12 +2,21 @@
 // src/cuda.cu:1304-1434; caller src/barrier.cpp:280-300).  The optimizer logic
 // stays with the reference's barrier.cpp; this solves K x = b on the GPU.
 //
-// Every vector and every scalar of the iteration lives on the device: the dot
-// products are two-stage fixed-tree reductions, and the step scalars (rho,
-// alpha, omega, beta) are formed by a one-thread kernel in the reference's
-// expressions and order, so nothing but a four-flag status crosses PCIe per
-// iteration.  The operator is CSR, one warp per row (lane-strided entries, a
-// fixed shuffle tree), with FP64 or FP32 values and FP64 vectors and sums.
+// The systems are small (tens of thousands of unknowns, a few entries a row), so
+// an iteration is latency: as separate launches (two products, five dots in two
+// stages, the vector updates and one-thread scalar steps: 26 of them, and one
+// read of the state) it took about 75 us.  One cooperative kernel runs the
+// iterations instead.  A thread owns element e of every vector, a CTA 256
+// consecutive ones, and the rows of K with them, so a product and its dot need
+// no exchange; what is left are five grid barriers an iteration, each with one
+// or two reductions: CTA partials, which every CTA adds up for itself in one
+// fixed order, and with them forms the step scalars in the reference's
+// expressions and order.  Vectors that others gather (y and z) go through L2.
+// A call on a saddle point of 24,000 unknowns and 184 k entries, with its uploads
+// and allocations: 5.9 ms before, 1.7 ms now (one allocation, too).
+//
+// The grid is resident (cooperative launch) and its waits are bounded; a CTA
+// that gives up sets NewtonState::fault.
 // Included by nk_engine.cu.
 #pragma once
 #include "nk_common.cuh"
@@ -20,185 +29,328 @@
 namespace nk {
 
 struct NewtonState {
-    double rho, previous, alpha, omega, beta, divisor, ss, tt, ts, rr, target;
+    double rho, previous, alpha, omega, target;
     int stop;      // 0 running, 1 converged, 2 breakdown
     int converged; // 1 once a residual met the target
+    int fault;     // a wait was given up
 };
 
+constexpr int kNewtonChunk = 64;          // iterations of one launch
+constexpr int kNewtonMaxPolls = 4 << 20;  // seconds: the barrier's bound
+
+template <class V> struct NewtonView {
+    int64_t n;
+    const int64_t *ptr, *idx;
+    const V *val;
+    const double *rhs, *dinv;
+    double *x, *r, *p, *v, *s, *t, *y, *z;
+    double *part;   // two sums per CTA, for each of the iteration's barriers in turn
+    unsigned *sync; // [0] arrivals, [1] CTAs done; zero between launches
+    NewtonState *st;
+    double tolerance;
+    int iterations, first; // of this launch; first: form r, rho and the target
+};
+
+// Row `base + lane`'s product with x, for the warp's 32 rows: 8, 16 or 32 lanes a
+// row (the warp's longest row decides), lane-strided, then a fixed shuffle tree.
+// A row's sum is the 32-lane one whatever the width: the other lanes would add
+// zeros.  Loads of four turns are in flight together.
 template <class V>
-__global__ void newton_spmv(int64_t n, const int64_t *__restrict__ ptr,
-                            const int64_t *__restrict__ idx, const V *__restrict__ val,
-                            const double *__restrict__ x, double *__restrict__ y,
-                            const NewtonState *st) {
-    if (st->stop)
-        return;
+__device__ __forceinline__ double newton_rows(const NewtonView<V> &K, int64_t base, const double *x) {
     const int lane = threadIdx.x & 31;
-    const int64_t first = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    const int64_t stride = (int64_t(gridDim.x) * blockDim.x) >> 5;
-    for (int64_t r = first; r < n; r += stride) {
-        double acc = 0;
-        for (int64_t k = ptr[r] + lane; k < ptr[r + 1]; k += 32)
-            acc += double(val[k]) * x[idx[k]];
+    const int64_t row = base + lane, start = K.ptr[base < K.n ? base : K.n];
+    const int at = row < K.n ? int(K.ptr[row] - start) : 0;
+    const int len = row < K.n ? int(K.ptr[row + 1] - start) - at : 0;
+    const int top = __reduce_max_sync(0xffffffffu, len);
+    const int L = top <= 8 ? 8 : top <= 16 ? 16 : 32, per = 32 / L; // lanes a row, rows a turn
+    constexpr int U = 4;
+    double mine = 0;
+    for (int it0 = 0; it0 < L; it0 += U) {
+        int64_t j[U];
+        double w[U], acc[U];
+        int rest[U], from[U];
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1)
-            acc += __shfl_xor_sync(0xffffffffu, acc, off);
-        if (lane == 0)
-            y[r] = acc;
+        for (int u = 0; u < U; ++u) {
+            const int q = (it0 + u) * per + lane / L, k = lane % L;
+            from[u] = __shfl_sync(0xffffffffu, at, q) + k;
+            rest[u] = __shfl_sync(0xffffffffu, len, q) - k;
+            j[u] = rest[u] > 0 ? K.idx[start + from[u]] : -1;
+            w[u] = rest[u] > 0 ? double(K.val[start + from[u]]) : 0.;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            acc[u] = j[u] >= 0 ? 0. + w[u] * __ldcg(x + j[u]) : 0.;
+        if (top > 32)
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                for (int k = 32; k < rest[u]; k += 32)
+                    acc[u] += double(K.val[start + from[u] + k]) *
+                              __ldcg(x + K.idx[start + from[u] + k]);
+        for (int off = L / 2; off > 0; off >>= 1)
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                acc[u] += __shfl_xor_sync(0xffffffffu, acc[u], off);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const double total = __shfl_sync(0xffffffffu, acc[u], (lane % per) * L);
+            if (lane / per == it0 + u)
+                mine = total;
+        }
     }
+    return mine;
 }
 
-// part[block] = sum of a[j] * b[j] over the block's grid-stride share
-__global__ void newton_dot_partial(int64_t n, const double *__restrict__ a,
-                                   const double *__restrict__ b, double *__restrict__ part,
-                                   const NewtonState *st) {
-    __shared__ double red[kWarps];
-    if (st->stop)
-        return; // block-uniform
-    double v = 0;
-    const int64_t stride = int64_t(gridDim.x) * blockDim.x;
-    for (int64_t j = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; j < n; j += stride)
-        v += a[j] * b[j];
-    double t[1] = {v};
-    cta_sum<1>(t, red);
-    if (threadIdx.x == 0)
-        part[blockIdx.x] = t[0];
-}
-// *out = sum of part[0 .. blocks) in a fixed order
-__global__ void newton_dot_finish(int blocks, const double *__restrict__ part, double *out,
-                                  const NewtonState *st) {
-    __shared__ double red[kWarps];
-    if (st->stop)
-        return;
-    double v = 0;
-    for (int b = threadIdx.x; b < blocks; b += blockDim.x)
-        v += part[b];
-    double t[1] = {v};
-    cta_sum<1>(t, red);
-    if (threadIdx.x == 0)
-        *out = t[0];
+// Grid barrier; false when the wait was given up.  What the CTA wrote before it
+// is released; what others wrote is read through L2.
+template <class V>
+__device__ __forceinline__ bool newton_barrier(const NewtonView<V> &K, unsigned *barrier, int *ok) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(K.sync) : "memory");
+        const unsigned need = ++*barrier * gridDim.x;
+        unsigned seen;
+        int polls = 0;
+        do {
+            asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(K.sync) : "memory");
+        } while (seen < need && ++polls < kNewtonMaxPolls);
+        if (seen < need) {
+            *ok = 0;
+            atomicExch(&K.st->fault, 1);
+        }
+    }
+    __syncthreads();
+    return *ok != 0;
 }
 
-// The iteration's scalar steps, one thread; `step` says which point of the
-// iteration has been reached (the reference's host statements in order).
-__global__ void newton_scalars(NewtonState *s, int step) {
-    if (s->stop)
-        return;
-    switch (step) {
-    case 0: // rho known: breakdown test, beta
-        if (!isfinite(s->rho) || fabs(s->rho) < 1e-300 || fabs(s->omega) < 1e-300) {
-            s->stop = 2;
-            return;
-        }
-        s->beta = (s->rho / s->previous) * (s->alpha / s->omega);
-        break;
-    case 1: // divisor known: alpha
-        if (!isfinite(s->divisor) || fabs(s->divisor) < 1e-300) {
-            s->stop = 2;
-            return;
-        }
-        s->alpha = s->rho / s->divisor;
-        break;
-    case 2: // ss known: early exit on s (x is updated by the caller's kernel)
-        if (sqrt(s->ss) <= s->target) {
-            s->converged = 1;
-            s->stop = 3; // x += alpha p still to do, then stop
-        }
-        break;
-    case 3: // tt, ts known: omega
-        if (!isfinite(s->tt) || s->tt < 1e-300) {
-            s->stop = 2;
-            return;
-        }
-        s->omega = s->ts / s->tt;
-        break;
-    case 4: // rr known
-        s->converged = sqrt(s->rr) <= s->target;
-        if (s->converged)
-            s->stop = 1;
-        s->previous = s->rho;
-        break;
+// Grid-wide sums of (a, b) in every thread: CTA trees, a barrier, and the CTAs'
+// sums added by every CTA in one order.  `turn` picks the partials' place.
+template <class V>
+__device__ __forceinline__ bool newton_sum(const NewtonView<V> &K, int turn, unsigned *barrier,
+                                           double (&ab)[2], double *red, double *out, int *ok) {
+    double *part = K.part + size_t(turn) * 2 * gridDim.x;
+    cta_sum<2>(ab, red);
+    if (threadIdx.x == 0) {
+        __stcg(part + 2 * blockIdx.x, ab[0]);
+        __stcg(part + 2 * blockIdx.x + 1, ab[1]);
     }
+    if (!newton_barrier(K, barrier, ok))
+        return false;
+    ab[0] = ab[1] = 0;
+    for (unsigned b = threadIdx.x; b < gridDim.x; b += kThreads) {
+        ab[0] += __ldcg(part + 2 * b);
+        ab[1] += __ldcg(part + 2 * b + 1);
+    }
+    cta_sum<2>(ab, red);
+    if (threadIdx.x == 0) {
+        out[0] = ab[0];
+        out[1] = ab[1];
+    }
+    __syncthreads();
+    ab[0] = out[0];
+    ab[1] = out[1];
+    return true;
 }
 
-// out = ca a + cb b + cc c with the coefficients of `which` (the reference's
-// linear_combine calls): 0 p = r + beta p - beta omega v; 1 s = r - alpha v;
-// 2 x = x + alpha p (exit on s); 3 x = x + alpha p + omega s; 4 r = s - omega t.
-__global__ void newton_combine(int64_t n, double *out, const double *a, const double *b,
-                               const double *c, NewtonState *st, int which) {
-    const int stop = st->stop;
-    if (which == 2 ? stop != 3 : stop != 0)
-        return;
-    double ca = 1, cb = 0, cc = 0;
-    switch (which) {
-    case 0: cb = st->beta; cc = -st->beta * st->omega; break;
-    case 1: cb = -st->alpha; break;
-    case 2: cb = st->alpha; break;
-    case 3: cb = st->alpha; cc = st->omega; break;
-    default: cb = -st->omega; break;
+template <class V>
+__global__ void __launch_bounds__(kThreads, 4) newton_kernel(NewtonView<V> K) {
+    __shared__ double red[kWarps * 2], sums[2];
+    __shared__ unsigned barrier; // thread 0's count
+    __shared__ int ok;
+    const int64_t n = K.n, first = int64_t(blockIdx.x) * kThreads + threadIdx.x,
+                  stride = int64_t(gridDim.x) * kThreads;
+    const int64_t tops = (n + 31) / 32 * 32; // whole warps for the row products
+    if (threadIdx.x == 0) {
+        barrier = 0;
+        ok = 1;
     }
-    const int64_t stride = int64_t(gridDim.x) * blockDim.x;
-    for (int64_t j = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; j < n; j += stride)
-        out[j] = ca * a[j] + cb * b[j] + cc * c[j];
-}
-// out = dinv * in (the right preconditioner), while the iteration runs
-__global__ void newton_scale(int64_t n, double *__restrict__ out, const double *__restrict__ dinv,
-                             const double *__restrict__ in, const NewtonState *st) {
-    if (st->stop)
-        return;
-    const int64_t stride = int64_t(gridDim.x) * blockDim.x;
-    for (int64_t j = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; j < n; j += stride)
-        out[j] = dinv[j] * in[j];
-}
-__global__ void newton_mark_done(NewtonState *st) {
-    if (st->stop == 3)
-        st->stop = 1;
+    __syncthreads();
+    double rho, previous = 1, alpha = 1, omega = 1, target;
+    int stop = 0, converged = 0, it = 0;
+    auto leave = [&] {
+        if (threadIdx.x != 0)
+            return;
+        if (blockIdx.x == 0) {
+            K.st->rho = rho;
+            K.st->previous = previous;
+            K.st->alpha = alpha;
+            K.st->omega = omega;
+            K.st->target = target;
+            K.st->stop = stop;
+            K.st->converged = converged;
+        }
+        if (atomicAdd(K.sync + 1, 1u) == gridDim.x - 1) { // the last CTA out
+            K.sync[0] = 0;
+            K.sync[1] = 0;
+        }
+    };
+    if (K.first) {
+        double ab[2] = {0, 0};
+        for (int64_t e = first; e < n; e += stride) {
+            const double b = K.rhs[e];
+            K.x[e] = K.p[e] = K.v[e] = 0;
+            K.r[e] = b;
+            ab[0] += b * b;
+        }
+        if (!newton_sum(K, 0, &barrier, ab, red, sums, &ok))
+            return;
+        const double norm = sqrt(ab[0]);
+        rho = ab[0]; // the shadow residual is rhs too
+        target = K.tolerance * (1 + norm);
+        converged = norm <= target;
+        stop = converged;
+    } else {
+        rho = K.st->rho;
+        previous = K.st->previous;
+        alpha = K.st->alpha;
+        omega = K.st->omega;
+        target = K.st->target;
+    }
+    for (; !stop && it < K.iterations; ++it) {
+        if (!isfinite(rho) || fabs(rho) < 1e-300 || fabs(omega) < 1e-300) {
+            stop = 2;
+            break;
+        }
+        const double beta = (rho / previous) * (alpha / omega);
+        // p = r + beta p - beta omega v, y = M^-1 p
+        for (int64_t e = first; e < n; e += stride) {
+            const double p = 1. * K.r[e] + beta * K.p[e] + (-beta * omega) * K.v[e];
+            K.p[e] = p;
+            __stcg(K.y + e, K.dinv[e] * p);
+        }
+        if (!newton_barrier(K, &barrier, &ok)) // y is complete
+            return;
+        // v = K y, <shadow, v>
+        double ab[2] = {0, 0};
+        for (int64_t e = first; e < tops; e += stride) {
+            const double v = newton_rows(K, e - (threadIdx.x & 31), K.y);
+            if (e < n) {
+                K.v[e] = v;
+                ab[0] += K.rhs[e] * v;
+            }
+        }
+        if (!newton_sum(K, 1, &barrier, ab, red, sums, &ok))
+            return;
+        if (!isfinite(ab[0]) || fabs(ab[0]) < 1e-300) {
+            stop = 2;
+            break;
+        }
+        alpha = rho / ab[0];
+        // s = r - alpha v, z = M^-1 s, <s, s>
+        ab[0] = ab[1] = 0;
+        for (int64_t e = first; e < n; e += stride) {
+            const double v = K.v[e], s = 1. * K.r[e] + (-alpha) * v + 0. * v;
+            K.s[e] = s;
+            __stcg(K.z + e, K.dinv[e] * s);
+            ab[0] += s * s;
+        }
+        if (!newton_sum(K, 2, &barrier, ab, red, sums, &ok))
+            return;
+        if (sqrt(ab[0]) <= target) { // converged on s: x = x + alpha y
+            for (int64_t e = first; e < n; e += stride) {
+                const double y = K.y[e];
+                K.x[e] = 1. * K.x[e] + alpha * y + 0. * y;
+            }
+            converged = 1;
+            stop = 1;
+            break;
+        }
+        // t = K z, <t, t>, <t, s>
+        ab[0] = ab[1] = 0;
+        for (int64_t e = first; e < tops; e += stride) {
+            const double t = newton_rows(K, e - (threadIdx.x & 31), K.z);
+            if (e < n) {
+                K.t[e] = t;
+                ab[0] += t * t;
+                ab[1] += t * K.s[e];
+            }
+        }
+        if (!newton_sum(K, 3, &barrier, ab, red, sums, &ok))
+            return;
+        if (!isfinite(ab[0]) || ab[0] < 1e-300) {
+            stop = 2;
+            break;
+        }
+        omega = ab[1] / ab[0];
+        // x = x + alpha y + omega z, r = s - omega t, <r, r> and the next <shadow, r>
+        ab[0] = ab[1] = 0;
+        for (int64_t e = first; e < n; e += stride) {
+            const double t = K.t[e], r = 1. * K.s[e] + (-omega) * t + 0. * t;
+            K.x[e] = 1. * K.x[e] + alpha * K.y[e] + omega * K.z[e];
+            K.r[e] = r;
+            ab[0] += r * r;
+            ab[1] += K.rhs[e] * r;
+        }
+        if (!newton_sum(K, 4, &barrier, ab, red, sums, &ok))
+            return;
+        converged = sqrt(ab[0]) <= target;
+        stop = converged;
+        previous = rho;
+        rho = ab[1];
+    }
+    leave();
 }
 
 // Diagonal right preconditioner of a Newton matrix, 1 / (its scale) per row:
 // |K_ii| where the diagonal carries the row; where it does not (a saddle
 // point's regularised zero block, |K_ii| < 1e-8 max_j |K_ij|), the diagonal of
 // the row's Schur complement, sum_j K_ij^2 / |K_jj| over the other entries.
-// Rows with neither keep 1.
-inline std::vector<double> newton_diagonal(const nk_csr &K) {
-    const int64_t n = K.rows;
-    std::vector<double> diag(static_cast<size_t>(n), 0.0), big(static_cast<size_t>(n), 0.0),
-        dinv(static_cast<size_t>(n), 1.0);
-    for (int64_t i = 0; i < n; ++i)
-        for (int64_t k = K.ptr[i]; k < K.ptr[i + 1]; ++k) {
-            big[size_t(i)] = std::max(big[size_t(i)], std::fabs(K.value[k]));
-            if (K.index[k] == i)
-                diag[size_t(i)] += K.value[k];
+// Rows with neither keep 1.  Two passes, a thread per row: the diagonals and
+// whether they carry their rows (diag: 0 where not), then the scales.
+__global__ void newton_diagonal(int64_t n, const int64_t *__restrict__ ptr,
+                                const int64_t *__restrict__ idx, const double *__restrict__ val,
+                                double *__restrict__ diag) {
+    const int64_t stride = int64_t(gridDim.x) * blockDim.x;
+    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
+        double d = 0, big = 0;
+        for (int64_t k = ptr[i]; k < ptr[i + 1]; ++k) {
+            const double a = fabs(val[k]);
+            big = big < a ? a : big;
+            if (idx[k] == i)
+                d += val[k];
         }
-    auto carries = [&](int64_t i) {
-        return std::fabs(diag[size_t(i)]) >= 1e-8 * big[size_t(i)] && diag[size_t(i)] != 0;
-    };
-    for (int64_t i = 0; i < n; ++i) {
-        if (carries(i)) {
-            dinv[size_t(i)] = 1 / std::fabs(diag[size_t(i)]);
-            continue;
-        }
-        double schur = 0;
-        for (int64_t k = K.ptr[i]; k < K.ptr[i + 1]; ++k) {
-            const int64_t j = K.index[k];
-            if (j != i && carries(j))
-                schur += K.value[k] * K.value[k] / std::fabs(diag[size_t(j)]);
-        }
-        if (schur > 0 && std::isfinite(schur))
-            dinv[size_t(i)] = 1 / schur;
+        diag[i] = fabs(d) >= 1e-8 * big ? d : 0.;
     }
-    return dinv;
+}
+__global__ void newton_scales(int64_t n, const int64_t *__restrict__ ptr,
+                              const int64_t *__restrict__ idx, const double *__restrict__ val,
+                              const double *__restrict__ diag, double *__restrict__ dinv) {
+    const int64_t stride = int64_t(gridDim.x) * blockDim.x;
+    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
+        double out = 1;
+        if (diag[i] != 0)
+            out = 1 / fabs(diag[i]);
+        else {
+            double schur = 0;
+            for (int64_t k = ptr[i]; k < ptr[i + 1]; ++k) {
+                const int64_t j = idx[k];
+                if (j != i && diag[j] != 0)
+                    schur += val[k] * val[k] / fabs(diag[j]);
+            }
+            if (schur > 0 && isfinite(schur))
+                out = 1 / schur;
+        }
+        dinv[i] = out;
+    }
+}
+__global__ void newton_ones(int64_t n, double *dinv) {
+    const int64_t stride = int64_t(gridDim.x) * blockDim.x;
+    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride)
+        dinv[i] = 1;
 }
 
 // Solves K x = rhs (K: n x n CSR, host arrays) by BiCGSTAB, right-preconditioned
-// by newton_diagonal when `precondition` (without it, the iteration is the
+// by newton_scales when `precondition` (without it, the iteration is the
 // reference's one exactly: every scaling is by 1).  The residual r stays the
 // unpreconditioned one, so the stopping test is the reference's.  Returns true
 // when a residual met the target ((fp32 ? 1e-6 : 1e-10) (1 + |rhs|)) before
-// breakdown, the iteration cap (min(20000, 10 n + 100)) or the time limit; x
-// gets the last iterate either way.  The arguments are checked by the caller.
-inline bool newton_solve(const nk_csr &K, const double *rhs, bool fp32, bool precondition,
-                         double time_limit, double *x_out, bool *timed_out) {
+// breakdown, the iteration cap (min(20000, 10 n + 100)) or the time limit
+// (looked at before every launch of kNewtonChunk iterations); x gets the last
+// iterate either way.  The arguments are checked by the caller.
+template <class V>
+inline bool newton_solve_t(const nk_csr &K, const double *rhs, bool precondition, double time_limit,
+                           double *x_out, bool *timed_out) {
     const int64_t n = K.rows, nnz = K.ptr[K.rows];
+    constexpr bool fp32 = sizeof(V) == 4;
     *timed_out = false;
     cudaStream_t s = nullptr;
     cuda_check(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "Newton stream");
@@ -210,102 +362,97 @@ inline bool newton_solve(const nk_csr &K, const double *rhs, bool fp32, bool pre
         }
     } guard_stream{s};
     const size_t nn = size_t(n), nz = size_t(std::max<int64_t>(1, nnz));
-    DevBuf<int64_t> dptr(nn + 1), didx(nz);
-    DevBuf<double> val64(fp32 ? 1 : nz);
-    DevBuf<float> val32(fp32 ? nz : 1);
-    DevBuf<double> x(nn), r(nn), anchor(nn), p(nn), v(nn), sv(nn), t(nn), y(nn), z(nn), dinv(nn);
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
+    int dev = 0, sms = 148, per = 0;
+    cuda_check(cudaGetDevice(&dev), "device");
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int vgrid = int(std::max<int64_t>(1, std::min<int64_t>((n + kThreads - 1) / kThreads,
-                                                                 int64_t(sms) * 4)));
-    const int mgrid = int(std::max<int64_t>(1, std::min<int64_t>((n + kWarps - 1) / kWarps,
-                                                                 int64_t(sms) * 8)));
-    DevBuf<double> part(static_cast<size_t>(vgrid));
-    DevBuf<NewtonState> st(1);
-    cuda_check(cudaMemcpyAsync(dptr.p, K.ptr, (nn + 1) * 8, cudaMemcpyHostToDevice, s), "Newton ptr");
-    if (nnz) {
-        cuda_check(cudaMemcpyAsync(didx.p, K.index, size_t(nnz) * 8, cudaMemcpyHostToDevice, s),
-                   "Newton idx");
-        if (fp32) {
-            std::vector<float> f(K.value, K.value + nnz);
-            cuda_check(cudaMemcpyAsync(val32.p, f.data(), size_t(nnz) * 4, cudaMemcpyHostToDevice, s),
-                       "Newton values");
-            cuda_check(cudaStreamSynchronize(s), "Newton values"); // f leaves scope
-        } else
-            cuda_check(cudaMemcpyAsync(val64.p, K.value, size_t(nnz) * 8, cudaMemcpyHostToDevice, s),
-                       "Newton values");
-    }
-    const std::vector<double> hdinv =
-        precondition ? newton_diagonal(K) : std::vector<double>(nn, 1.0);
-    cuda_check(cudaMemcpyAsync(dinv.p, hdinv.data(), nn * 8, cudaMemcpyHostToDevice, s),
-               "Newton preconditioner");
-    cuda_check(cudaMemcpyAsync(r.p, rhs, nn * 8, cudaMemcpyHostToDevice, s), "Newton rhs");
-    cuda_check(cudaMemcpyAsync(anchor.p, rhs, nn * 8, cudaMemcpyHostToDevice, s), "Newton rhs");
-    for (double *z : {x.p, p.p, v.p})
-        cuda_check(cudaMemsetAsync(z, 0, nn * 8, s), "Newton zero");
-    NewtonState h{};
-    h.previous = h.alpha = h.omega = 1;
-    cuda_check(cudaMemcpyAsync(st.p, &h, sizeof(h), cudaMemcpyHostToDevice, s), "Newton state");
-    auto dot = [&](const double *a, const double *b, double *out) {
-        newton_dot_partial<<<vgrid, kThreads, 0, s>>>(n, a, b, part.p, st.p);
-        newton_dot_finish<<<1, kThreads, 0, s>>>(vgrid, part.p, out, st.p);
+    cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, newton_kernel<V>, kThreads, 0),
+               "Newton occupancy");
+    const int grid = int(std::max<int64_t>(
+        1, std::min<int64_t>((n + kThreads - 1) / kThreads, int64_t(sms) * std::min(4, per))));
+    constexpr int kTurns = 5;
+    DevParts mem;
+    const size_t optr = mem.add<int64_t>(nn + 1), oidx = mem.add<int64_t>(nz),
+                 oval = mem.add<double>(nz), oval32 = mem.add<float>(fp32 ? nz : 0),
+                 orhs = mem.add<double>(nn), ovec = mem.add<double>(10 * nn),
+                 opart = mem.add<double>(size_t(kTurns) * 2 * size_t(grid)),
+                 ostate = mem.add<NewtonState>(1), osync = mem.add<unsigned>(2);
+    mem.alloc();
+    int64_t *dptr = mem.at<int64_t>(optr), *didx = mem.at<int64_t>(oidx);
+    double *dval = mem.at<double>(oval), *vec = mem.at<double>(ovec);
+    auto up = [&](void *d, const void *h, size_t bytes) {
+        if (bytes)
+            cuda_check(cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, s), "Newton upload");
     };
-    auto multiply = [&](const double *in, double *out) {
-        if (fp32)
-            newton_spmv<float><<<mgrid, kThreads, 0, s>>>(n, dptr.p, didx.p, val32.p, in, out, st.p);
-        else
-            newton_spmv<double><<<mgrid, kThreads, 0, s>>>(n, dptr.p, didx.p, val64.p, in, out, st.p);
-    };
-    auto combine = [&](double *out, const double *a, const double *b, const double *c, int which) {
-        newton_combine<<<vgrid, kThreads, 0, s>>>(n, out, a, b, c, st.p, which);
-    };
-    NewtonState *d = st.p;
-    // initial residual norm and target
-    dot(r.p, r.p, &d->rr);
-    cuda_check(cudaMemcpyAsync(&h, st.p, sizeof(h), cudaMemcpyDeviceToHost, s), "Newton state");
-    cuda_check(cudaStreamSynchronize(s), "Newton norm");
-    const double norm = std::sqrt(h.rr);
-    h.target = (fp32 ? 1e-6 : 1e-10) * (1 + norm);
-    h.converged = norm <= h.target;
-    h.stop = h.converged ? 1 : 0;
-    cuda_check(cudaMemcpyAsync(st.p, &h, sizeof(h), cudaMemcpyHostToDevice, s), "Newton state");
+    up(dptr, K.ptr, (nn + 1) * 8);
+    up(didx, K.index, size_t(nnz) * 8);
+    up(dval, K.value, size_t(nnz) * 8);
+    up(mem.at<double>(orhs), rhs, nn * 8);
+    cuda_check(cudaMemsetAsync(mem.at<unsigned>(osync), 0, 8, s), "Newton counters");
+    cuda_check(cudaMemsetAsync(mem.at<NewtonState>(ostate), 0, sizeof(NewtonState), s),
+               "Newton state");
+    NewtonView<V> v{};
+    v.n = n;
+    v.ptr = dptr;
+    v.idx = didx;
+    if constexpr (fp32) {
+        float *dval32 = mem.at<float>(oval32);
+        if (nnz)
+            to_float<<<grid_for(nnz), kThreads, 0, s>>>(nnz, dval, dval32);
+        v.val = dval32;
+    } else
+        v.val = dval;
+    v.rhs = mem.at<double>(orhs);
+    double *dinv = vec, *diag = vec + nn;
+    v.dinv = dinv;
+    double **dst[] = {&v.x, &v.r, &v.p, &v.v, &v.s, &v.t, &v.y, &v.z};
+    for (size_t k = 0; k < 8; ++k)
+        *dst[k] = vec + (2 + k) * nn;
+    v.part = mem.at<double>(opart);
+    v.sync = mem.at<unsigned>(osync);
+    v.st = mem.at<NewtonState>(ostate);
+    v.tolerance = fp32 ? 1e-6 : 1e-10;
+    if (precondition) {
+        newton_diagonal<<<grid_for(n), kThreads, 0, s>>>(n, dptr, didx, dval, diag);
+        newton_scales<<<grid_for(n), kThreads, 0, s>>>(n, dptr, didx, dval, diag, dinv);
+    } else
+        newton_ones<<<grid_for(n), kThreads, 0, s>>>(n, dinv);
+    cuda_check(cudaGetLastError(), "Newton preconditioner");
     const int64_t cap = std::min<int64_t>(20000, 10 * n + 100);
     const auto start = std::chrono::steady_clock::now();
-    for (int64_t it = 0; !h.stop && it < cap; ++it) {
-        if (std::chrono::duration<double>(std::chrono::steady_clock::now() - start).count() >=
-            time_limit) {
+    NewtonState h{};
+    for (int64_t it = 0; !h.stop && (it < cap || it == 0); it += v.iterations) {
+        // a first launch without time forms the target only, and a residual that
+        // already meets it still counts
+        const bool late = std::chrono::duration<double>(std::chrono::steady_clock::now() - start)
+                              .count() >= time_limit;
+        if (late && it > 0) {
             *timed_out = true;
             break;
         }
-        dot(anchor.p, r.p, &d->rho);
-        newton_scalars<<<1, 1, 0, s>>>(d, 0);
-        combine(p.p, r.p, p.p, v.p, 0);
-        newton_scale<<<vgrid, kThreads, 0, s>>>(n, y.p, dinv.p, p.p, d); // y = M^-1 p
-        multiply(y.p, v.p);
-        dot(anchor.p, v.p, &d->divisor);
-        newton_scalars<<<1, 1, 0, s>>>(d, 1);
-        combine(sv.p, r.p, v.p, v.p, 1);
-        dot(sv.p, sv.p, &d->ss);
-        newton_scalars<<<1, 1, 0, s>>>(d, 2);
-        combine(x.p, x.p, y.p, y.p, 2);
-        newton_mark_done<<<1, 1, 0, s>>>(d);
-        newton_scale<<<vgrid, kThreads, 0, s>>>(n, z.p, dinv.p, sv.p, d); // z = M^-1 s
-        multiply(z.p, t.p);
-        dot(t.p, t.p, &d->tt);
-        dot(t.p, sv.p, &d->ts);
-        newton_scalars<<<1, 1, 0, s>>>(d, 3);
-        combine(x.p, x.p, y.p, z.p, 3);
-        combine(r.p, sv.p, t.p, t.p, 4);
-        dot(r.p, r.p, &d->rr);
-        newton_scalars<<<1, 1, 0, s>>>(d, 4);
-        cuda_check(cudaGetLastError(), "Newton iteration");
-        cuda_check(cudaMemcpyAsync(&h, st.p, sizeof(h), cudaMemcpyDeviceToHost, s), "Newton state");
+        v.first = it == 0;
+        v.iterations = late ? 0 : int(std::min<int64_t>(kNewtonChunk, cap - it));
+        void *args[] = {&v};
+        cuda_check(cudaLaunchCooperativeKernel((const void *)newton_kernel<V>, dim3(unsigned(grid)),
+                                               dim3(kThreads), args, 0, s),
+                   "Newton iterations");
+        cuda_check(cudaMemcpyAsync(&h, v.st, sizeof(h), cudaMemcpyDeviceToHost, s), "Newton state");
         cuda_check(cudaStreamSynchronize(s), "Newton state");
+        if (h.fault)
+            throw Error(NK_ERR_CUDA, "a wait inside the Newton kernel was given up");
+        if (late) {
+            *timed_out = !h.stop;
+            break;
+        }
     }
-    cuda_check(cudaMemcpyAsync(x_out, x.p, nn * 8, cudaMemcpyDeviceToHost, s), "Newton solution");
+    cuda_check(cudaMemcpyAsync(x_out, v.x, nn * 8, cudaMemcpyDeviceToHost, s), "Newton solution");
     cuda_check(cudaStreamSynchronize(s), "Newton solution");
     return h.converged != 0;
+}
+
+inline bool newton_solve(const nk_csr &K, const double *rhs, bool fp32, bool precondition,
+                         double time_limit, double *x_out, bool *timed_out) {
+    return fp32 ? newton_solve_t<float>(K, rhs, precondition, time_limit, x_out, timed_out)
+                : newton_solve_t<double>(K, rhs, precondition, time_limit, x_out, timed_out);
 }
 
 } // namespace nk

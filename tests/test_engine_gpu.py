@@ -610,3 +610,37 @@ def test_sparse_q_rows_shared_by_lanes(gpu, oracle, kind, halpern):
         for u, w, z in zip(a.candidates(), b.candidates(), cpu.candidates()):
             assert np.array_equal(u, w)
             near(u, z)
+
+
+@pytest.mark.parametrize("n", [1, 31, 257, 40_000, 160_001])
+@pytest.mark.parametrize("wide", [False, True])
+def test_linear_solve_sizes(gpu, n, wide):
+    """BiCGSTAB in one kernel: rows of 1 to 6 entries (8 lanes a row) and with one
+    row of 50 (32 lanes, more than one stride), sizes below and above what the
+    grid's threads hold one element each of.  K = 4 I + E with at most 0.5 in
+    absolute sums off the diagonal per row, so ||K^-1|| <= 1/3.5 in the maximum
+    norm: the answer is within (1e-10 (1 + |rhs|)) / 3.5 of the exact one."""
+    rng = np.random.default_rng(n)
+    rows = [np.repeat(np.arange(n), 5)]
+    cols = [rng.integers(0, n, 5 * n)]
+    if wide and n > 200:
+        rows.append(np.full(50, n // 2))
+        cols.append(rng.choice(n, 50, replace=False))
+    rows, cols = np.concatenate(rows), np.concatenate(cols)
+    key = np.unique((rows * n + cols)[rows != cols])
+    r, c = key // n, key % n
+    off = rng.uniform(-1, 1, r.size) * 0.5 / np.maximum(1, np.bincount(r, minlength=n))[r]
+    order = np.lexsort((np.r_[c, np.arange(n)], np.r_[r, np.arange(n)]))
+    idx = np.r_[c, np.arange(n)][order].astype(np.int64)
+    val = np.r_[off, np.full(n, 4.0)][order]
+    ptr = np.r_[0, np.cumsum(np.bincount(r, minlength=n) + 1)].astype(np.int64)
+    rhs = rng.standard_normal(n)
+    for precondition in (True, False):
+        x, ok = gpu.linear_solve(ptr, idx, val, rhs, precondition=precondition)
+        assert ok
+        residual = rhs - np.add.reduceat(val * x[idx], ptr[:-1])
+        # the recurrence's residual met the target; its drift is rounding of a few dozen steps
+        target = 1e-10 * (1 + np.linalg.norm(rhs))
+        assert np.linalg.norm(residual) <= 2 * target
+    with pytest.raises(TimeoutError):
+        gpu.linear_solve(ptr, idx, val, rhs, time_limit=0.0)
