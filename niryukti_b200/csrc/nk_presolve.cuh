@@ -91,47 +91,57 @@ inline int64_t compact_csr(const nk_csr &M, int64_t rows, const int64_t *kept, c
         ~StreamGuard() { cudaStreamDestroy(s); }
     } guard_stream{s};
     const int64_t nnz = M.ptr[M.rows];
-    DevBuf<int64_t> dptr(size_t(M.rows + 1)), didx(size_t(std::max<int64_t>(1, nnz))),
-        dkept(size_t(std::max<int64_t>(1, rows))), dmap(size_t(std::max<int64_t>(1, M.cols))),
-        counts(size_t(rows + 1)), optr(size_t(rows + 1));
-    DevBuf<double> dval(size_t(std::max<int64_t>(1, nnz)));
+    size_t temp = 0;
+    cuda_check(cub::DeviceScan::ExclusiveSum(nullptr, temp, static_cast<int64_t *>(nullptr),
+                                             static_cast<int64_t *>(nullptr), rows + 1, s),
+               "compaction scan size");
+    // one allocation; the output holds at most `capacity` entries and the source's
+    const size_t most = size_t(std::max<int64_t>(1, std::min(nnz, capacity)));
+    DevParts mem;
+    const size_t optr_ = mem.add<int64_t>(size_t(M.rows + 1)), oidx_ = mem.add<int64_t>(size_t(nnz)),
+                 oval_ = mem.add<double>(size_t(nnz)), okept_ = mem.add<int64_t>(size_t(rows)),
+                 omap_ = mem.add<int64_t>(size_t(M.cols)),
+                 ocounts_ = mem.add<int64_t>(size_t(rows + 1)),
+                 oout_ = mem.add<int64_t>(size_t(rows + 1)), owork_ = mem.add<unsigned char>(temp),
+                 ooidx_ = mem.add<int64_t>(most), ooval_ = mem.add<double>(most);
+    mem.alloc();
+    int64_t *dptr = mem.at<int64_t>(optr_), *didx = mem.at<int64_t>(oidx_),
+            *dkept = mem.at<int64_t>(okept_), *dmap = mem.at<int64_t>(omap_),
+            *counts = mem.at<int64_t>(ocounts_), *optr = mem.at<int64_t>(oout_),
+            *oidx = mem.at<int64_t>(ooidx_);
+    double *dval = mem.at<double>(oval_), *oval = mem.at<double>(ooval_);
     auto up = [&](void *d, const void *h, size_t bytes) {
         if (bytes)
             cuda_check(cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, s), "compaction upload");
     };
-    up(dptr.p, M.ptr, size_t(M.rows + 1) * 8);
-    up(didx.p, M.index, size_t(nnz) * 8);
-    up(dval.p, M.value, size_t(nnz) * 8);
-    up(dkept.p, kept, size_t(rows) * 8);
-    up(dmap.p, map, size_t(M.cols) * 8);
+    up(dptr, M.ptr, size_t(M.rows + 1) * 8);
+    up(didx, M.index, size_t(nnz) * 8);
+    up(dval, M.value, size_t(nnz) * 8);
+    up(dkept, kept, size_t(rows) * 8);
+    up(dmap, map, size_t(M.cols) * 8);
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int grid = int(std::max<int64_t>(1, std::min<int64_t>((rows + kWarps - 1) / kWarps,
                                                                 int64_t(sms) * 8)));
-    compact_count<<<grid, kThreads, 0, s>>>(rows, dkept.p, dptr.p, didx.p, dmap.p, counts.p);
+    compact_count<<<grid, kThreads, 0, s>>>(rows, dkept, dptr, didx, dmap, counts);
     cuda_check(cudaGetLastError(), "compaction count");
-    size_t temp = 0;
-    cuda_check(cub::DeviceScan::ExclusiveSum(nullptr, temp, counts.p, optr.p, rows + 1, s),
-               "compaction scan size");
-    DevBuf<unsigned char> work(std::max<size_t>(1, temp));
-    cuda_check(cub::DeviceScan::ExclusiveSum(work.p, temp, counts.p, optr.p, rows + 1, s),
+    cuda_check(cub::DeviceScan::ExclusiveSum(mem.at<unsigned char>(owork_), temp, counts, optr,
+                                             rows + 1, s),
                "compaction scan");
-    cuda_check(cudaMemcpyAsync(out_ptr, optr.p, size_t(rows + 1) * 8, cudaMemcpyDeviceToHost, s),
+    cuda_check(cudaMemcpyAsync(out_ptr, optr, size_t(rows + 1) * 8, cudaMemcpyDeviceToHost, s),
                "compaction offsets");
     cuda_check(cudaStreamSynchronize(s), "compaction offsets");
     const int64_t total = out_ptr[rows];
     if (total > capacity)
         throw Error(NK_ERR_INVALID, "compaction output capacity is too small");
     if (total) {
-        DevBuf<int64_t> oidx(static_cast<size_t>(total));
-        DevBuf<double> oval(static_cast<size_t>(total));
-        compact_scatter<<<grid, kThreads, 0, s>>>(rows, dkept.p, dptr.p, didx.p, dval.p, dmap.p,
-                                                  optr.p, oidx.p, oval.p);
+        compact_scatter<<<grid, kThreads, 0, s>>>(rows, dkept, dptr, didx, dval, dmap, optr, oidx,
+                                                  oval);
         cuda_check(cudaGetLastError(), "compaction scatter");
-        cuda_check(cudaMemcpyAsync(out_index, oidx.p, size_t(total) * 8, cudaMemcpyDeviceToHost, s),
+        cuda_check(cudaMemcpyAsync(out_index, oidx, size_t(total) * 8, cudaMemcpyDeviceToHost, s),
                    "compaction indices");
-        cuda_check(cudaMemcpyAsync(out_value, oval.p, size_t(total) * 8, cudaMemcpyDeviceToHost, s),
+        cuda_check(cudaMemcpyAsync(out_value, oval, size_t(total) * 8, cudaMemcpyDeviceToHost, s),
                    "compaction values");
         cuda_check(cudaStreamSynchronize(s), "compaction completion");
     }
@@ -164,75 +174,142 @@ __device__ __forceinline__ void propose_upper(double *address, double value) {
     }
 }
 
-// One pass over the rows, one thread per row (a row's activity bounds are
-// sums in the row's entry order with directed rounding, so they are not split
-// across lanes).  Reads the bounds of the previous pass (lb, ub) and proposes
-// into new_lb / new_ub; flags a row whose activity range misses [rl, ru].
-__global__ void propagate_rows(int64_t rows, const int64_t *__restrict__ ptr,
-                               const int64_t *__restrict__ index, const double *__restrict__ a,
-                               const int *__restrict__ integer, const double *__restrict__ lb,
-                               const double *__restrict__ ub, const double *__restrict__ rl,
-                               const double *__restrict__ ru, double *new_lb, double *new_ub,
-                               int *failed) {
-    const int64_t stride = int64_t(gridDim.x) * blockDim.x;
-    for (int64_t row = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; row < rows; row += stride) {
-        const int64_t b = ptr[row], e = ptr[row + 1];
-        double low = 0, high = 0;
-        int low_inf = 0, high_inf = 0;
-        for (int64_t k = b; k < e; ++k) {
-            const double v = a[k];
-            if (v == 0)
-                continue;
-            const int64_t j = index[k];
-            const double lo = __dmul_rd(v, v > 0 ? lb[j] : ub[j]);
-            const double hi = __dmul_ru(v, v > 0 ? ub[j] : lb[j]);
-            if (isinf(lo))
-                ++low_inf;
-            else
-                low = __dadd_rd(low, lo);
-            if (isinf(hi))
-                ++high_inf;
-            else
-                high = __dadd_ru(high, hi);
+// The least and greatest of an entry's contribution to its row's activity.
+__device__ __forceinline__ double term_low(double v, double lb, double ub) {
+    return __dmul_rd(v, v > 0 ? lb : ub);
+}
+__device__ __forceinline__ double term_high(double v, double lb, double ub) {
+    return __dmul_ru(v, v > 0 ? ub : lb);
+}
+
+// A row's activity range: the finite terms' directed-rounding sums in entry
+// order (not split across lanes: the order is part of the result) and how many
+// terms are infinite.
+struct RowActivity {
+    double low = 0, high = 0;
+    int low_inf = 0, high_inf = 0;
+    __device__ __forceinline__ void add(double lo, double hi) {
+        if (isinf(lo))
+            ++low_inf;
+        else
+            low = __dadd_rd(low, lo);
+        if (isinf(hi))
+            ++high_inf;
+        else
+            high = __dadd_ru(high, hi);
+    }
+    __device__ __forceinline__ bool misses(double rlo, double rhi) const {
+        return (!low_inf && low > rhi) || (!high_inf && high < rlo);
+    }
+};
+
+// The bounds that entry v of a row implies on its column j.
+__device__ __forceinline__ void propose_entry(double v, int64_t j, const RowActivity &r, double rlo,
+                                              double rhi, const int *integer, double lb, double ub,
+                                              double *new_lb, double *new_ub) {
+    const double end_low = v > 0 ? lb : ub, end_high = v > 0 ? ub : lb;
+    const double tl = __dmul_rd(v, end_low), th = __dmul_ru(v, end_high);
+    // the rest of the row: removing a term needs the opposite rounding
+    const double rest_low = r.low_inf - int(isinf(tl)) ? -INFINITY
+                            : isinf(tl)                ? r.low
+                                        : __dsub_rd(r.low, __dmul_ru(v, end_low));
+    const double rest_high = r.high_inf - int(isinf(th)) ? INFINITY
+                             : isinf(th)                 ? r.high
+                                         : __dsub_ru(r.high, __dmul_rd(v, end_high));
+    double l = -INFINITY, u = INFINITY;
+    if (isfinite(rlo) && isfinite(rest_high)) {
+        const double num = __dsub_rd(rlo, rest_high);
+        if (v > 0)
+            l = __ddiv_rd(num, v);
+        else
+            u = __ddiv_ru(num, v);
+    }
+    if (isfinite(rhi) && isfinite(rest_low)) {
+        const double num = __dsub_ru(rhi, rest_low);
+        if (v > 0)
+            u = __ddiv_ru(num, v);
+        else
+            l = __ddiv_rd(num, v);
+    }
+    const bool whole = integer[j] != 0;
+    if (isfinite(l) && (!whole || fabs(l) < 0x1p52))
+        propose_lower(new_lb + j, whole ? ceil(l) : l);
+    if (isfinite(u) && (!whole || fabs(u) < 0x1p52))
+        propose_upper(new_ub + j, whole ? floor(u) : u);
+}
+
+// One pass over the rows.  Reads the bounds of the previous pass (lb, ub) and
+// proposes into new_lb / new_ub; flags a row whose activity range misses
+// [rl, ru].  A thread per row walking its entries twice is two chains of
+// dependent, uncoalesced loads (78 us for 20,000 rows of 16 entries); so a warp
+// takes 32 rows together: the terms are formed flat, entry by entry, into shared
+// memory, a lane adds up its row's in order, and the proposals are formed flat
+// again (48 us).  32 rows of more than kPropEntries entries keep the walk.
+constexpr int kPropWarps = 4, kPropEntries = 640;
+__global__ void __launch_bounds__(kPropWarps * 32)
+    propagate_rows(int64_t rows, const int64_t *__restrict__ ptr,
+                   const int64_t *__restrict__ index, const double *__restrict__ a,
+                   const int *__restrict__ integer, const double *__restrict__ lb,
+                   const double *__restrict__ ub, const double *__restrict__ rl,
+                   const double *__restrict__ ru, double *new_lb, double *new_ub, int *failed) {
+    // a term's place is its entry's plus its row's, so that lanes reading rows of
+    // one length do not meet in a bank
+    __shared__ double lows[kPropWarps][kPropEntries + 32], highs[kPropWarps][kPropEntries + 32];
+    __shared__ unsigned char owner[kPropWarps][kPropEntries];
+    __shared__ RowActivity activity[kPropWarps][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t groups = (rows + 31) / 32, stride = int64_t(gridDim.x) * kPropWarps;
+    for (int64_t g = int64_t(blockIdx.x) * kPropWarps + w; g < groups; g += stride) {
+        const int64_t row = 32 * g + lane, base = ptr[32 * g];
+        const int64_t b = ptr[row < rows ? row : rows], e = ptr[row < rows ? row + 1 : rows];
+        const double rlo = row < rows ? rl[row] : 0., rhi = row < rows ? ru[row] : 0.;
+        const int64_t total = __shfl_sync(0xffffffffu, e, 31) - base;
+        RowActivity r;
+        if (total > kPropEntries) {
+            for (int64_t k = b; k < e; ++k) {
+                const double v = a[k];
+                if (v != 0)
+                    r.add(term_low(v, lb[index[k]], ub[index[k]]),
+                          term_high(v, lb[index[k]], ub[index[k]]));
+            }
+            if (row < rows && r.misses(rlo, rhi))
+                atomicExch(failed, 1);
+            for (int64_t k = b; k < e; ++k)
+                if (a[k] != 0)
+                    propose_entry(a[k], index[k], r, rlo, rhi, integer, lb[index[k]], ub[index[k]],
+                                  new_lb, new_ub);
+            continue;
         }
-        const double rlo = rl[row], rhi = ru[row];
-        if ((!low_inf && low > rhi) || (!high_inf && high < rlo))
+        const int first = int(b - base), last = int(e - base), n = int(total);
+        for (int k = first; k < last; ++k)
+            owner[w][k] = static_cast<unsigned char>(lane);
+        __syncwarp();
+        for (int k = lane; k < n; k += 32) {
+            const double v = a[base + k];
+            const int64_t j = index[base + k];
+            const double l = lb[j], u = ub[j];
+            const int at = k + owner[w][k];
+            // a zero coefficient has no term, whatever its column's bounds
+            lows[w][at] = v != 0 ? term_low(v, l, u) : 0.;
+            highs[w][at] = v != 0 ? term_high(v, l, u) : 0.;
+        }
+        __syncwarp();
+        for (int k = first; k < last; ++k)
+            r.add(lows[w][k + lane], highs[w][k + lane]);
+        if (row < rows && r.misses(rlo, rhi))
             atomicExch(failed, 1);
-        for (int64_t k = b; k < e; ++k) {
-            const double v = a[k];
-            if (v == 0)
-                continue;
-            const int64_t j = index[k];
-            const double end_low = v > 0 ? lb[j] : ub[j], end_high = v > 0 ? ub[j] : lb[j];
-            const double term_low = __dmul_rd(v, end_low), term_high = __dmul_ru(v, end_high);
-            // the rest of the row: removing a term needs the opposite rounding
-            const double rest_low = low_inf - int(isinf(term_low)) ? -INFINITY
-                                    : isinf(term_low)              ? low
-                                                : __dsub_rd(low, __dmul_ru(v, end_low));
-            const double rest_high = high_inf - int(isinf(term_high)) ? INFINITY
-                                     : isinf(term_high)               ? high
-                                                : __dsub_ru(high, __dmul_rd(v, end_high));
-            double l = -INFINITY, u = INFINITY;
-            if (isfinite(rlo) && isfinite(rest_high)) {
-                const double num = __dsub_rd(rlo, rest_high);
-                if (v > 0)
-                    l = __ddiv_rd(num, v);
-                else
-                    u = __ddiv_ru(num, v);
+        activity[w][lane] = r;
+        __syncwarp();
+        for (int k0 = 0; k0 < n; k0 += 32) { // whole warps: the bounds come by shuffle
+            const int k = k0 + lane, q = k < n ? owner[w][k] : 0;
+            const double lo = __shfl_sync(0xffffffffu, rlo, q), hi = __shfl_sync(0xffffffffu, rhi, q);
+            if (k < n && a[base + k] != 0) {
+                const int64_t j = index[base + k];
+                propose_entry(a[base + k], j, activity[w][q], lo, hi, integer, lb[j], ub[j], new_lb,
+                              new_ub);
             }
-            if (isfinite(rhi) && isfinite(rest_low)) {
-                const double num = __dsub_ru(rhi, rest_low);
-                if (v > 0)
-                    u = __ddiv_ru(num, v);
-                else
-                    l = __ddiv_rd(num, v);
-            }
-            const bool whole = integer[j] != 0;
-            if (isfinite(l) && (!whole || fabs(l) < 0x1p52))
-                propose_lower(new_lb + j, whole ? ceil(l) : l);
-            if (isfinite(u) && (!whole || fabs(u) < 0x1p52))
-                propose_upper(new_ub + j, whole ? floor(u) : u);
         }
+        __syncwarp();
     }
 }
 
@@ -250,47 +327,51 @@ inline bool propagate_bounds(const nk_csr &A, const int *integer, const double *
         cudaStream_t s;
         ~StreamGuard() { cudaStreamDestroy(s); }
     } guard_stream{s};
-    const size_t nb = size_t(std::max<int64_t>(1, n));
-    DevBuf<int64_t> dptr(size_t(m + 1)), didx(size_t(std::max<int64_t>(1, nnz)));
-    DevBuf<double> dval(static_cast<size_t>(std::max<int64_t>(1, nnz))),
-        drl(static_cast<size_t>(m)), dru(static_cast<size_t>(m));
-    DevBuf<double> olb(nb), oub(nb), nlb(nb), nub(nb);
-    DevBuf<int> dint(nb), dfail(1);
+    // one allocation; the bounds of the last pass and of this one lie together
+    DevParts mem;
+    const size_t optr_ = mem.add<int64_t>(size_t(m + 1)), oidx_ = mem.add<int64_t>(size_t(nnz)),
+                 oval_ = mem.add<double>(size_t(nnz)), orl_ = mem.add<double>(2 * size_t(m)),
+                 oold_ = mem.add<double>(2 * size_t(n)), onew_ = mem.add<double>(2 * size_t(n)),
+                 oint_ = mem.add<int>(size_t(n)), ofail_ = mem.add<int>(1);
+    mem.alloc();
+    int64_t *dptr = mem.at<int64_t>(optr_), *didx = mem.at<int64_t>(oidx_);
+    double *dval = mem.at<double>(oval_), *drl = mem.at<double>(orl_), *dru = drl + m;
+    double *olb = mem.at<double>(oold_), *oub = olb + n, *nlb = mem.at<double>(onew_), *nub = nlb + n;
+    int *dint = mem.at<int>(oint_), *dfail = mem.at<int>(ofail_);
     auto up = [&](void *d, const void *h, size_t bytes) {
         if (bytes)
             cuda_check(cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, s), "propagation upload");
     };
-    up(dptr.p, A.ptr, size_t(m + 1) * 8);
-    up(didx.p, A.index, size_t(nnz) * 8);
-    up(dval.p, A.value, size_t(nnz) * 8);
-    up(drl.p, rl, size_t(m) * 8);
-    up(dru.p, ru, size_t(m) * 8);
-    up(dint.p, integer, size_t(n) * sizeof(int));
-    up(olb.p, lb, size_t(n) * 8);
-    up(oub.p, ub, size_t(n) * 8);
-    up(nlb.p, lb, size_t(n) * 8);
-    up(nub.p, ub, size_t(n) * 8);
-    cuda_check(cudaMemsetAsync(dfail.p, 0, sizeof(int), s), "propagation flag");
+    up(dptr, A.ptr, size_t(m + 1) * 8);
+    up(didx, A.index, size_t(nnz) * 8);
+    up(dval, A.value, size_t(nnz) * 8);
+    up(drl, rl, size_t(m) * 8);
+    up(dru, ru, size_t(m) * 8);
+    up(dint, integer, size_t(n) * sizeof(int));
+    up(olb, lb, size_t(n) * 8);
+    up(oub, ub, size_t(n) * 8);
+    cuda_check(cudaMemcpyAsync(nlb, olb, size_t(n) * 16, cudaMemcpyDeviceToDevice, s),
+               "propagation bounds");
+    cuda_check(cudaMemsetAsync(dfail, 0, sizeof(int), s), "propagation flag");
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int grid = int(std::max<int64_t>(1, std::min<int64_t>((m + kThreads - 1) / kThreads,
-                                                                int64_t(sms) * 8)));
+    const int grid = int(std::max<int64_t>(1, std::min<int64_t>(
+        (m + 32 * kPropWarps - 1) / (32 * kPropWarps), int64_t(sms) * 8)));
     for (int pass = 0; pass < passes; ++pass) {
-        propagate_rows<<<grid, kThreads, 0, s>>>(m, dptr.p, didx.p, dval.p, dint.p, olb.p, oub.p,
-                                                 drl.p, dru.p, nlb.p, nub.p, dfail.p);
+        propagate_rows<<<grid, kPropWarps * 32, 0, s>>>(m, dptr, didx, dval, dint, olb, oub, drl, dru,
+                                                        nlb, nub, dfail);
         cuda_check(cudaGetLastError(), "propagation pass");
-        cuda_check(cudaMemcpyAsync(olb.p, nlb.p, size_t(n) * 8, cudaMemcpyDeviceToDevice, s),
-                   "propagation lower");
-        cuda_check(cudaMemcpyAsync(oub.p, nub.p, size_t(n) * 8, cudaMemcpyDeviceToDevice, s),
-                   "propagation upper");
+        if (pass + 1 < passes)
+            cuda_check(cudaMemcpyAsync(olb, nlb, size_t(n) * 16, cudaMemcpyDeviceToDevice, s),
+                       "propagation bounds");
     }
     int failed = 0;
-    cuda_check(cudaMemcpyAsync(&failed, dfail.p, sizeof(int), cudaMemcpyDeviceToHost, s),
+    cuda_check(cudaMemcpyAsync(&failed, dfail, sizeof(int), cudaMemcpyDeviceToHost, s),
                "propagation flag");
-    cuda_check(cudaMemcpyAsync(lb, nlb.p, size_t(n) * 8, cudaMemcpyDeviceToHost, s),
+    cuda_check(cudaMemcpyAsync(lb, nlb, size_t(n) * 8, cudaMemcpyDeviceToHost, s),
                "propagation lower");
-    cuda_check(cudaMemcpyAsync(ub, nub.p, size_t(n) * 8, cudaMemcpyDeviceToHost, s),
+    cuda_check(cudaMemcpyAsync(ub, nub, size_t(n) * 8, cudaMemcpyDeviceToHost, s),
                "propagation upper");
     cuda_check(cudaStreamSynchronize(s), "propagation completion");
     if (failed)

@@ -644,3 +644,27 @@ def test_linear_solve_sizes(gpu, n, wide):
         assert np.linalg.norm(residual) <= 2 * target
     with pytest.raises(TimeoutError):
         gpu.linear_solve(ptr, idx, val, rhs, time_limit=0.0)
+
+
+@pytest.mark.parametrize("rows,per", [(1, 3), (33, 1), (64, 20), (65, 21), (200, 60), (500, 9)])
+def test_propagate_bounds_row_groups(gpu, oracle, rows, per):
+    """Bound propagation by groups of 32 rows: a last group of one row, empty rows,
+    zero coefficients, infinite bounds, groups of exactly the 640 entries that fit
+    a warp's buffers and of more, which a lane walks; bit-identical to the
+    sequential restatement."""
+    rng = np.random.default_rng(100 * rows + per)
+    n = 3 * rows + per
+    entries = [(i, int(j), float(v)) for i in range(rows) if rows == 64 or i % 11 != 5
+               for j, v in zip(np.sort(rng.choice(n, per, replace=False)),
+                               np.round(rng.standard_normal(per), 1))]
+    m = tiny(n, rows, entries)
+    lb, ub = rng.uniform(-5, 0, n), rng.uniform(0, 40, n)
+    lb[::13], ub[::17] = -np.inf, np.inf
+    m.rl, m.ru = rng.uniform(-30, -10, rows), rng.uniform(10, 30, rows)
+    m.rl[::5] = -np.inf
+    integer = (np.arange(n) % 3 == 0).astype(np.int32)
+    got = gpu.propagate_bounds(m, integer, lb, ub, 4)
+    want = oracle.propagate_bounds(m, integer, lb, ub, 4)
+    assert got[0] == want[0]
+    for u, w in zip(got[1:], want[1:]):
+        assert np.array_equal(u.view(np.int64), w.view(np.int64))
