@@ -26,19 +26,12 @@
 #ifndef NK_FUSED_THREADS
 #define NK_FUSED_THREADS 1024 // threads per CTA of the fused trial kernels
 #endif
-#ifndef NK_SPLIT_PIPE
-#define NK_SPLIT_PIPE 0 // 1: software-pipelined dot for split-row segments
-#endif
-#ifndef NK_DUAL_GATHER
-#define NK_DUAL_GATHER 0 // gather flavour of the dual kernel's dx loads (gather_as)
-#endif
 #ifndef NK_PREFETCH
 #define NK_PREFETCH 1 // 1: load a row's epilogue vectors before its dot product
 #endif
 
 namespace nk {
 
-constexpr int kDualGather = NK_DUAL_GATHER;
 // The fused kernels run 1024 threads per SM (64 registers each) in CTAs of
 // kFusedThreads; larger CTAs give each CTA a larger slice of shared memory.
 constexpr int kFusedThreads = NK_FUSED_THREADS;
@@ -176,15 +169,11 @@ __device__ __forceinline__ bool split_chunk(double *wpart /* this warp's 32 */, 
 // start; on true, *row and *total hold the completed row.
 // *cross receives the row's counter when the row spans chunks (-1 when it
 // lies in this chunk).
-template <class Acc, int G = 0, class V, class I, class X>
+template <class Acc, int U, class V, class I, class X>
 __device__ __noinline__ bool split_lane(const Sell<V, I> M, int64_t vr, int len,
                                         const X *__restrict__ x, const double *init_vec,
                                         double *wpart, int64_t *row, double *total, int *cross) {
-#if NK_SPLIT_PIPE
-    const double part = double(sell_dot_pipelined<Acc, kUnrollSplit>(M, vr, len, Acc(0), x));
-#else
-    const double part = double(sell_dot<Acc, kUnrollSplit, G>(M, vr, len, Acc(0), x));
-#endif
+    const double part = double(sell_dot<Acc, U>(M, vr, len, Acc(0), x));
     const int4 sg = M.seg[vr];
     *row = sg.x;
     *cross = sg.w;
@@ -358,10 +347,10 @@ __global__ void __launch_bounds__(kFusedThreads, kFusedMinBlocks)
                     int cross = -1;
                     bool done;
                     if constexpr (FP32G) // FP32 sums add c_j afterwards, in FP64
-                        done = split_lane<Acc>(At, vr, At.len[vr], y32, nullptr,
+                        done = split_lane<Acc, 4>(At, vr, At.len[vr], y32, nullptr,
                                                wpart[threadIdx.x >> 5], &j, &g, &cross);
                     else
-                        done = split_lane<Acc>(At, vr, At.len[vr], y, v.c,
+                        done = split_lane<Acc, 4>(At, vr, At.len[vr], y, v.c,
                                                wpart[threadIdx.x >> 5], &j, &g, &cross);
                     if (done) {
                         if constexpr (FP32G)
@@ -465,7 +454,8 @@ __device__ inline void store_control(Control *ctl, const Control &s) {
 // of them); the schedule lists them as "combine chunks" (encoded -k-1 for
 // rows [32k, 32k+32)) in place of their split-row chunks, and a lane adds its
 // row's run sums in slot order (panel by panel, runs in CSR order).
-template <class Acc, class V, class I, bool FP32G, bool SPLIT, bool PANEL = false>
+// U: entries of its row or segment that a lane loads before adding them.
+template <class Acc, class V, class I, bool FP32G, bool SPLIT, bool PANEL = false, int U = 4>
 __global__ void __launch_bounds__(kFusedThreads, kFusedMinBlocks)
     dual_kernel(Sell<V, I> A, Vecs v) {
     __shared__ double wpart[SPLIT ? kFusedWarps : 1][32];
@@ -552,11 +542,9 @@ __global__ void __launch_bounds__(kFusedThreads, kFusedMinBlocks)
 #endif
                     double delta;
                     if constexpr (FP32G)
-                        delta = double(sell_dot<Acc, kUnroll, kDualGather>(A, vr, len, Acc(0),
-                                                                         v.dx32));
+                        delta = double(sell_dot<Acc, U>(A, vr, len, Acc(0), v.dx32));
                     else
-                        delta = double(sell_dot<Acc, kUnroll, kDualGather>(A, vr, len, Acc(0),
-                                                                         v.dx));
+                        delta = double(sell_dot<Acc, U>(A, vr, len, Acc(0), v.dx));
 #if NK_PREFETCH
                     finish(i, delta, yi, axi, rli, rui, ai, dy2, cpl);
 #else
@@ -571,11 +559,11 @@ __global__ void __launch_bounds__(kFusedThreads, kFusedMinBlocks)
                         int cross = -1;
                         bool done;
                         if constexpr (FP32G)
-                            done = split_lane<Acc, kDualGather>(A, vr, A.len[vr], v.dx32, nullptr,
+                            done = split_lane<Acc, U>(A, vr, A.len[vr], v.dx32, nullptr,
                                                                 wpart[threadIdx.x >> 5], &i,
                                                                 &delta, &cross);
                         else
-                            done = split_lane<Acc, kDualGather>(A, vr, A.len[vr], v.dx, nullptr,
+                            done = split_lane<Acc, U>(A, vr, A.len[vr], v.dx, nullptr,
                                                                 wpart[threadIdx.x >> 5], &i,
                                                                 &delta, &cross);
                         if (done) {

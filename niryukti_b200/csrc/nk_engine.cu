@@ -466,6 +466,25 @@ template <class Acc, class V, class I> PrimalFn<V, I> primal_kernel_for(bool spa
                      : primal_kernel<Acc, V, I, true, F, false>;
     return split ? primal_kernel<Acc, V, I, false, F, true> : primal_kernel<Acc, V, I, false, F, false>;
 }
+// The dual kernel instance.  With long rows a lane loads 8 entries ahead where a
+// warp's walk through a split chunk, up to 256 steps, shows in the kernel's time,
+// and 4 where the SM's lookups set it (or there is no long row) and 8 only cost
+// registers.  us with 4 and with 8 on power-law LPs: 47 / 35 at 2 M entries,
+// 49 / 41 at 5 M, 62 / 55 at 8 M, 72 / 69 at 12 M, 87 / 89 at 16 M, 107 / 109 at
+// 20 M; without long rows 31 / 32 at 4 M, 64 / 67 at 11 M.
+template <class V, class I> using DualFn = void (*)(Sell<V, I>, Vecs);
+constexpr int64_t kDeepEntries = int64_t(13) << 20;
+template <class Acc, class V, class I> DualFn<V, I> dual_kernel_for(const SellMatrix &A, bool panels) {
+    constexpr bool F = sizeof(Acc) == 4;
+    const bool deep = A.nsr > 0 && A.nnz < kDeepEntries;
+    if (panels)
+        return deep ? dual_kernel<Acc, V, I, F, false, true, 8>
+                    : dual_kernel<Acc, V, I, F, false, true, 4>;
+    if (A.nsv > 0)
+        return deep ? dual_kernel<Acc, V, I, F, true, false, 8>
+                    : dual_kernel<Acc, V, I, F, true, false, 4>;
+    return dual_kernel<Acc, V, I, F, false, false, 4>;
+}
 
 template <class V, bool QP> const void *resident_kernel_of(bool split, bool halpern) {
     if (halpern)
@@ -600,12 +619,8 @@ struct Engine {
                 pan.view<V>(), dxp, ctl.p);
             if (ev[3])
                 mark(3);
-            dual_kernel<Acc, V, I, F32, false, true><<<grid_d, kFusedThreads, smem_d(), stream>>>(a,
-                                                                                                v);
-        } else if (A.nsv > 0)
-            dual_kernel<Acc, V, I, F32, true><<<grid_d, kFusedThreads, smem_d(), stream>>>(a, v);
-        else
-            dual_kernel<Acc, V, I, F32, false><<<grid_d, kFusedThreads, smem_d(), stream>>>(a, v);
+        }
+        dual_kernel_for<Acc, V, I>(A, panels)<<<grid_d, kFusedThreads, smem_d(), stream>>>(a, v);
         if (ev[2])
             mark(2);
         if (halpern)
@@ -1625,11 +1640,8 @@ void build_panels(PanelMatrix &P, int64_t rows, int64_t cols, const std::vector<
 // grids hold exactly the CTAs that fit on the device at once; their slot
 // memory is sized after the schedules are built (attach_slots).
 template <class Acc, class V, class I> void configure(Engine &E) {
-    constexpr bool F32 = sizeof(Acc) == 4;
     const void *pk = (const void *)primal_kernel_for<Acc, V, I>(E.sparse_q, E.At.nsv > 0);
-    const void *dk = E.panels           ? (const void *)dual_kernel<Acc, V, I, F32, false, true>
-                     : E.A.nsv > 0 ? (const void *)dual_kernel<Acc, V, I, F32, true>
-                                        : (const void *)dual_kernel<Acc, V, I, F32, false>;
+    const void *dk = (const void *)dual_kernel_for<Acc, V, I>(E.A, E.panels);
     // the slot arrays stay far below the default 48 KB; the grids are sized
     // without them, which the occupancy check after the schedules confirms
     E.grid_p = occupancy_grid(pk, (E.At.nv + 31) / 32, kFusedThreads, 0);
@@ -1637,11 +1649,8 @@ template <class Acc, class V, class I> void configure(Engine &E) {
     E.grid_s = occupancy_grid((const void *)spmv_kernel<V, I>, int64_t(1) << 40);
 }
 template <class Acc, class V, class I> void attach_slots(Engine &E) {
-    constexpr bool F32 = sizeof(Acc) == 4;
     const void *pk = (const void *)primal_kernel_for<Acc, V, I>(E.sparse_q, E.At.nsv > 0);
-    const void *dk = E.panels           ? (const void *)dual_kernel<Acc, V, I, F32, false, true>
-                     : E.A.nsv > 0 ? (const void *)dual_kernel<Acc, V, I, F32, true>
-                                        : (const void *)dual_kernel<Acc, V, I, F32, false>;
+    const void *dk = (const void *)dual_kernel_for<Acc, V, I>(E.A, E.panels);
     for (auto [k, bytes, grid] : {std::tuple<const void *, size_t, int>{pk, E.smem_p(), E.grid_p},
                                   {dk, E.smem_d(), E.grid_d}}) {
         if (bytes > 48 * 1024)
@@ -2094,6 +2103,20 @@ Engine *create_engine(const nk_csr *Ah, const nk_csr *Qh, const double *hc, cons
         for (int64_t i = 0; i < m; ++i)
             engine_rlen[size_t(i)] = rlen[size_t(rperm[size_t(i)])];
         plan_resident(*E, lists_t, lists_a, engine_rlen, s);
+    }
+    // Column panels cost a launch and a pass over the run sums, about 25 us
+    // together, and pay for that from about 4 M entries in the long rows on.  us a
+    // trial with and without: 1.2 M of them (power-law, 2 M entries in all) 62 / 41,
+    // 2.4 M (power-law, 4 M) 75 / 52, 2.4 M (block-angular) 59 / 49, 3 M 63 / 56,
+    // 9 M 81 / 91.  (FP32 sums keep them: their rounding is the panels'.  So do
+    // resident models, whose profiled kernels use them.)
+    if (E->panels && !E->resident.on && !E->wide && o->precision != NK_PRECISION_FP32 &&
+        E->pan.entries < NK_PANEL_MIN_ENTRIES) {
+        E->panels = false;
+        E->pan = PanelMatrix{};
+        use_schedule(E->A, lists_a, s);
+        o->precision == NK_PRECISION_FP64 ? attach_slots<double, double, int32_t>(*E)
+                                          : attach_slots<double, float, int32_t>(*E);
     }
     E->split_p.alloc(size_t(std::max(1, E->At.ncounters)));
     E->split_d.alloc(size_t(2 * std::max(1, E->A.ncounters)));

@@ -48,6 +48,9 @@
 #ifndef NK_PANEL_MIN_RUN
 #define NK_PANEL_MIN_RUN 32 // panels only when long rows average this many entries per panel
 #endif
+#ifndef NK_PANEL_MIN_ENTRIES
+#define NK_PANEL_MIN_ENTRIES (int64_t(4) << 20) // ... and the long rows hold this many
+#endif
 #ifndef NK_PANEL_MIN_SPLIT
 #define NK_PANEL_MIN_SPLIT 64 // segments are cut into runs of no fewer entries than this
 #endif

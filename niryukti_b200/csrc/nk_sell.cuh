@@ -24,15 +24,6 @@
 
 namespace nk {
 
-#ifndef NK_UNROLL
-#define NK_UNROLL 4
-#endif
-#ifndef NK_UNROLL_SPLIT
-#define NK_UNROLL_SPLIT 4
-#endif
-constexpr int kUnroll = NK_UNROLL;            // independent loads in flight per lane
-constexpr int kUnrollSplit = NK_UNROLL_SPLIT; // the same for split-row segments
-
 template <class V, class I> struct Sell {
     const int64_t *cptr;   // nchunks + 1 element offsets
     const int32_t *len;    // length of each virtual row
@@ -53,7 +44,7 @@ template <class V, class I> struct Sell {
 // Sequential dot product of virtual row v (entries in CSR order) starting
 // from acc; U entries' loads are issued before their products are added.
 // Used inside the fused PDHG kernels, where registers are scarce.
-template <class Acc, int U = kUnroll, int G = 0, class V, class I, class X>
+template <class Acc, int U = 4, class V, class I, class X>
 __device__ __forceinline__ Acc sell_dot(const Sell<V, I> &M, int64_t v, int len, Acc acc,
                                         const X *__restrict__ x) {
     const int64_t base = M.cptr[v >> 5] + (v & 31);
@@ -71,14 +62,14 @@ __device__ __forceinline__ Acc sell_dot(const Sell<V, I> &M, int64_t v, int len,
         X g[U];
 #pragma unroll
         for (int u = 0; u < U; ++u)
-            g[u] = gather_as<G>(x + j[u]);
+            g[u] = gather_load(x + j[u]);
 #pragma unroll
         for (int u = 0; u < U; ++u)
             acc = acc + Acc(w[u]) * Acc(g[u]);
     }
     for (; k < len; ++k)
         acc = acc + Acc(stream_load(vp + int64_t(k) * 32)) *
-                        Acc(gather_as<G>(x + stream_load(ip + int64_t(k) * 32)));
+                        Acc(gather_load(x + stream_load(ip + int64_t(k) * 32)));
     return acc;
 }
 
@@ -86,7 +77,7 @@ __device__ __forceinline__ Acc sell_dot(const Sell<V, I> &M, int64_t v, int len,
 // index/value loads of block b+1, and only then are block b's products added,
 // so each block costs about one memory round trip instead of two.  It needs
 // more registers; the plain SpMV kernel uses it.
-template <class Acc, int U = kUnroll, class V, class I, class X>
+template <class Acc, int U = 4, class V, class I, class X>
 __device__ __forceinline__ Acc sell_dot_pipelined(const Sell<V, I> &M, int64_t v, int len, Acc acc,
                                                   const X *__restrict__ x) {
     if (len <= 0)

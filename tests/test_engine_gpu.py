@@ -668,3 +668,25 @@ def test_propagate_bounds_row_groups(gpu, oracle, rows, per):
     assert got[0] == want[0]
     for u, w in zip(got[1:], want[1:]):
         assert np.array_equal(u.view(np.int64), w.view(np.int64))
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("nnz,len_hi,panels", [(1_600_000, 5000, False), (1_600_000, 9000, False),
+                                               (9_000_000, 9000, True)])
+def test_long_rows_past_the_resident_size(gpu, oracle, nnz, len_hi, panels, precision):
+    """Models too large for the resident trials: long rows as split rows where they
+    hold fewer than 4 M entries (rows of more than 8,192 across chunks), by column
+    panel above; against the CPU's sequential sums over 20 fixed-step trials.  A row
+    of 9,000 terms regrouped rounds within 9,000 ulp of its terms' magnitude,
+    2e-12, per trial: 1e-10 in all."""
+    m = synth.power_law_lp(m=60_000, n=40_000, nnz=nnz, seed=11, len_lo=2 if not panels else 100,
+                           len_hi=len_hi)
+    if precision == "mixed":
+        m.val = m.val.astype(np.float32).astype(np.float64)
+    g = gpu.PdhgBackend(m, graphs=True, precision=precision)
+    assert (g.layout_info()["panels"] > 0) == panels
+    cpu = oracle.model(m).backend(np.zeros(m.n), np.zeros(m.m))
+    tau, sigma = step_sizes(m)
+    assert cpu.advance(20, tau, sigma) == g.advance(20, tau, sigma)
+    for u, w in zip(g.candidates(), cpu.candidates()):
+        near(u, w, 1e-10)
