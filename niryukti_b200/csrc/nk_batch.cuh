@@ -388,7 +388,8 @@ class Batch {
         d_ctl_.alloc(size_t(o.capacity));
         d_mask_.alloc(size_t(o.capacity));
         d_src_.alloc(size_t(o.capacity));
-        cuda_check(cudaMemset(d_ctl_.p, 0, sizeof(BCtl) * size_t(o.capacity)), "controls");
+        cuda_check(cudaMemsetAsync(d_ctl_.p, 0, sizeof(BCtl) * size_t(o.capacity), stream_),
+                   "controls");
         cuda_check(cudaMallocHost(reinterpret_cast<void **>(&h_ctl_), sizeof(BCtl) * size_t(o.capacity)),
                    "pinned");
         std::memset(h_ctl_, 0, sizeof(BCtl) * size_t(o.capacity));
@@ -727,7 +728,10 @@ class Batch {
             throw Error(NK_ERR_MEMORY, "batch instance layout exceeds its estimate");
         cuda_check(cudaStreamSynchronize(stream_), "instance upload");
         const int b = int(&S - slots_.data());
-        cuda_check(cudaMemcpy(d_ins_.p + b, &d, sizeof(BInst), cudaMemcpyHostToDevice), "descriptor");
+        // every upload is on the batch's stream: a plain cudaMemcpy from pageable
+        // memory may land after its kernels have started
+        cuda_check(cudaMemcpyAsync(d_ins_.p + b, &d, sizeof(BInst), cudaMemcpyHostToDevice, stream_),
+                   "descriptor");
         // initial activity A x0 and control
         BCtl c{};
         c.factor = 1;
@@ -735,7 +739,8 @@ class Batch {
         c.active = 1;
         c.fp64 = f64 ? 1 : 0;
         h_ctl_[b] = c;
-        cuda_check(cudaMemcpy(d_ctl_.p + b, &c, sizeof(BCtl), cudaMemcpyHostToDevice), "control");
+        cuda_check(cudaMemcpyAsync(d_ctl_.p + b, &c, sizeof(BCtl), cudaMemcpyHostToDevice, stream_),
+                   "control");
         // initial activity A x0 with the values the trials use, each row summed
         // in CSR order (the device SpMV's order)
         std::vector<double> ax0(static_cast<size_t>(B.m), 0.0);
@@ -750,9 +755,12 @@ class Batch {
             ax0[size_t(r)] = sum;
         }
         if (B.m) {
-            cuda_check(cudaMemcpy(d.ax[0], ax0.data(), size_t(B.m) * 8, cudaMemcpyHostToDevice), "activity");
-            cuda_check(cudaMemcpy(d.ax[1], ax0.data(), size_t(B.m) * 8, cudaMemcpyHostToDevice), "activity");
+            for (double *ax : d.ax)
+                cuda_check(cudaMemcpyAsync(ax, ax0.data(), size_t(B.m) * 8, cudaMemcpyHostToDevice,
+                                           stream_),
+                           "activity");
         }
+        cuda_check(cudaStreamSynchronize(stream_), "instance upload"); // d, c, ax0 leave scope
     }
 
     // ---------------------------------------------------------------- lists
@@ -887,10 +895,11 @@ class Batch {
                 out[size_t(fill[size_t(owner[k])]++)] = items[k];
             ensure(W.items, out.size());
             ensure(W.coff, coff.size());
-            cuda_check(cudaMemcpy(W.items.p, out.data(), out.size() * sizeof(BWork),
-                                  cudaMemcpyHostToDevice), "lists");
-            cuda_check(cudaMemcpy(W.coff.p, coff.data(), coff.size() * sizeof(int),
-                                  cudaMemcpyHostToDevice), "lists");
+            cuda_check(cudaMemcpyAsync(W.items.p, out.data(), out.size() * sizeof(BWork),
+                                       cudaMemcpyHostToDevice, stream_), "lists");
+            cuda_check(cudaMemcpyAsync(W.coff.p, coff.data(), coff.size() * sizeof(int),
+                                       cudaMemcpyHostToDevice, stream_), "lists");
+            cuda_check(cudaStreamSynchronize(stream_), "lists"); // out, coff leave scope
             W.count = int(items.size());
             W.ncta = ncta;
         };
@@ -915,8 +924,8 @@ class Batch {
         auto up = [&](auto &d, const auto &h) {
             ensure(d, std::max<size_t>(1, h.size()));
             if (!h.empty())
-                cuda_check(cudaMemcpy(d.p, h.data(), h.size() * sizeof(h[0]), cudaMemcpyHostToDevice),
-                           "lists");
+                cuda_check(cudaMemcpyAsync(d.p, h.data(), h.size() * sizeof(h[0]),
+                                           cudaMemcpyHostToDevice, stream_), "lists");
         };
         up(d_cols_, cols);
         up(d_rows_, rows);
@@ -925,6 +934,7 @@ class Batch {
         up(d_cc_, cc);
         up(d_rf_, rf);
         up(d_rc_, rc);
+        cuda_check(cudaStreamSynchronize(stream_), "lists"); // the host lists leave scope
         ensure(d_pp_, size_t(std::max(1, ncols_)));
         ensure(d_pd_, size_t(std::max(1, 2 * nrows_)));
         ensure(d_pk_, size_t(std::max(1, ncols_ + nrows_)) * kBatchKkt);

@@ -336,8 +336,11 @@ struct DeviceSolve {
             d.alloc(size_t(std::max<int64_t>(1, len)));
             for (int64_t i = 0; i < len; ++i)
                 h[size_t(i)] = value(i);
-            if (len)
-                cuda_check(cudaMemcpy(d.p, h.data(), size_t(len) * 8, cudaMemcpyHostToDevice), "constants");
+            if (len) { // on the engine's stream, whose kernels read it; h is reused
+                cuda_check(cudaMemcpyAsync(d.p, h.data(), size_t(len) * 8, cudaMemcpyHostToDevice, s),
+                           "constants");
+                cuda_check(cudaStreamSynchronize(s), "constants");
+            }
         };
         put(cs, n, [&](int64_t i) { return prep.column_scale[size_t(cperm[size_t(i)])]; });
         put(olb, n, [&](int64_t i) { return orig.lb[size_t(prep.cols[size_t(cperm[size_t(i)])])]; });
