@@ -197,7 +197,10 @@ __global__ void __launch_bounds__(kBatchMaxThreads, 1024 / kBatchMaxThreads)
                     I.xa[j] = aj + (xj - aj) * pw;
                 if (sq)
                     g = g + (qa + qj * xj);
-                double t = (xj - tau * g) / (1 + tau * (sq ? 0. : qj));
+                const double den = 1 + tau * (sq ? 0. : qj);
+                double t = xj - tau * g;
+                if (den != 1) // x / 1 is x
+                    t = t / den;
                 t = t < lj ? lj : (uj < t ? uj : t);
                 xt[j] = t;
                 const double d = t - xj;
@@ -271,55 +274,86 @@ __global__ void __launch_bounds__(kBatchMaxThreads, 1024 / kBatchMaxThreads)
     }
 }
 
-// One warp per active instance: combine its chunk partials in list order and
-// apply the acceptance rule (decide() of nk_device.cuh without Halpern).
-__global__ void batch_decide(BCtl *ctl, const int *__restrict__ slots, int nslots,
-                             const int *col_first, const int *col_count, const int *row_first,
-                             const int *row_count, const double *part_p, const double *part_d) {
-    const int lane = threadIdx.x & 31;
-    const int warps = int((int64_t(gridDim.x) * blockDim.x) >> 5);
-    for (int k = int((int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5); k < nslots; k += warps) {
-        const int b = slots[k];
-        double p = 0, d = 0, c = 0;
-        for (int t = lane; t < col_count[k]; t += 32)
-            p += part_p[col_first[k] + t];
-        for (int t = lane; t < row_count[k]; t += 32) {
-            d += part_d[2 * (row_first[k] + t)];
-            c += part_d[2 * (row_first[k] + t) + 1];
-        }
-        p = warp_sum(p);
-        d = warp_sum(d);
-        c = warp_sum(c);
-        if (lane != 0)
-            continue;
-        BCtl &s = ctl[b];
-        if (!s.active)
-            continue;
-        const double factor = s.factor;
-        const double tau = s.tau * factor, sigma = s.sigma * factor;
-        const double energy = p / tau + d / sigma;
-        const double limit = fabs(c) > 0 ? energy / (2 * fabs(c)) : INFINITY;
-        const bool finite = isfinite(energy) && isfinite(c);
-        const bool accept = finite && (!s.adaptive || limit >= 1);
-        if (s.adaptive) {
-            const double kk = s.accepted + 2;
-            double mult = fmin((1 - pow(kk, -.3)) * limit, 1 + pow(kk, -.6));
-            if (!finite || !isfinite(mult) || mult <= 0)
-                mult = .5;
-            s.factor = clampd(factor * mult, 1e-12, 1e12);
-        }
-        s.accept = accept ? 1 : 0;
-        s.pending = 0;
-        if (accept) {
-            s.mass += factor;
-            s.accepted += 1;
-            s.weight = factor / s.mass;
-            s.cur ^= 1;
-            s.pending = 1;
-            s.pending_w = s.weight;
-        } else
-            s.rejected += 1;
+// The sum of part[0], part[step], ... (count of them) as one lane-strided pass and
+// a shuffle tree; 16 loads of each lane are in flight, the adds stay in order.
+__device__ __forceinline__ double strided_sum(const double *part, int count, int step) {
+    constexpr int U = 16;
+    double s = 0;
+    int t = threadIdx.x & 31;
+    for (; t + (U - 1) * 32 < count; t += U * 32) {
+        double a[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            a[u] = __ldcg(part + int64_t(step) * (t + u * 32));
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            s += a[u];
     }
+    double a[U - 1];
+#pragma unroll
+    for (int u = 0; u < U - 1; ++u)
+        a[u] = t + u * 32 < count ? __ldcg(part + int64_t(step) * (t + u * 32)) : 0.;
+#pragma unroll
+    for (int u = 0; u < U - 1; ++u)
+        if (t + u * 32 < count)
+            s += a[u];
+    return warp_sum(s);
+}
+
+// One CTA of four warps per active instance: dx^2, dy^2 and dy * delta each by one
+// warp, its chunk partials in list order, the powers of the acceptance rule by the
+// fourth; then the rule itself (decide() of nk_device.cuh without Halpern).  What
+// bounds it is the largest instance's chain of loads: with one warp for all three
+// sums, a few loads ahead, a trial of 96 instances of up to 100,000 columns took
+// 173 us, with this kernel 162.
+constexpr int kDecideThreads = 128;
+__global__ void __launch_bounds__(kDecideThreads)
+    batch_decide(BCtl *ctl, const int *__restrict__ slots, int nslots, const int *col_first,
+                 const int *col_count, const int *row_first, const int *row_count,
+                 const double *part_p, const double *part_d) {
+    __shared__ double v[5]; // p, d, c, and (accepted + 2) to the powers -.3 and -.6
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, k = blockIdx.x;
+    if (k >= nslots)
+        return;
+    BCtl &s = ctl[slots[k]];
+    if (!s.active)
+        return;
+    if (warp < 3) {
+        const double sum = warp == 0
+                               ? strided_sum(part_p + col_first[k], col_count[k], 1)
+                               : strided_sum(part_d + 2 * int64_t(row_first[k]) + (warp - 1),
+                                             row_count[k], 2);
+        if (lane == 0)
+            v[warp] = sum;
+    } else if (lane < 2 && s.adaptive)
+        v[3 + lane] = pow(s.accepted + 2, lane ? -.6 : -.3);
+    __syncthreads();
+    if (threadIdx.x != 0)
+        return;
+    const double p = v[0], d = v[1], c = v[2];
+    const double factor = s.factor;
+    const double tau = s.tau * factor, sigma = s.sigma * factor;
+    const double energy = p / tau + d / sigma;
+    const double limit = fabs(c) > 0 ? energy / (2 * fabs(c)) : INFINITY;
+    const bool finite = isfinite(energy) && isfinite(c);
+    const bool accept = finite && (!s.adaptive || limit >= 1);
+    if (s.adaptive) {
+        double mult = fmin((1 - v[3]) * limit, 1 + v[4]);
+        if (!finite || !isfinite(mult) || mult <= 0)
+            mult = .5;
+        s.factor = clampd(factor * mult, 1e-12, 1e12);
+    }
+    s.accept = accept ? 1 : 0;
+    s.pending = 0;
+    if (accept) {
+        s.mass += factor;
+        s.accepted += 1;
+        s.weight = factor / s.mass;
+        s.cur ^= 1;
+        s.pending = 1;
+        s.pending_w = s.weight;
+    } else
+        s.rejected += 1;
 }
 
 // ------------------------------------------------------------------ element work
