@@ -11,7 +11,9 @@ results as instances finish.  Every call goes through libnkpdhg.so.
 from __future__ import annotations
 
 import ctypes as C
+import os
 import threading
+from concurrent.futures import ThreadPoolExecutor
 
 import numpy as np
 
@@ -213,10 +215,12 @@ def estimate_bytes(model) -> float:
 
 
 def solve_batch(models, **options) -> list:
-    """Solve every model; results in input order.  Instances that do not fit
-    the memory budget wait and join as earlier ones finish."""
+    """Solve every model; results in input order.  Models are prepared on all host
+    cores.  Instances that do not fit the memory budget wait and join as earlier
+    ones finish."""
     with BatchEngine(**options) as eng:
-        items = [eng.prepare(m) for m in models]
+        with ThreadPoolExecutor(max_workers=max(1, min(len(models), os.cpu_count() or 1))) as pool:
+            items = list(pool.map(eng.prepare, models))
         results = [None] * len(models)
         waiting = list(range(len(models)))
         while waiting or eng.info()["active"]:
