@@ -747,12 +747,16 @@ __global__ void restart_point(int64_t n, int64_t m, const int64_t *col_perm,
 }
 
 // ------------------------------------------------------------------ plain SpMV
-// out = M x (engine order on both sides, FP64 accumulation): activity rebasing
-// and the monitor.
+// out = M x (engine order on both sides, FP64 accumulation): activity rebasing,
+// the monitor and the candidates; two vectors in one launch with gridDim.y = 2
+// (a matrix without rows split across chunks: those meet in M's slots).
 template <class V, class I>
-__global__ void __launch_bounds__(kThreads) spmv_kernel(Sell<V, I> M, const double *x,
-                                                        double *out) {
+__global__ void __launch_bounds__(kThreads) spmv_kernel(Sell<V, I> M, const double *x0,
+                                                        double *out0, const double *x1,
+                                                        double *out1) {
     __shared__ double wpart[kWarps][32];
+    const double *x = blockIdx.y ? x1 : x0;
+    double *out = blockIdx.y ? out1 : out0;
     const int lane = threadIdx.x & 31;
     for (int64_t ch = first_chunk(); ch * 32 < M.nv; ch += chunk_stride()) {
         const int64_t vr = ch * 32 + lane;

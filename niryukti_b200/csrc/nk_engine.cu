@@ -694,26 +694,40 @@ struct Engine {
     int vbits() const { return precision == NK_PRECISION_FP64 ? 64 : 32; }
 
     template <class V, class I>
-    void spmv_t(const SellMatrix &M, const double *xin, double *out) {
+    void spmv_t(const SellMatrix &M, const double *x0, double *out0, const double *x1,
+                double *out1) {
         if (M.nv == 0)
             return;
         int g = int(std::max<int64_t>(1, std::min<int64_t>((M.nv / 32 + kWarps) / kWarps, grid_s)));
-        spmv_kernel<V, I><<<g, kThreads, 0, stream>>>(M.view<V, I>(), xin, out);
+        spmv_kernel<V, I><<<dim3(unsigned(g), x1 ? 2 : 1), kThreads, 0, stream>>>(
+            M.view<V, I>(), x0, out0, x1, out1);
+    }
+    void spmv_v(const SellMatrix &M, const double *x0, double *out0, const double *x1,
+                double *out1) {
+        if (M.vbits == 64) {
+            if (M.wide)
+                spmv_t<double, int64_t>(M, x0, out0, x1, out1);
+            else
+                spmv_t<double, int32_t>(M, x0, out0, x1, out1);
+        } else {
+            if (M.wide)
+                spmv_t<float, int64_t>(M, x0, out0, x1, out1);
+            else
+                spmv_t<float, int32_t>(M, x0, out0, x1, out1);
+        }
+        cuda_check(cudaGetLastError(), "spmv launch");
     }
     // out = M * xin with FP64 accumulation (activity rebasing, the monitor).
     void spmv(const SellMatrix &M, const double *xin, double *out) {
-        if (M.vbits == 64) {
-            if (M.wide)
-                spmv_t<double, int64_t>(M, xin, out);
-            else
-                spmv_t<double, int32_t>(M, xin, out);
-        } else {
-            if (M.wide)
-                spmv_t<float, int64_t>(M, xin, out);
-            else
-                spmv_t<float, int32_t>(M, xin, out);
-        }
-        cuda_check(cudaGetLastError(), "spmv launch");
+        spmv_v(M, xin, out, nullptr, nullptr);
+    }
+    // The products of two vectors, in one launch where M allows it.
+    void spmv_pair(const SellMatrix &M, const double *x0, double *out0, const double *x1,
+                   double *out1) {
+        if (M.ncounters == 0)
+            return spmv_v(M, x0, out0, x1, out1);
+        spmv(M, x0, out0);
+        spmv(M, x1, out1);
     }
     // out = Q xin (FP64 sums)
     void q_spmv(const double *xin, double *out) {

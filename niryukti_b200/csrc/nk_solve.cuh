@@ -74,7 +74,54 @@ __device__ void block_combine(double (&v)[NV], unsigned max_mask, double *smem /
         }
 }
 
-__global__ void __launch_bounds__(kThreads) kkt_partial(KktArgs a, double *part) {
+// Combines `blocks` rows of NV partials into out[0..NV) with one CTA, in a
+// fixed order (deterministic).
+template <int NV>
+__device__ __forceinline__ void finish_partials(const double *part, int blocks, unsigned max_mask,
+                                                double *out, double *smem /* kWarps*NV */) {
+    double v[NV];
+#pragma unroll
+    for (int t = 0; t < NV; ++t)
+        v[t] = 0;
+    for (int b = threadIdx.x; b < blocks; b += blockDim.x)
+#pragma unroll
+        for (int t = 0; t < NV; ++t) {
+            double p = __ldcg(part + b * NV + t);
+            v[t] = (max_mask >> t & 1) ? fmax(v[t], p) : v[t] + p;
+        }
+    block_combine<NV>(v, max_mask, smem);
+    if (threadIdx.x == 0)
+#pragma unroll
+        for (int t = 0; t < NV; ++t)
+            out[t] = v[t];
+}
+
+// The end of a kernel whose CTAs (gridDim.x of them for each blockIdx.y) each have
+// NV values in thread 0: the last CTA of a row combines them, so that no second
+// launch has to.
+template <int NV>
+__device__ __forceinline__ void close_partials(const double (&v)[NV], double *part, unsigned *arrive,
+                                               unsigned max_mask, double *out, double *smem) {
+    __shared__ bool last;
+    if (threadIdx.x == 0) {
+        for (int t = 0; t < NV; ++t)
+            part[blockIdx.x * NV + t] = v[t];
+        __threadfence();
+        last = atomicAdd(arrive, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last)
+        return;
+    __threadfence();
+    finish_partials<NV>(part, int(gridDim.x), max_mask, out, smem);
+    if (threadIdx.x == 0)
+        *arrive = 0;
+}
+
+// The candidates by blockIdx.y; out gets kKktValues each.
+__global__ void __launch_bounds__(kThreads) kkt_candidates(KktArgs a0, KktArgs a1, double *part,
+                                                           unsigned *arrive, double *out) {
+    const KktArgs &a = blockIdx.y ? a1 : a0;
     __shared__ double smem[kWarps * kKktValues];
     double v[kKktValues] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
     const int64_t stride = int64_t(gridDim.x) * blockDim.x;
@@ -146,39 +193,16 @@ __global__ void __launch_bounds__(kThreads) kkt_partial(KktArgs a, double *part)
         }
     }
     block_combine<kKktValues>(v, kKktMaxMask, smem);
-    if (threadIdx.x == 0)
-        for (int t = 0; t < kKktValues; ++t)
-            part[blockIdx.x * kKktValues + t] = v[t];
-}
-
-// Combines `blocks` rows of NV partials into out[0..NV) with one CTA, in a
-// fixed order (deterministic).
-template <int NV>
-__global__ void __launch_bounds__(kThreads) finish_partials(const double *part, int blocks,
-                                                            unsigned max_mask, double *out) {
-    __shared__ double smem[kWarps * NV];
-    double v[NV];
-#pragma unroll
-    for (int t = 0; t < NV; ++t)
-        v[t] = 0;
-    for (int b = threadIdx.x; b < blocks; b += blockDim.x)
-#pragma unroll
-        for (int t = 0; t < NV; ++t) {
-            double p = part[b * NV + t];
-            v[t] = (max_mask >> t & 1) ? fmax(v[t], p) : v[t] + p;
-        }
-    block_combine<NV>(v, max_mask, smem);
-    if (threadIdx.x == 0)
-#pragma unroll
-        for (int t = 0; t < NV; ++t)
-            out[t] = v[t];
+    close_partials<kKktValues>(v, part + blockIdx.y * gridDim.x * kKktValues, arrive + blockIdx.y,
+                               kKktMaxMask, out + blockIdx.y * kKktValues, smem);
 }
 
 // Sum (a - b)^2 over n columns and over m rows (restart displacement).
 __global__ void __launch_bounds__(kThreads) displacement_partial(int64_t n, int64_t m,
                                                                  const double *x, const double *ex,
                                                                  const double *y, const double *ey,
-                                                                 double *part) {
+                                                                 double *part, unsigned *arrive,
+                                                                 double *out) {
     __shared__ double smem[kWarps * 2];
     double v[2] = {0, 0};
     const int64_t stride = int64_t(gridDim.x) * blockDim.x;
@@ -194,10 +218,7 @@ __global__ void __launch_bounds__(kThreads) displacement_partial(int64_t n, int6
         }
     }
     block_combine<2>(v, 0u, smem);
-    if (threadIdx.x == 0) {
-        part[blockIdx.x * 2] = v[0];
-        part[blockIdx.x * 2 + 1] = v[1];
-    }
+    close_partials<2>(v, part, arrive, 0u, out, smem);
 }
 
 // Farkas screen of a candidate ray r = y - ey (ey may be null) with
@@ -209,10 +230,15 @@ __global__ void __launch_bounds__(kThreads) displacement_partial(int64_t n, int6
 // 1 + 2 that bound in plain FP64 (-sum r_i b_i + sum_j min over the box of
 // (A^T r)_j x_j); 3 the magnitude of its terms.
 constexpr int kRayValues = 4;
-__global__ void __launch_bounds__(kThreads) ray_screen(int64_t n, int64_t m, const double *y,
-                                                       const double *ey, const double *aty,
-                                                       const double *atey, KktArgs a,
-                                                       double *part) {
+// Four rays by blockIdx.y: candidate 0's y and candidate 1's, then each less the
+// epoch's.
+struct RayArgs {
+    const double *y[2], *aty[2], *ey, *atey;
+};
+__global__ void __launch_bounds__(kThreads) ray_screen(int64_t n, int64_t m, RayArgs rays, KktArgs a,
+                                                       double *part, unsigned *arrive, double *out) {
+    const double *y = rays.y[blockIdx.y & 1], *aty = rays.aty[blockIdx.y & 1];
+    const double *ey = blockIdx.y & 2 ? rays.ey : nullptr, *atey = blockIdx.y & 2 ? rays.atey : nullptr;
     __shared__ double smem[kWarps * kRayValues];
     double v[kRayValues] = {0, 0, 0, 0};
     const int64_t stride = int64_t(gridDim.x) * blockDim.x;
@@ -244,9 +270,8 @@ __global__ void __launch_bounds__(kThreads) ray_screen(int64_t n, int64_t m, con
         }
     }
     block_combine<kRayValues>(v, 1u, smem);
-    if (threadIdx.x == 0)
-        for (int t = 0; t < kRayValues; ++t)
-            part[blockIdx.x * kRayValues + t] = v[t];
+    close_partials<kRayValues>(v, part + blockIdx.y * gridDim.x * kRayValues, arrive + blockIdx.y, 1u,
+                               out + blockIdx.y * kRayValues, smem);
 }
 
 // ------------------------------------------------------------------ driver
@@ -275,9 +300,9 @@ struct DeviceSolve {
     std::unique_ptr<Engine> E;
     int64_t n = 0, m = 0;
     DevBuf<double> cs, olb, oub, rs, shift, orl, oru;       // KKT constants, engine order
-    DevBuf<double> k_ax, k_aty[2], k_qx, best_x, best_y, epoch_x, epoch_y, epoch_aty, part, out;
-    double *host_out = nullptr; // pinned: 2 candidates x kKktValues, 2 displacement sums,
-                                // 3 rays x kRayValues
+    DevBuf<double> k_ax[2], k_aty[2], k_qx[2], best_x, best_y, epoch_x, epoch_y, epoch_aty, part, out;
+    DevBuf<unsigned> arrive; // of the reductions in flight: zero between launches
+    double *host_out = nullptr; // pinned copy of out
     int grid = 148;
     double os = 1, cscale = 1, offset_o = 0, offset_s = 0, cfixed = 0;
     bool orig_is_qp = false; // the caller's model has quadratic terms (cached: O(n) to test)
@@ -368,11 +393,13 @@ struct DeviceSolve {
             put(shift, m, [&](int64_t i) { return sh[size_t(rperm[size_t(i)])]; });
         }
         auto vec = [&](DevBuf<double> &d, int64_t len) { d.alloc(size_t(std::max<int64_t>(1, len))); };
-        vec(k_ax, m);
+        vec(k_ax[0], m);
+        vec(k_ax[1], m);
         vec(k_aty[0], n);
         vec(k_aty[1], n);
         vec(epoch_aty, n);
-        vec(k_qx, n);
+        vec(k_qx[0], E->sparse_q ? n : 0);
+        vec(k_qx[1], E->sparse_q ? n : 0);
         vec(best_x, n);
         vec(best_y, m);
         vec(epoch_x, n);
@@ -381,8 +408,10 @@ struct DeviceSolve {
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         grid = int(std::max<int64_t>(1, std::min<int64_t>(int64_t(sms) * 4, (std::max(n, m) + kThreads - 1) / kThreads)));
-        part.alloc(size_t(grid) * std::max(kKktValues, kRayValues));
+        part.alloc(size_t(grid) * std::max(2 * kKktValues, 4 * kRayValues));
         out.alloc(kOutValues);
+        arrive.alloc(4);
+        cuda_check(cudaMemsetAsync(arrive.p, 0, arrive.bytes(), s), "driver setup");
         cuda_check(cudaMallocHost(reinterpret_cast<void **>(&host_out), kOutValues * sizeof(double)),
                    "pinned");
         int cur = current();
@@ -392,8 +421,9 @@ struct DeviceSolve {
         cuda_check(cudaStreamSynchronize(s), "driver setup");
     }
 
-    static constexpr int kOutValues = 2 * kKktValues + 2 + 3 * kRayValues;
-    static constexpr int kRayOut = 2 * kKktValues + 2;
+    // out: the candidates' KKT values, four rays, the displacement
+    static constexpr int kRayOut = 2 * kKktValues, kMoveOut = kRayOut + 4 * kRayValues,
+                         kOutValues = kMoveOut + 2;
 
     // epoch = current iterate (after a restart), with its A^T epoch_y
     void set_epoch(int cur) {
@@ -414,57 +444,42 @@ struct DeviceSolve {
         return E->host_ctl->cur;
     }
 
-    // Launches the evaluation of the prepared point (x, y) into out[slot]; the
-    // products A x, A^T y (and Q x) are recomputed, not taken from the
-    // engine's incrementally updated activity.
     KktArgs args(const double *x, const double *y, int slot) {
-        return KktArgs{n, m, x, y, k_ax.p, k_aty[slot].p, E->sparse_q ? k_qx.p : nullptr, E->c.p,
-                       E->q.p, cs.p, olb.p, oub.p, rs.p, shift.p, orl.p, oru.p, os, cscale,
+        return KktArgs{n, m, x, y, k_ax[slot].p, k_aty[slot].p, E->sparse_q ? k_qx[slot].p : nullptr,
+                       E->c.p, E->q.p, cs.p, olb.p, oub.p, rs.p, shift.p, orl.p, oru.p, os, cscale,
                        E->sparse_q ? 1 : 0};
     }
-    void evaluate(const double *x, const double *y, int slot) {
+    // Launches the evaluation of the prepared points (x, y)[0] and [1] into out; the
+    // products A x, A^T y (and Q x) are recomputed, not taken from the engine's
+    // incrementally updated activity.  With `rays` also the screen of the
+    // candidate rays.  Small models' checks are launches and waits: both points
+    // share each launch, reductions end in their own, and one transfer brings all.
+    void evaluate(const double *const (&x)[2], const double *const (&y)[2], bool rays) {
         cudaStream_t s = E->stream;
         if (m)
-            E->spmv(E->A, x, k_ax.p);
+            E->spmv_pair(E->A, x[0], k_ax[0].p, x[1], k_ax[1].p);
         if (n)
-            E->spmv(E->At, y, k_aty[slot].p);
+            E->spmv_pair(E->At, y[0], k_aty[0].p, y[1], k_aty[1].p);
         if (E->sparse_q)
-            E->q_spmv(x, k_qx.p);
-        KktArgs a = args(x, y, slot);
-        kkt_partial<<<grid, kThreads, 0, s>>>(a, part.p);
-        finish_partials<kKktValues><<<1, kThreads, 0, s>>>(part.p, grid, kKktMaxMask,
-                                                          out.p + slot * kKktValues);
+            for (int k = 0; k < 2; ++k)
+                E->q_spmv(x[k], k_qx[k].p);
+        kkt_candidates<<<dim3(unsigned(grid), 2), kThreads, 0, s>>>(
+            args(x[0], y[0], 0), args(x[1], y[1], 1), part.p, arrive.p, out.p);
+        if (rays)
+            ray_screen<<<dim3(unsigned(grid), 4), kThreads, 0, s>>>(
+                n, m, RayArgs{{y[0], y[1]}, {k_aty[0].p, k_aty[1].p}, epoch_y.p, epoch_aty.p},
+                args(nullptr, nullptr, 0), part.p, arrive.p, out.p + kRayOut);
         cuda_check(cudaGetLastError(), "kkt evaluation");
+        fetch(0, rays ? kMoveOut : kRayOut);
     }
-    void displacement(const double *x, const double *y) {
-        cudaStream_t s = E->stream;
-        displacement_partial<<<grid, kThreads, 0, s>>>(n, m, x, epoch_x.p, y, epoch_y.p, part.p);
-        finish_partials<2><<<1, kThreads, 0, s>>>(part.p, grid, 0u, out.p + 2 * kKktValues);
-        cuda_check(cudaGetLastError(), "displacement");
-    }
-    // Screens the three candidate rays of the infeasibility test on the device:
-    // ray 0 the chosen candidate's y (slot `chosen`), ray 1 the other one's,
-    // ray 2 the chosen y minus the epoch y.  Returns, per ray, whether the
-    // outward-rounded host bound could still be positive.
-    std::array<bool, 3> screen_rays(const double *y_chosen, int chosen, const double *y_other) {
-        cudaStream_t s = E->stream;
-        const double *ys[3] = {y_chosen, y_other, y_chosen};
-        const double *eys[3] = {nullptr, nullptr, epoch_y.p};
-        const double *atys[3] = {k_aty[chosen].p, k_aty[1 - chosen].p, k_aty[chosen].p};
-        const double *ateys[3] = {nullptr, nullptr, epoch_aty.p};
-        KktArgs a = args(nullptr, nullptr, 0);
-        for (int r = 0; r < 3; ++r) {
-            ray_screen<<<grid, kThreads, 0, s>>>(n, m, ys[r], eys[r], atys[r], ateys[r], a, part.p);
-            finish_partials<kRayValues><<<1, kThreads, 0, s>>>(part.p, grid, 1u,
-                                                               out.p + kRayOut + r * kRayValues);
-        }
-        cuda_check(cudaGetLastError(), "ray screen");
-        cuda_check(cudaMemcpyAsync(host_out + kRayOut, out.p + kRayOut, 3 * kRayValues * 8,
-                                   cudaMemcpyDeviceToHost, s), "ray screen");
-        cuda_check(cudaStreamSynchronize(s), "ray screen");
+    // Whether the outward-rounded host bound of each ray of the infeasibility test
+    // could still be positive (after evaluate with rays): ray 0 the chosen
+    // candidate's y, ray 1 the other one's, ray 2 the chosen y minus the epoch y.
+    std::array<bool, 3> screened_rays(int chosen) const {
+        const int ray[3] = {chosen, 1 - chosen, 2 + chosen};
         std::array<bool, 3> ok{};
         for (int r = 0; r < 3; ++r) {
-            const double *v = host_out + kRayOut + r * kRayValues;
+            const double *v = host_out + kRayOut + ray[r] * kRayValues;
             // FP64 sums of the bound's terms err by far less than 1e-9 of their
             // magnitude: at or below that margin the exact bound cannot be
             // positive (a zero ray has bound 0 and magnitude 0)
@@ -472,8 +487,17 @@ struct DeviceSolve {
         }
         return ok;
     }
-    void fetch(int values) {
-        cuda_check(cudaMemcpyAsync(host_out, out.p, size_t(values) * 8, cudaMemcpyDeviceToHost, E->stream),
+    // {sum (x - epoch x)^2, sum (y - epoch y)^2}
+    std::pair<double, double> displacement(const double *x, const double *y) {
+        displacement_partial<<<grid, kThreads, 0, E->stream>>>(n, m, x, epoch_x.p, y, epoch_y.p,
+                                                               part.p, arrive.p, out.p + kMoveOut);
+        cuda_check(cudaGetLastError(), "displacement");
+        fetch(kMoveOut, 2);
+        return {host_out[kMoveOut], host_out[kMoveOut + 1]};
+    }
+    void fetch(int first, int values) {
+        cuda_check(cudaMemcpyAsync(host_out + first, out.p + first, size_t(values) * 8,
+                                   cudaMemcpyDeviceToHost, E->stream),
                    "evaluation result");
         cuda_check(cudaStreamSynchronize(E->stream), "evaluation sync");
     }
@@ -591,9 +615,8 @@ struct Driver {
             previous_rejected = E.rejected;
             tick = SteadyClock::now();
             int cur = D.current();
-            D.evaluate(E.x[cur].p, E.y[cur].p, 0);
-            D.evaluate(E.xa.p, E.ya.p, 1);
-            D.fetch(2 * kKktValues);
+            const double *const px[2] = {E.x[cur].p, E.xa.p}, *const py[2] = {E.y[cur].p, E.ya.p};
+            D.evaluate(px, py, certify && R.iterations >= 1000);
             R.device_checks++;
             checks++;
             Accuracy ca = D.finish(D.host_out), aa = D.finish(D.host_out + kKktValues);
@@ -645,7 +668,7 @@ struct Driver {
             if (certify && R.iterations >= 1000 && ca.primal > o.tol) {
                 tick = SteadyClock::now();
                 const double *other_y = avg ? E.y[cur].p : E.ya.p;
-                auto ok = D.screen_rays(cy, avg ? 1 : 0, other_y);
+                auto ok = D.screened_rays(avg ? 1 : 0);
                 if ((ok[0] || ok[1] || ok[2]) &&
                     infeasible(ok[0] ? cy : nullptr, ok[1] ? other_y : nullptr,
                                ok[2] ? cy : nullptr))
@@ -665,11 +688,7 @@ struct Driver {
                                 since_restart >= std::max<int64_t>(2000, R.iterations / 2));
             if (o.restart && restart_due) {
                 if (o.adaptive) {
-                    D.displacement(cx, cy);
-                    cuda_check(cudaMemcpyAsync(D.host_out + 2 * kKktValues, D.out.p + 2 * kKktValues,
-                                               16, cudaMemcpyDeviceToHost, E.stream), "displacement");
-                    cuda_check(cudaStreamSynchronize(E.stream), "displacement");
-                    double dx = D.host_out[2 * kKktValues], dy = D.host_out[2 * kKktValues + 1];
+                    const auto [dx, dy] = D.displacement(cx, cy);
                     if (dx > 1e-24 && dy > 1e-24) {
                         double target_w = std::clamp(std::sqrt(dy / dx), 1e-4, 1e4);
                         weight = std::sqrt(weight * target_w);

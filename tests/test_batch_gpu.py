@@ -128,3 +128,33 @@ def test_autotuner_reports_a_variant(batch):
         assert info["dual_variant"]["threads"] in (128, 256, 512)
         ms, bts = eng.time_trials(10)
         assert ms > 0 and bts > 0
+
+
+@pytest.mark.parametrize("m", [16, 257, 8160, 8200])
+def test_decision_sums_over_many_chunks(gpu, m):
+    """The decision adds an instance's chunk partials lane by lane, 16 strides ahead:
+    one chunk, a few, and 510 and 513 column chunks (one side and the other of a
+    whole turn).  Against the single solve over one check of 20 trials, whose step
+    sums are grouped otherwise: adaptive steps carry last-bit differences forward
+    about tenfold every eight trials, so 20 trials leave them below 1e-12; held to
+    1e-9, where a lost or doubled partial moves the first step by its share."""
+    from niryukti_b200 import batch, solver
+    model = synth.random_lp(m=m, n=2 * m, per_col=4, seed=m)
+    options = dict(iteration_limit=20, check_every=20, tol=1e-12)
+    a = batch.solve_batch([model], **options)[0]
+    b = solver.solve(model, **options)
+    assert a["iterations"] == b["iterations"]
+    assert np.max(np.abs(a["x"] - b["x"])) <= 1e-9 * (1 + np.max(np.abs(b["x"])))
+    assert abs(a["kkt"] - b["kkt"]) <= 1e-9 * (1 + b["kkt"])
+
+
+def test_placement_tuning_changes_no_result(gpu):
+    """With 64 or more instances the tuner also tries its items dealt; results are
+    those of an untuned batch, bit for bit."""
+    from niryukti_b200 import batch
+    models = [synth.random_lp(m=40 + 3 * k, n=90 + 7 * k, per_col=4, seed=k) for k in range(70)]
+    tuned, plain = (batch.solve_batch(models, iteration_limit=300, autotune=flag)
+                    for flag in (True, False))
+    for u, w in zip(tuned, plain):
+        assert u["iterations"] == w["iterations"]
+        assert np.array_equal(u["x"], w["x"]) and np.array_equal(u["y"], w["y"])
