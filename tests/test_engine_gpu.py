@@ -690,3 +690,32 @@ def test_long_rows_past_the_resident_size(gpu, oracle, nnz, len_hi, panels, prec
     assert cpu.advance(20, tau, sigma) == g.advance(20, tau, sigma)
     for u, w in zip(g.candidates(), cpu.candidates()):
         near(u, w, 1e-10)
+
+
+def test_resident_trials_from_several_threads(gpu):
+    """Four engines advanced from four threads at once, each on its own stream: the
+    resident grids take every SM, so they must run one after the other, whole; each
+    engine ends where it ends alone, bit for bit."""
+    import threading
+    models = [synth.random_lp(m=m, n=n, per_col=4, seed=m) for m, n in
+              ((400, 1000), (9000, 20000), (2000, 5000), (20000, 50001))]
+    steps = [step_sizes(m) for m in models]
+
+    def run(k, out):
+        g = gpu.PdhgBackend(models[k], adaptive=True, graphs=True)
+        for _ in range(25):
+            g.advance(40, *steps[k])
+        out[k] = g.candidates()
+
+    alone, together = {}, {}
+    for k in range(4):
+        run(k, alone)
+    threads = [threading.Thread(target=run, args=(k, together)) for k in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert len(together) == 4
+    for k in range(4):
+        for u, w in zip(alone[k], together[k]):
+            assert np.array_equal(u, w)
