@@ -124,7 +124,7 @@ nk_status nk_pdhg_stats(nk_pdhg *h, int64_t *trials, int64_t *device_bytes);
  * + decision) steps in milliseconds; the dual step includes the panel kernel
  * when A's long rows are stored by column panel.  With graphs on, each trial
  * replays one captured trial whose events are graph nodes, as the graph path
- * runs it.  The trials advance the iterate. */
+ * runs it.  The trials advance the iterate as nk_pdhg_advance's do, bit for bit. */
 nk_status nk_pdhg_profile(nk_pdhg *h, int count, double tau, double sigma, double *ms_primal,
                           double *ms_dual);
 /* The same, kernel by kernel: ms[0] the primal kernel, ms[1] the panel kernel
@@ -136,7 +136,9 @@ nk_status nk_pdhg_profile_kernels(nk_pdhg *h, int count, double tau, double sigm
  * panel width in columns, the number of panels, the number of runs (a long
  * row's entries in one panel, cut into pieces of 64 or more entries where
  * they would hold up a lane; each run has its own partial sum) (all 0 without
- * panels), and the kernel launches per trial.  Null outputs are skipped. */
+ * panels), and the kernel launches of a trial that runs as kernels of its own
+ * (nk_pdhg_profile; nk_pdhg_advance runs a small or medium model's trials
+ * together in one launch).  Null outputs are skipped. */
 nk_status nk_pdhg_layout_info(nk_pdhg *h, int64_t *long_rows, int64_t *panel_width,
                               int *panels, int64_t *runs, int *kernels_per_trial);
 /* Profiling (no reference counterpart): mean duration in milliseconds of `reps`

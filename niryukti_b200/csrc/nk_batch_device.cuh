@@ -14,7 +14,7 @@
 //
 // One PDHG trial of the whole batch is three launches: batch_primal (A^T y,
 // projected primal step), batch_dual (A dx, interval prox) and batch_decide
-// (one warp per instance: the acceptance rule and step-size update of
+// (one CTA per instance: the acceptance rule and step-size update of
 // src/cuda.cu:285-335, i.e. the single engine's decide() without Halpern).
 #pragma once
 

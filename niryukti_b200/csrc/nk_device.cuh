@@ -1,6 +1,8 @@
 // Kernels of the B200 PDHG engine (host side: nk_engine.cu).
 //
-// One PDHG trial is two kernels over SELL-32 matrices (nk_sell.cuh):
+// One PDHG trial of a large model is two kernels over SELL-32 matrices
+// (nk_sell.cuh); smaller models' trials run inside one launch (nk_resident.cuh),
+// with the same arithmetic:
 //   (q_rows_kernel Q x of the current iterate, for a sparse Q)
 //   primal_kernel  g = c + A^T y (+ Q x + q.x)   -- one lane per row of A^T
 //                  trial x = clamp((x - tau g)/(1 + tau q), lb, ub), dx, sum dx^2

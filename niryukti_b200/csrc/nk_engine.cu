@@ -1718,8 +1718,8 @@ std::vector<int> own_ranges(const std::vector<int32_t> &chunk_len, int parts) {
 }
 
 // Turns the resident kernel on (nk_resident.cuh) for a model that it can run as the
-// kernel path does, bit for bit (with column panels, up to the rounding of the
-// long rows' sums): 32-bit indices, FP64 sums, no row split across chunks; and
+// kernel path does, bit for bit (with column panels, which only fixed and Halpern
+// steps reach here, up to the rounding of the long rows' sums): 32-bit indices, FP64 sums, no row split across chunks; and
 // that fits: a CTA's products of either matrix and its rows' state in shared
 // memory (up to about 1.5 M entries).  Up to there it is the faster path,
 // measured in us a trial on LPs with 6 entries per column (FP64, adaptive),
@@ -2112,7 +2112,13 @@ Engine *create_engine(const nk_csr *Ah, const nk_csr *Qh, const double *hc, cons
         E->wide ? attach_slots<double, float, int64_t>(*E) : attach_slots<double, float, int32_t>(*E);
     else
         E->wide ? attach_slots<float, float, int64_t>(*E) : attach_slots<float, float, int32_t>(*E);
-    {
+    // Adaptive steps amplify a difference of rounding about tenfold every few
+    // trials, so a model whose long rows the panels sum keeps its panels, and their
+    // order of addition, under them.  (4 x 4,000 rows of a block-angular LP with 372
+    // linking rows: the sequential sums' iterates, as accurate, were 5e-8 away after
+    // 40 trials.)  Fixed and Halpern steps don't amplify it.
+    const bool panel_order = E->panels && E->adaptive;
+    if (!panel_order) {
         std::vector<int64_t> engine_rlen(static_cast<size_t>(m)); // longest first
         for (int64_t i = 0; i < m; ++i)
             engine_rlen[size_t(i)] = rlen[size_t(rperm[size_t(i)])];
@@ -2124,8 +2130,8 @@ Engine *create_engine(const nk_csr *Ah, const nk_csr *Qh, const double *hc, cons
     // 2.4 M (power-law, 4 M) 75 / 52, 2.4 M (block-angular) 59 / 49, 3 M 63 / 56,
     // 9 M 81 / 91.  (FP32 sums keep them: their rounding is the panels'.  So do
     // resident models, whose profiled kernels use them.)
-    if (E->panels && !E->resident.on && !E->wide && o->precision != NK_PRECISION_FP32 &&
-        E->pan.entries < NK_PANEL_MIN_ENTRIES) {
+    if (E->panels && !panel_order && !E->resident.on && !E->wide &&
+        o->precision != NK_PRECISION_FP32 && E->pan.entries < NK_PANEL_MIN_ENTRIES) {
         E->panels = false;
         E->pan = PanelMatrix{};
         use_schedule(E->A, lists_a, s);

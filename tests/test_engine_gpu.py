@@ -557,6 +557,19 @@ def test_resident_trials_match_the_kernel_path(gpu, kind, method):
         assert a.rejected_steps() > 0
 
 
+def test_adaptive_steps_keep_the_panels_order(gpu):
+    """Adaptive steps amplify rounding, so a model with column panels runs them
+    under advance() too: its points are the profiled panel kernels', bit for bit."""
+    m = synth.power_law_lp(m=3000, n=6000, nnz=60000, seed=4, len_hi=3000)
+    tau, sigma = step_sizes(m)
+    a, b = (gpu.PdhgBackend(m, adaptive=True, graphs=True) for _ in range(2))
+    assert a.layout_info()["panels"] > 0
+    a.advance(80, tau, sigma)
+    b.profile_kernels(80, tau, sigma)
+    for u, w in zip(a.candidates(), b.candidates()):
+        assert np.array_equal(u, w)
+
+
 def test_panel_engines_of_different_widths_coexist(gpu):
     """Two engines whose panels differ in width: the kernel's shared-memory limit
     belongs to both, so the wider one still runs after the narrower was built."""
