@@ -1833,7 +1833,7 @@ void plan_resident(Engine &E, const CtaLists &lists_t, const CtaLists &lists_a,
     R.slot_a = R.slot_t + st.size();
     R.own_q = R.slot_a + sa.size();
     R.sync = reinterpret_cast<unsigned *>(P.lists.p + lists.size() - 2);
-    const size_t np = size_t(R.lists_p) * R.width_p, nd = size_t(2) * R.lists_d * R.width_d;
+    const size_t np = size_t(2) * R.lists_p * R.width_p, nd = size_t(4) * R.lists_d * R.width_d;
     P.work.alloc(np + nd + kResWords + (E.halpern ? size_t(E.n + E.m) : 0));
     cuda_check(cudaMemsetAsync(P.work.p, 0, P.work.bytes(), s), "resident buffers");
     R.sum_p = P.work.p;

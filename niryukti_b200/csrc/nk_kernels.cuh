@@ -23,6 +23,21 @@ template <class T> __device__ __forceinline__ T stream_load(const T *p) {
 }
 template <class T> __device__ __forceinline__ T gather_load(const T *p) { return __ldg(p); }
 
+// Exchange between the CTAs of a cooperative grid: an arrival releases the CTA's
+// writes (those of its other threads too, after a CTA barrier), and a thread that
+// has seen the count acquires them (for its CTA after another CTA barrier).
+// Every acquire drops the SM's L1.  Polling with it is cheaper than relaxed polls
+// and one fence behind them: 6.6 against 7.3 us a trial of the resident kernel on
+// a 2,000 x 5,000 LP.
+__device__ __forceinline__ void release_arrival(unsigned *counter) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(counter) : "memory");
+}
+__device__ __forceinline__ unsigned acquire_arrivals(const unsigned *counter) {
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(counter) : "memory");
+    return v;
+}
+
 // Deterministic CTA reduction of NV doubles (fixed tree) over a CTA of W
 // warps; result in thread 0.
 template <int NV, int W = kWarps>

@@ -100,19 +100,19 @@ __device__ __forceinline__ double newton_rows(const NewtonView<V> &K, int64_t ba
     return mine;
 }
 
-// Grid barrier; false when the wait was given up.  What the CTA wrote before it
-// is released; what others wrote is read through L2.
+// Grid barrier; false when the wait was given up.  What the CTA wrote before it is
+// released, what the others wrote acquired.
 template <class V>
 __device__ __forceinline__ bool newton_barrier(const NewtonView<V> &K, unsigned *barrier, int *ok) {
     __syncthreads();
     if (threadIdx.x == 0) {
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(K.sync) : "memory");
+        release_arrival(K.sync);
         const unsigned need = ++*barrier * gridDim.x;
         unsigned seen;
         int polls = 0;
-        do {
-            asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(K.sync) : "memory");
-        } while (seen < need && ++polls < kNewtonMaxPolls);
+        do
+            seen = acquire_arrivals(K.sync);
+        while (seen < need && ++polls < kNewtonMaxPolls);
         if (seen < need) {
             *ok = 0;
             atomicExch(&K.st->fault, 1);

@@ -4,7 +4,7 @@
 // What bounds such a model is latency, not bandwidth.  A 2,000 x 5,000 LP spends
 // 16 us a trial in the two fused kernels for 0.6 MB of matrix: a launch each, a
 // handful of CTAs, and one lane per row walking its entries in dependent rounds
-// of loads.  Here, 6.0 us a trial (30,011 x 60,037 with 360 k entries: 8.1 us
+// of loads.  Here, 6.3 us a trial (30,011 x 60,037 with 360 k entries: 8.4 us
 // against 21.6), a persistent grid keeps its rows and columns for all trials:
 //   - CTA b owns a contiguous range of SELL chunks of A^T and one of A, of
 //     balanced length; the state of their columns and rows stays in its shared
@@ -29,12 +29,14 @@
 //     of a 30,011 x 60,037 LP.
 // So a trajectory is the same, bit for bit, whichever path runs it.
 //
-// What is left of a trial is mostly the two barriers (about 1.2 us each), the
+// What is left of a trial is mostly the two barriers (1.2 to 1.4 us each), the
 // decision (about 2 us, less what the gathers beside it take) and the gathers,
 // one lookup per SM cycle (0.55 ns per entry of a CTA).  512 threads: with 768 or
 // 1,024 the registers spill (8.9 us on the 360 k LP).
 //
-// The barrier is an atomic arrival counter that one thread per CTA polls.  The
+// The barrier is an atomic arrival counter that one thread per CTA polls, each
+// arrival a release and each poll an acquire.  (Relaxed polls save up to 0.4 us a
+// trial, but then nothing orders what the other CTAs wrote before the reads.)  The
 // grid is launched cooperatively, so every CTA is resident; the polls are
 // bounded all the same, and a CTA that gives up sets Control::fault, which the
 // host turns into an error.
@@ -61,8 +63,8 @@ struct ResidentView {
     const int *own_q;           // sparse Q: CTA b owns its rows [own_q[b], own_q[b+1])
     int lists_p, lists_d;       // CTA lists of the two-kernel schedule
     int width_p, width_d;       // their lengths, padded to a multiple of 32 (zero slots)
-    double *sum_p;              // dx^2 per chunk
-    double *sum_d;              // dy^2 per chunk, then dy * delta per chunk
+    double *sum_p;              // dx^2 per chunk, for every other trial in turn
+    double *sum_d;              // dy^2 per chunk, then dy * delta per chunk; likewise
     unsigned long long *word;   // the decision message
     double *last_x, *last_y;    // Halpern: the trial points T not yet copied to xa, ya
     // shared memory: entries of the products, of A^T and of A, virtual columns
@@ -71,6 +73,10 @@ struct ResidentView {
     int hot;   // leading entries of y that a CTA copies for its gathers (a multiple of 32)
     int stage; // what is copied to shared memory: 0 the state, 1 also the bounds, 2 also the entries
     unsigned *sync; // [0] barrier arrivals, [1] CTAs done; zero between launches
+    __device__ double *sums_p(int trial) const { return sum_p + (trial & 1) * lists_p * width_p; }
+    __device__ double *sums_d(int trial) const {
+        return sum_d + (trial & 1) * 2 * lists_d * width_d;
+    }
 };
 
 // A CTA's dynamic shared memory: the products; y's hot entries; per virtual column x twice, its
@@ -84,18 +90,16 @@ inline size_t resident_shared_bytes(const ResidentView &R, size_t value_bytes) {
            (R.stage == 2 ? (size_t(R.entries_t) + size_t(R.entries_a)) * (value_bytes + 4) : 0);
 }
 
-// Waits until `need` arrivals have been counted; false when the wait was given up.
-// The poll is relaxed on purpose: an acquire would drop the SM's L1, which holds
-// the entries where shared memory does not; what other CTAs wrote is read
-// through L2 (__ldcg).
+// Waits until `need` arrivals have been counted, and acquires what the arrived CTAs
+// wrote; false when the wait was given up.
 __device__ __forceinline__ bool wait_arrivals(const unsigned *counter, unsigned need, Control *ctl,
                                               int *ok) {
     if (threadIdx.x == 0) {
         int polls = 0;
         unsigned seen;
-        do {
-            asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(counter) : "memory");
-        } while (seen < need && ++polls < kResMaxPolls);
+        do
+            seen = acquire_arrivals(counter);
+        while (seen < need && ++polls < kResMaxPolls);
         if (seen < need) {
             *ok = 0;
             atomicExch(&ctl->fault, 1);
@@ -105,13 +109,19 @@ __device__ __forceinline__ bool wait_arrivals(const unsigned *counter, unsigned 
     return *ok != 0;
 }
 
-// Grid barrier number k of this launch (k = 1, 2, ...) of the CTAs that hold
-// rows; the arrival releases the CTA's writes.
+// The arrivals counted when grid barrier k of a launch (k = 1, 2, ...: two a
+// trial) is complete: those of the CTAs that hold rows at each, and the last CTA's
+// once a trial from the second on, before its first barrier (see there).
+__device__ __forceinline__ unsigned arrivals_at(unsigned k) {
+    return k * (gridDim.x - 1) + (k - 1) / 2;
+}
+
+// Grid barrier k for a CTA that holds rows; the arrival releases the CTA's writes.
 __device__ __forceinline__ bool grid_barrier(unsigned *counter, unsigned k, Control *ctl, int *ok) {
     __syncthreads();
     if (threadIdx.x == 0)
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(counter) : "memory");
-    return wait_arrivals(counter, k * (gridDim.x - 1), ctl, ok);
+        release_arrival(counter);
+    return wait_arrivals(counter, arrivals_at(k), ctl, ok);
 }
 
 // src[j], from the copy of its first `hot` entries where it lies there, else
@@ -262,7 +272,6 @@ __device__ __forceinline__ void resident_decider(const ResidentView &R, Vecs &v,
     __shared__ double list_p[kResMaxLists], list_d[2 * kResMaxLists], tree[3][kResMaxLists / 32];
     __shared__ double powers[2];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const unsigned others = gridDim.x - 1;
     const bool adaptive = (c.flags & 1) != 0;
     const int top = R.lists_p > R.lists_d ? R.lists_p : R.lists_d;
     const int rows = (top + 31) / 32; // warps of the two-kernel path's last CTA that hold a term
@@ -271,12 +280,12 @@ __device__ __forceinline__ void resident_decider(const ResidentView &R, Vecs &v,
     for (; t < trials && c.restart == 0; ++t) {
         if (adaptive && warp == kResWarps - 1 && lane < 2)
             powers[lane] = pow(c.accepted + 2, lane ? -.6 : -.3);
-        if (!wait_arrivals(R.sync, (2u * unsigned(t) + 1u) * others, v.ctl, &ok)) // dx^2
+        if (!wait_arrivals(R.sync, arrivals_at(2u * unsigned(t) + 1u), v.ctl, &ok)) // dx^2
             return;
-        all_list_sums(R.sum_p, R.lists_p, R.width_p, list_p);
-        if (!wait_arrivals(R.sync, (2u * unsigned(t) + 2u) * others, v.ctl, &ok)) // dy^2, dy * delta
+        all_list_sums(R.sums_p(t), R.lists_p, R.width_p, list_p);
+        if (!wait_arrivals(R.sync, arrivals_at(2u * unsigned(t) + 2u), v.ctl, &ok)) // dy^2, dy * delta
             return;
-        all_list_sums(R.sum_d, 2 * R.lists_d, R.width_d, list_d);
+        all_list_sums(R.sums_d(t), 2 * R.lists_d, R.width_d, list_d);
         __syncthreads();
         if (warp < rows) {
             const int b = warp * 32 + lane;
@@ -318,6 +327,12 @@ __device__ __forceinline__ void resident_decider(const ResidentView &R, Vecs &v,
             }
         }
         __syncthreads();
+        // The terms of this trial are read: if another follows, its first barrier
+        // waits for this arrival, and the trial after it overwrites them.  (The
+        // decision words need no release: nothing that others wrote is read on
+        // their account.)
+        if (threadIdx.x == 0 && t + 1 < trials && c.restart == 0)
+            release_arrival(R.sync);
     }
     if (threadIdx.x == 0) {
         if (t < trials) // a requested Halpern restart froze the rest
@@ -521,7 +536,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
                 }
                 mine = warp_total(mine);
                 if (lane == 0)
-                    __stcg(R.sum_p + slot_t[k], mine);
+                    __stcg(R.sums_p(t) + slot_t[k], mine);
             }
         }
         if (!grid_barrier(R.sync, ++barrier, v.ctl, &ok)) // dx is complete
@@ -593,8 +608,8 @@ __global__ void __launch_bounds__(kResThreads, 1)
                     cpl += __shfl_xor_sync(0xffffffffu, cpl, off);
                 }
                 if (lane == 0) {
-                    __stcg(R.sum_d + slot_a[k], dy2);
-                    __stcg(R.sum_d + R.lists_d * R.width_d + slot_a[k], cpl);
+                    __stcg(R.sums_d(t) + slot_a[k], dy2);
+                    __stcg(R.sums_d(t) + R.lists_d * R.width_d + slot_a[k], cpl);
                 }
             }
         }

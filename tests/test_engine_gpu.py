@@ -732,3 +732,24 @@ def test_resident_trials_from_several_threads(gpu):
     for k in range(4):
         for u, w in zip(alone[k], together[k]):
             assert np.array_equal(u, w)
+
+
+def test_resident_trials_frozen_in_mid_chunk(gpu):
+    """A Halpern restart requested by the tenth of 40 trials freezes the other 30, and
+    the next launches' barriers start from zero again: bit for bit the trials that
+    run as kernels of their own, over several restarts and chunk lengths."""
+    model, d = load_golden("steps_lp_halpern")
+    tau, sigma = float(d["tau"]), float(d["sigma"])
+    options = dict(halpern=True, reflection=0.5, residual_restarts=True, graphs=True)
+    a, b = gpu.PdhgBackend(model, **options), gpu.PdhgBackend(model, **options)
+    requests = 0
+    for count in (40, 40, 1, 2, 3, 40, 17, 40):
+        a.advance(count, tau, sigma)
+        b.profile_kernels(count, tau, sigma)
+        for u, w in zip(a.candidates(), b.candidates()):
+            assert np.array_equal(u, w)
+        if a.restart_requested():
+            requests += 1
+            for g in (a, b):
+                g.reset_candidate(True)
+    assert requests >= 1
