@@ -141,6 +141,10 @@ nk_status nk_pdhg_profile_kernels(nk_pdhg *h, int count, double tau, double sigm
  * together in one launch).  Null outputs are skipped. */
 nk_status nk_pdhg_layout_info(nk_pdhg *h, int64_t *long_rows, int64_t *panel_width,
                               int *panels, int64_t *runs, int *kernels_per_trial);
+/* Whether nk_pdhg_advance runs the trials together in one launch, and if so what
+ * that launch keeps in shared memory beside the iterate: 0 nothing, 1 the bounds
+ * and costs, 2 also the matrix entries.  Null outputs are skipped. */
+nk_status nk_pdhg_trial_path(nk_pdhg *h, int *resident, int *stage);
 /* Profiling (no reference counterpart): mean duration in milliseconds of `reps`
  * plain SpMVs (no fused epilogue) with A (which = 0, input x) or A^T (which = 1,
  * input y) on the resident iterate; results go to scratch, iterates unchanged. */

@@ -2458,6 +2458,16 @@ nk_status nk_pdhg_layout_info(nk_pdhg *h, int64_t *long_rows, int64_t *panel_wid
             *kernels_per_trial = 2 + (e.panels ? 1 : 0) + (e.halpern ? 1 : 0);
     });
 }
+nk_status nk_pdhg_trial_path(nk_pdhg *h, int *resident, int *stage) {
+    return guard([&] {
+        NK_HANDLE
+        const auto &r = h->e->resident;
+        if (resident)
+            *resident = r.on;
+        if (stage)
+            *stage = r.on ? r.view.stage : 0;
+    });
+}
 nk_status nk_pdhg_time_spmv(nk_pdhg *h, int which, int reps, double *ms) {
     return guard([&] {
         NK_HANDLE

@@ -468,11 +468,12 @@ __global__ void __launch_bounds__(kResThreads, 1)
         }
         products_t(y);
     }
-    // the sum of column l's products (a split region's segment), from c_l
+    // the sum of column l's products, from c_l (from 0: a split region's segment, and
+    // the lanes past the last column, where an unstaged c has no entry)
     auto row_sum = [&](int k) {
         const int l = k * 32 + lane;
-        const bool split = SPLIT && (t0 + k) * 32 < At.nsv;
-        return add_products(prod + at_t[k] + lane, len_t[l], split ? 0. : bc[l]);
+        const bool whole = (!SPLIT || (t0 + k) * 32 >= At.nsv) && t0 * 32 + l < At.nv;
+        return add_products(prod + at_t[k] + lane, len_t[l], whole ? bc[l] : 0.);
     };
     bool unsaved = false; // Halpern: last_x / last_y hold the accepted point, the averages do not
     unsigned barrier = 0;

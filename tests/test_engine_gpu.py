@@ -753,3 +753,33 @@ def test_resident_trials_frozen_in_mid_chunk(gpu):
             for g in (a, b):
                 g.reset_candidate(True)
     assert requests >= 1
+
+
+@pytest.mark.parametrize("method", ["adaptive", "halpern", "mixed"])
+@pytest.mark.parametrize("split", [False, True])
+def test_resident_trials_with_unstaged_bounds(gpu, split, method):
+    """The largest resident models keep only the iterate in shared memory and read
+    bounds and costs where they lie: a last chunk of one column (31 lanes past the
+    end of c), without and with columns long enough to be split (400 entries; the
+    other columns then start at a chunk of their own).  Bit for bit the trials that
+    run as kernels of their own."""
+    m = synth.random_lp(m=100_003, n=270_017 + (2 if split else 0), per_col=5, seed=12)
+    if split:
+        rng = np.random.default_rng(13)
+        rows = np.repeat(np.arange(m.m), np.diff(m.ptr))
+        extra = [rng.choice(m.m, 400, replace=False) * m.n + j for j in (7, 200_000)]
+        key, first = np.unique(np.concatenate([rows * m.n + m.idx, *extra]), return_index=True)
+        m.val = np.concatenate([m.val, rng.standard_normal(800)])[first]
+        m.idx = key % m.n
+        m.ptr = np.r_[0, np.cumsum(np.bincount(key // m.n, minlength=m.m))].astype(np.int64)
+    tau, sigma = step_sizes(m)
+    options = dict(adaptive=method != "halpern", halpern=method == "halpern", graphs=True,
+                   precision="mixed" if method == "mixed" else "fp64")
+    a, b = gpu.PdhgBackend(m, **options), gpu.PdhgBackend(m, **options)
+    info = a.layout_info()
+    assert info["resident"] and info["resident_stage"] == 0, info
+    for count in (1, 2, 30):
+        a.advance(count, tau, sigma)
+        b.profile_kernels(count, tau, sigma)
+        for u, w in zip(a.candidates(), b.candidates()):
+            assert np.array_equal(u, w)
