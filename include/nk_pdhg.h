@@ -145,6 +145,10 @@ nk_status nk_pdhg_layout_info(nk_pdhg *h, int64_t *long_rows, int64_t *panel_wid
  * that launch keeps in shared memory beside the iterate: 0 nothing, 1 the bounds
  * and costs, 2 also the matrix entries.  Null outputs are skipped. */
 nk_status nk_pdhg_trial_path(nk_pdhg *h, int *resident, int *stage);
+/* For tests: leaves the state that a trial launch leaves which gave up a wait.  The
+ * next nk_pdhg_advance or profiling call runs no trial of such a launch and returns
+ * NK_ERR_CUDA; the calls after it run as usual. */
+nk_status nk_pdhg_mark_fault(nk_pdhg *h);
 /* Profiling (no reference counterpart): mean duration in milliseconds of `reps`
  * plain SpMVs (no fused epilogue) with A (which = 0, input x) or A^T (which = 1,
  * input y) on the resident iterate; results go to scratch, iterates unchanged. */

@@ -652,6 +652,33 @@ struct Engine {
 
     // trials of one resident launch (bounds its run time and its barrier count)
     static constexpr int kResidentTrials = 4096;
+    void run_resident(int count) {
+        for (; count > 0; count -= kResidentTrials)
+            launch_resident(std::min(count, kResidentTrials));
+    }
+    // Throws if a resident launch since the last sync_ctl() gave up a wait (those
+    // queued behind it did nothing).  Its counters are then as for a new engine; the
+    // iterate is not, until reset() or restore().
+    void check_resident() {
+        if (!host_ctl->fault)
+            return;
+        host_ctl->fault = 0;
+        push_ctl();
+        cuda_check(cudaMemsetAsync(resident.view.sync, 0, 2 * sizeof(unsigned), stream),
+                   "trial counters");
+        throw Error(NK_ERR_CUDA, "a wait inside the trial kernel was given up");
+    }
+    // The state that a wait given up leaves behind, for tests of what follows it.
+    void mark_fault() {
+        if (!resident.on)
+            throw Error(NK_ERR_UNSUPPORTED, "no resident trials");
+        sync_ctl();
+        host_ctl->fault = 1;
+        push_ctl();
+        cuda_check(cudaMemsetAsync(resident.view.sync, 1, 2 * sizeof(unsigned), stream),
+                   "trial counters");
+        cuda_check(cudaStreamSynchronize(stream), "trial counters");
+    }
     void launch_resident(int count) {
         if (precision == NK_PRECISION_FP64)
             launch_resident_t<double>(count);
@@ -835,8 +862,7 @@ struct Engine {
         int left = count;
         ctl_known = false;
         if (resident.on) {
-            for (; left > 0; left -= kResidentTrials)
-                launch_resident(std::min(left, kResidentTrials));
+            run_resident(left);
         } else if (graphs) {
             for (int k = 7; k >= 0 && left > 0; --k)
                 while (left >= (1 << k)) {
@@ -850,14 +876,7 @@ struct Engine {
         cuda_check(cudaGetLastError(), "trial launch");
         trials += count;
         sync_ctl();
-        if (host_ctl->fault) {
-            host_ctl->fault = 0;
-            push_ctl();
-            ctl_known = false;
-            cuda_check(cudaMemsetAsync(resident.view.sync, 0, 2 * sizeof(unsigned), stream),
-                       "trial counters");
-            throw Error(NK_ERR_CUDA, "a wait inside the trial kernel was given up");
-        }
+        check_resident();
         int64_t now = int64_t(host_ctl->accepted);
         int progress = int(now - accepted);
         accepted = now;
@@ -1213,11 +1232,11 @@ struct Engine {
         }
         if (replay) {
             copy_state(true);
-            for (int left = count; left > 0; left -= kResidentTrials)
-                launch_resident(std::min(left, kResidentTrials));
+            run_resident(count);
         }
         trials += count;
         sync_ctl();
+        check_resident();
         accepted = int64_t(host_ctl->accepted);
         rejected = int64_t(host_ctl->rejected);
         *ms_primal = tp / count;
@@ -2466,6 +2485,12 @@ nk_status nk_pdhg_trial_path(nk_pdhg *h, int *resident, int *stage) {
             *resident = r.on;
         if (stage)
             *stage = r.on ? r.view.stage : 0;
+    });
+}
+nk_status nk_pdhg_mark_fault(nk_pdhg *h) {
+    return guard([&] {
+        NK_HANDLE
+        h->e->mark_fault();
     });
 }
 nk_status nk_pdhg_time_spmv(nk_pdhg *h, int which, int reps, double *ms) {

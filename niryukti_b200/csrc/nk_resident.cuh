@@ -365,6 +365,8 @@ __global__ void __launch_bounds__(kResThreads, 1)
         ok = 1;
     }
     __syncthreads();
+    if (c.fault) // an earlier launch gave up a wait: its counters are no longer whole
+        return;
     if (blockIdx.x == gridDim.x - 1) {
         resident_decider<HALPERN>(R, v, c, ok, trials, tag);
         resident_leave(R);

@@ -78,6 +78,7 @@ def library() -> C.CDLL:
     L.nk_pdhg_layout_info.argtypes = [C.c_void_p, _I, _I, C.POINTER(C.c_int), _I,
                                       C.POINTER(C.c_int)]
     L.nk_pdhg_trial_path.argtypes = [C.c_void_p, C.POINTER(C.c_int), C.POINTER(C.c_int)]
+    L.nk_pdhg_mark_fault.argtypes = [C.c_void_p]
     L.nk_pdhg_schedule_info.argtypes = [C.c_void_p, C.POINTER(C.c_int), _I, C.POINTER(C.c_int),
                                         _I, C.POINTER(C.c_int), C.POINTER(C.c_int)]
     L.nk_pdhg_stream.argtypes = [C.c_void_p, C.POINTER(C.c_void_p)]

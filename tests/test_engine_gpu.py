@@ -783,3 +783,28 @@ def test_resident_trials_with_unstaged_bounds(gpu, split, method):
         b.profile_kernels(count, tau, sigma)
         for u, w in zip(a.candidates(), b.candidates()):
             assert np.array_equal(u, w)
+
+
+def test_a_wait_given_up_is_reported_once(gpu):
+    """After a trial launch that gave up a wait (marked here as one leaves it),
+    advance() of several queued launches and profile_kernels() report it without
+    having run a trial, and the calls after that run from whole counters: bit for bit
+    an engine that never failed."""
+    m = synth.power_law_lp(m=3000, n=6000, nnz=60000, seed=4, len_hi=3000)
+    tau, sigma = step_sizes(m)
+    a, b = gpu.PdhgBackend(m, graphs=True), gpu.PdhgBackend(m, graphs=True)
+    info = a.layout_info()
+    assert info["resident"] and info["panels"] > 0, info
+    for call in (lambda: a.advance(9000, tau, sigma), lambda: a.profile_kernels(5, tau, sigma)):
+        a.advance(7, tau, sigma)
+        b.advance(7, tau, sigma)
+        gpu.check(gpu.library().nk_pdhg_mark_fault(a._h))
+        with pytest.raises(gpu.EngineError) as e:
+            call()
+        assert e.value.status == "CUDA"
+        assert a.advance(7, tau, sigma) == b.advance(7, tau, sigma) == 7
+        for u, w in zip(a.candidates(), b.candidates()):
+            assert np.array_equal(u, w)
+    wide = gpu.PdhgBackend(m, indices="64")
+    with pytest.raises(gpu.EngineError):
+        gpu.check(gpu.library().nk_pdhg_mark_fault(wide._h))
