@@ -1675,8 +1675,8 @@ void build_panels(PanelMatrix &P, int64_t rows, int64_t cols, const std::vector<
 template <class Acc, class V, class I> void configure(Engine &E) {
     const void *pk = (const void *)primal_kernel_for<Acc, V, I>(E.sparse_q, E.At.nsv > 0);
     const void *dk = (const void *)dual_kernel_for<Acc, V, I>(E.A, E.panels);
-    // the slot arrays stay far below the default 48 KB; the grids are sized
-    // without them, which the occupancy check after the schedules confirms
+    // the grids are sized without the slot arrays (they pass 48 KB from about 14.5 M
+    // rows on), which the occupancy check after the schedules confirms
     E.grid_p = occupancy_grid(pk, (E.At.nv + 31) / 32, kFusedThreads, 0);
     E.grid_d = occupancy_grid(dk, (E.A.nv + 31) / 32, kFusedThreads, 0);
     E.grid_s = occupancy_grid((const void *)spmv_kernel<V, I>, int64_t(1) << 40);
@@ -1686,10 +1686,11 @@ template <class Acc, class V, class I> void attach_slots(Engine &E) {
     const void *dk = (const void *)dual_kernel_for<Acc, V, I>(E.A, E.panels);
     for (auto [k, bytes, grid] : {std::tuple<const void *, size_t, int>{pk, E.smem_p(), E.grid_p},
                                   {dk, E.smem_d(), E.grid_d}}) {
-        if (bytes > 48 * 1024)
-            cuda_check(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            int(bytes)),
-                       "slot memory");
+        // the limit is the kernel's, not this engine's: an engine with more slots may
+        // be alive
+        cuda_check(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        int(smem_budget(k, kFusedMinBlocks))),
+                   "slot memory");
         int per = 0, dev = 0, sms = 148;
         cuda_check(cudaGetDevice(&dev), "device");
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

@@ -808,3 +808,19 @@ def test_a_wait_given_up_is_reported_once(gpu):
     wide = gpu.PdhgBackend(m, indices="64")
     with pytest.raises(gpu.EngineError):
         gpu.check(gpu.library().nk_pdhg_mark_fault(wide._h))
+
+
+def test_slot_limits_of_large_engines_coexist(gpu):
+    """The step rule's slots of 20 M rows take 66 KB of shared memory a CTA, those of
+    15 M rows 50 KB: the kernel's limit belongs to both engines, so the larger one
+    still runs after the smaller was built."""
+    def model(m, n):
+        val = np.where(np.arange(m) % 2 == 0, 1.0, -1.0)
+        ptr, idx = np.arange(m + 1, dtype=np.int64), np.arange(m, dtype=np.int64) % n
+        return synth.Model(m=m, n=n, ptr=ptr, idx=idx, val=val, c=np.ones(n), q=np.zeros(n),
+                           lb=np.zeros(n), ub=np.ones(n), rl=np.zeros(m), ru=np.ones(m),
+                           name="rows of one entry", x0=np.zeros(n))
+    large = gpu.PdhgBackend(model(20_000_000, 1_000_000))
+    small = gpu.PdhgBackend(model(15_000_000, 1_000_000))
+    assert large.advance(2, 0.01, 0.01) == 2
+    assert small.advance(2, 0.01, 0.01) == 2
