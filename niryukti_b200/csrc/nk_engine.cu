@@ -998,13 +998,18 @@ struct Engine {
         cuda_check(cudaStreamSynchronize(stream), "reset"); // the caller may reuse hx, hy
     }
 
+    // out of A x and A^T y, for the monitor and time_spmv()
+    void product_buffers() {
+        if (!mon_ax.p)
+            mon_ax.alloc(size_t(std::max<int64_t>(1, m)));
+        if (!mon_aty.p)
+            mon_aty.alloc(size_t(std::max<int64_t>(1, n)));
+    }
     double monitor() {
-        if (!mon_ax.p) {
-            mon_ax.alloc(std::max<int64_t>(1, m));
-            mon_aty.alloc(std::max<int64_t>(1, n));
+        product_buffers();
+        if (!mon_out.p) {
             mon_qx.alloc(std::max<int64_t>(1, n));
             mon_part.alloc(size_t(5 * 148 * 8));
-            mon_out.alloc(2);
             mon_arrive.alloc(1);
             cuda_check(cudaMemsetAsync(mon_arrive.p, 0, sizeof(unsigned), stream), "monitor");
             std::vector<double> hc(static_cast<size_t>(n));
@@ -1013,6 +1018,7 @@ struct Engine {
             cscale = 1;
             for (double v : hc)
                 cscale = std::max(cscale, 1 + std::abs(v));
+            mon_out.alloc(2); // last: a call that failed above starts over
         }
         flush();
         sync_ctl();
@@ -1251,10 +1257,7 @@ struct Engine {
     double time_spmv(int which, int reps) {
         if (reps <= 0)
             throw Error(NK_ERR_INVALID, "reps must be positive");
-        if (!mon_ax.p) {
-            mon_ax.alloc(std::max<int64_t>(1, m));
-            mon_aty.alloc(std::max<int64_t>(1, n));
-        }
+        product_buffers();
         sync_ctl();
         int cur = host_ctl->cur;
         cudaEvent_t a, b;

@@ -83,3 +83,14 @@ def test_host_formula_matches_reference_cuda_monitor(kind, tmp_path):
     d = np.load(out)
     model = {"lp": lp_with_diagonal_q, "qp": qp_with_sparse_q}[kind]()
     close(float(d["monitor"]), monitor(model, d["x"], d["y"], d["xa"], d["ya"]))
+
+
+def test_monitor_after_a_timed_product(gpu):
+    """time_spmv() shares the monitor's product buffers: called first, it leaves the
+    monitor's own still to be allocated."""
+    model = lp_with_diagonal_q()
+    a, b = (gpu.PdhgBackend(model, adaptive=True, graphs=True) for _ in range(2))
+    for g in (a, b):
+        g.advance(50, 0.05, 0.05)
+    assert a.time_spmv("A", 2) > 0 and a.time_spmv("At", 2) > 0
+    assert a.monitor() == b.monitor()
