@@ -2478,7 +2478,7 @@ nk_status nk_pdhg_layout_info(nk_pdhg *h, int64_t *long_rows, int64_t *panel_wid
         if (runs)
             *runs = e.panels ? e.pan.slots : 0;
         if (kernels_per_trial)
-            *kernels_per_trial = 2 + (e.panels ? 1 : 0) + (e.halpern ? 1 : 0);
+            *kernels_per_trial = 2 + (e.sparse_q ? 1 : 0) + (e.panels ? 1 : 0) + (e.halpern ? 1 : 0);
     });
 }
 nk_status nk_pdhg_trial_path(nk_pdhg *h, int *resident, int *stage) {

@@ -824,3 +824,14 @@ def test_slot_limits_of_large_engines_coexist(gpu):
     small = gpu.PdhgBackend(model(15_000_000, 1_000_000))
     assert large.advance(2, 0.01, 0.01) == 2
     assert small.advance(2, 0.01, 0.01) == 2
+
+
+def test_kernels_of_a_trial_are_counted(gpu):
+    """The launches of a trial that runs as kernels of its own: the primal and the
+    dual one, Q x of a sparse Q, and Halpern's commit."""
+    m = sparse_qp_model()
+    assert gpu.PdhgBackend(m).layout_info()["kernels_per_trial"] == 3
+    assert gpu.PdhgBackend(m, halpern=True).layout_info()["kernels_per_trial"] == 4
+    m = synth.random_lp(m=70, n=131, per_col=2, seed=5)
+    assert gpu.PdhgBackend(m).layout_info()["kernels_per_trial"] == 2
+    assert gpu.PdhgBackend(m, halpern=True).layout_info()["kernels_per_trial"] == 3
