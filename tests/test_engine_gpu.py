@@ -835,3 +835,47 @@ def test_kernels_of_a_trial_are_counted(gpu):
     m = synth.random_lp(m=70, n=131, per_col=2, seed=5)
     assert gpu.PdhgBackend(m).layout_info()["kernels_per_trial"] == 2
     assert gpu.PdhgBackend(m, halpern=True).layout_info()["kernels_per_trial"] == 3
+
+
+def panel_model(kind, precision="fp64"):
+    """A model whose long rows lie in several column panels, or cut into runs in one."""
+    m = (synth.power_law_lp(m=20000, n=100000, nnz=500000, seed=3, len_hi=5000)
+         if kind == "several panels" else
+         synth.power_law_lp(m=3000, n=6000, nnz=60000, seed=4, len_hi=3000))
+    if precision == "mixed":
+        m.val = m.val.astype(np.float32).astype(np.float64)
+    return m
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("kind", ["several panels", "cut runs"])
+def test_panel_kernel_under_adaptive_steps(gpu, oracle, kind, precision):
+    """The panel kernel against the oracle where advance() launches it: a small model's
+    fixed steps run resident, without it, its adaptive steps never do.  A long row of
+    up to 5,000 terms, regrouped, rounds within 5,000 ulp, 6e-13, a trial, and adaptive
+    steps carry that forward about tenfold every eight trials: 1e-9 over 10 accepted
+    steps, where a lost or doubled run moves the point by its share."""
+    m = panel_model(kind, precision)
+    g = gpu.PdhgBackend(m, adaptive=True, graphs=True, precision=precision)
+    info = g.layout_info()
+    assert not info["resident"] and info["kernels_per_trial"] == 3, info
+    assert info["panels"] >= 2 if kind == "several panels" else \
+        info["panels"] == 1 and info["panel_runs"] > info["panel_rows"], info
+    cpu = oracle.model(m).backend(np.zeros(m.n), np.zeros(m.m), adaptive=True)
+    tau, sigma = step_sizes(m)
+    advance_to(g, cpu.advance(10, tau, sigma), tau, sigma)
+    assert g.rejected_steps() == cpu.rejected_steps()
+    for u, w in zip(g.candidates(), cpu.candidates()):
+        near(u, w, 1e-9)
+
+
+def test_adaptive_panel_engines_of_different_widths_coexist(gpu):
+    """The panel kernel's shared-memory limit belongs to every engine: the one with wide
+    panels still launches it after one with narrow panels was built."""
+    models = [panel_model(kind) for kind in ("several panels", "cut runs")]
+    wide, narrow = (gpu.PdhgBackend(m, adaptive=True) for m in models)
+    info = [g.layout_info() for g in (wide, narrow)]
+    assert info[0]["panel_width"] > info[1]["panel_width"] > 0
+    assert not (info[0]["resident"] or info[1]["resident"])
+    for g, m in zip((wide, narrow), models):
+        assert g.advance(20, *step_sizes(m)) > 0
