@@ -13,7 +13,16 @@
 // fixed order, and with them forms the step scalars in the reference's
 // expressions and order.  Vectors that others gather (y and z) go through L2.
 // A call on a saddle point of 24,000 unknowns and 184 k entries, with its uploads
-// and allocations: 5.9 ms before, 1.7 ms now (one allocation, too).
+// and allocations: 5.9 ms before, 1.8 ms now (one allocation, too).
+//
+// A row of more than 32 entries has a warp of the whole grid to itself, before the
+// product's elements are formed, for a barrier more a product: left to the warp of
+// its element it waits its turn among 32 rows.  Calls with and without the extra
+// phase, ms, and as separate launches: 2,000 rows of 800 entries 3.6 / 6.5 / 11.5,
+// 24,000 short rows with 64 long ones of 3,000 entries 2.3 / 13.9 / 6.2, 200,000
+// with 32 of 25,000 9.5 / 109 / 23, 24,000 rows of 46 entries 3.1 / 3.9 / 8.2.
+// From 32 entries on, because a lane then has one at most in the short rows' turns;
+// 64 and 128 are no faster (10,000 rows of 100: 2.8, 2.9 and 3.2 ms).
 //
 // The grid is resident (cooperative launch) and its waits are bounded; a CTA
 // that gives up sets NewtonState::fault.
@@ -35,13 +44,17 @@ struct NewtonState {
     int fault;     // a wait was given up
 };
 
-constexpr int kNewtonChunk = 64;          // iterations of one launch
-constexpr int kNewtonMaxPolls = 4 << 20;  // seconds: the barrier's bound
+constexpr int kNewtonLong = 32;          // rows of more entries have a warp each
+constexpr int kNewtonChunk = 64;         // iterations of one launch
+constexpr int kNewtonMaxPolls = 4 << 20; // seconds: the barrier's bound
 
 template <class V> struct NewtonView {
     int64_t n;
     const int64_t *ptr, *idx;
     const V *val;
+    const int64_t *long_rows; // rows of more than kNewtonLong entries
+    int64_t nlong;
+    int element_ctas;         // the first CTAs: those that own elements
     const double *rhs, *dinv;
     double *x, *r, *p, *v, *s, *t, *y, *z;
     double *part;   // two sums per CTA, for each of the iteration's barriers in turn
@@ -54,38 +67,33 @@ template <class V> struct NewtonView {
 // Row `base + lane`'s product with x, for the warp's 32 rows: 8, 16 or 32 lanes a
 // row (the warp's longest row decides), lane-strided, then a fixed shuffle tree.
 // A row's sum is the 32-lane one whatever the width: the other lanes would add
-// zeros.  Loads of four turns are in flight together.
+// zeros.  Loads of four turns are in flight together.  A long row's product is 0
+// here: newton_long_rows has it.
 template <class V>
 __device__ __forceinline__ double newton_rows(const NewtonView<V> &K, int64_t base, const double *x) {
     const int lane = threadIdx.x & 31;
-    const int64_t row = base + lane, start = K.ptr[base < K.n ? base : K.n];
-    const int at = row < K.n ? int(K.ptr[row] - start) : 0;
-    const int len = row < K.n ? int(K.ptr[row + 1] - start) - at : 0;
+    const int64_t row = base + lane, at = K.ptr[row < K.n ? row : K.n],
+                  entries = row < K.n ? K.ptr[row + 1] - at : 0;
+    const int len = entries > kNewtonLong ? 0 : int(entries);
     const int top = __reduce_max_sync(0xffffffffu, len);
     const int L = top <= 8 ? 8 : top <= 16 ? 16 : 32, per = 32 / L; // lanes a row, rows a turn
     constexpr int U = 4;
     double mine = 0;
     for (int it0 = 0; it0 < L; it0 += U) {
-        int64_t j[U];
+        int64_t j[U], from[U];
         double w[U], acc[U];
-        int rest[U], from[U];
+        int rest[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const int q = (it0 + u) * per + lane / L, k = lane % L;
             from[u] = __shfl_sync(0xffffffffu, at, q) + k;
             rest[u] = __shfl_sync(0xffffffffu, len, q) - k;
-            j[u] = rest[u] > 0 ? K.idx[start + from[u]] : -1;
-            w[u] = rest[u] > 0 ? double(K.val[start + from[u]]) : 0.;
+            j[u] = rest[u] > 0 ? K.idx[from[u]] : -1;
+            w[u] = rest[u] > 0 ? double(K.val[from[u]]) : 0.;
         }
 #pragma unroll
         for (int u = 0; u < U; ++u)
             acc[u] = j[u] >= 0 ? 0. + w[u] * __ldcg(x + j[u]) : 0.;
-        if (top > 32)
-#pragma unroll
-            for (int u = 0; u < U; ++u)
-                for (int k = 32; k < rest[u]; k += 32)
-                    acc[u] += double(K.val[start + from[u] + k]) *
-                              __ldcg(x + K.idx[start + from[u] + k]);
         for (int off = L / 2; off > 0; off >>= 1)
 #pragma unroll
             for (int u = 0; u < U; ++u)
@@ -98,6 +106,38 @@ __device__ __forceinline__ double newton_rows(const NewtonView<V> &K, int64_t ba
         }
     }
     return mine;
+}
+
+// The long rows' products with x into out, one warp a row over the whole grid:
+// lane-strided sums, loads of eight strides in flight, and the tree of newton_rows.
+template <class V>
+__device__ __forceinline__ void newton_long_rows(const NewtonView<V> &K, const double *x,
+                                                 double *out) {
+    const int lane = threadIdx.x & 31;
+    const int64_t stride = int64_t(gridDim.x) * kWarps;
+    for (int64_t q = int64_t(blockIdx.x) * kWarps + (threadIdx.x >> 5); q < K.nlong; q += stride) {
+        const int64_t row = K.long_rows[q], end = K.ptr[row + 1];
+        constexpr int U = 8;
+        double acc = 0;
+        for (int64_t k = K.ptr[row] + lane; k < end; k += 32 * U) {
+            double w[U], g[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const bool in = k + 32 * u < end;
+                w[u] = in ? double(K.val[k + 32 * u]) : 0.;
+                g[u] = in ? __ldcg(x + K.idx[k + 32 * u]) : 0.;
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (k + 32 * u < end)
+                    acc += w[u] * g[u];
+        }
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1)
+            acc += __shfl_xor_sync(0xffffffffu, acc, off);
+        if (lane == 0)
+            __stcg(out + row, acc);
+    }
 }
 
 // Grid barrier; false when the wait was given up.  What the CTA wrote before it is
@@ -156,9 +196,17 @@ __global__ void __launch_bounds__(kThreads, 4) newton_kernel(NewtonView<V> K) {
     __shared__ double red[kWarps * 2], sums[2];
     __shared__ unsigned barrier; // thread 0's count
     __shared__ int ok;
-    const int64_t n = K.n, first = int64_t(blockIdx.x) * kThreads + threadIdx.x,
-                  stride = int64_t(gridDim.x) * kThreads;
+    // the CTAs past element_ctas only walk long rows
+    const int64_t n = blockIdx.x < K.element_ctas ? K.n : 0,
+                  first = int64_t(blockIdx.x) * kThreads + threadIdx.x,
+                  stride = int64_t(K.element_ctas) * kThreads;
     const int64_t tops = (n + 31) / 32 * 32; // whole warps for the row products
+    // element e of K x; with long rows `out` (v or t) holds theirs
+    auto product = [&](int64_t e, const double *x, const double *out) {
+        const double short_row = newton_rows(K, e - (threadIdx.x & 31), x);
+        return e < n && K.nlong > 0 && K.ptr[e + 1] - K.ptr[e] > kNewtonLong ? __ldcg(out + e)
+                                                                           : short_row;
+    };
     if (threadIdx.x == 0) {
         barrier = 0;
         ok = 1;
@@ -219,10 +267,15 @@ __global__ void __launch_bounds__(kThreads, 4) newton_kernel(NewtonView<V> K) {
         }
         if (!newton_barrier(K, &barrier, &ok)) // y is complete
             return;
+        if (K.nlong > 0) {
+            newton_long_rows(K, K.y, K.v);
+            if (!newton_barrier(K, &barrier, &ok))
+                return;
+        }
         // v = K y, <shadow, v>
         double ab[2] = {0, 0};
         for (int64_t e = first; e < tops; e += stride) {
-            const double v = newton_rows(K, e - (threadIdx.x & 31), K.y);
+            const double v = product(e, K.y, K.v);
             if (e < n) {
                 K.v[e] = v;
                 ab[0] += K.rhs[e] * v;
@@ -254,10 +307,15 @@ __global__ void __launch_bounds__(kThreads, 4) newton_kernel(NewtonView<V> K) {
             stop = 1;
             break;
         }
+        if (K.nlong > 0) {
+            newton_long_rows(K, K.z, K.t);
+            if (!newton_barrier(K, &barrier, &ok))
+                return;
+        }
         // t = K z, <t, t>, <t, s>
         ab[0] = ab[1] = 0;
         for (int64_t e = first; e < tops; e += stride) {
-            const double t = newton_rows(K, e - (threadIdx.x & 31), K.z);
+            const double t = product(e, K.z, K.t);
             if (e < n) {
                 K.t[e] = t;
                 ab[0] += t * t;
@@ -294,21 +352,61 @@ __global__ void __launch_bounds__(kThreads, 4) newton_kernel(NewtonView<V> K) {
 // |K_ii| where the diagonal carries the row; where it does not (a saddle
 // point's regularised zero block, |K_ii| < 1e-8 max_j |K_ij|), the diagonal of
 // the row's Schur complement, sum_j K_ij^2 / |K_jj| over the other entries.
-// Rows with neither keep 1.  Two passes, a thread per row: the diagonals and
-// whether they carry their rows (diag: 0 where not), then the scales.
+// Rows with neither keep 1.  Two passes: the diagonals and whether they carry
+// their rows (diag: 0 where not), then the scales.  A thread takes a row; a long
+// row (newton_long_*) a warp, which loads 32 entries at a time and adds them in
+// the same order, entry by entry.
+__device__ __forceinline__ double carrying(double d, double big) {
+    return fabs(d) >= 1e-8 * big ? d : 0.;
+}
+__device__ __forceinline__ double schur_term(double a, int64_t i, int64_t j, const double *diag) {
+    return j != i && diag[j] != 0 ? a * a / fabs(diag[j]) : 0.;
+}
+__device__ __forceinline__ double newton_scale(double d, double schur) {
+    return d != 0 ? 1 / fabs(d) : schur > 0 && isfinite(schur) ? 1 / schur : 1.;
+}
 __global__ void newton_diagonal(int64_t n, const int64_t *__restrict__ ptr,
                                 const int64_t *__restrict__ idx, const double *__restrict__ val,
                                 double *__restrict__ diag) {
     const int64_t stride = int64_t(gridDim.x) * blockDim.x;
     for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
+        const int64_t b = ptr[i], e = ptr[i + 1];
+        if (e - b > kNewtonLong)
+            continue;
         double d = 0, big = 0;
-        for (int64_t k = ptr[i]; k < ptr[i + 1]; ++k) {
+        for (int64_t k = b; k < e; ++k) {
             const double a = fabs(val[k]);
             big = big < a ? a : big;
             if (idx[k] == i)
                 d += val[k];
         }
-        diag[i] = fabs(d) >= 1e-8 * big ? d : 0.;
+        diag[i] = carrying(d, big);
+    }
+}
+__global__ void newton_long_diagonal(int64_t nlong, const int64_t *__restrict__ long_rows,
+                                     const int64_t *__restrict__ ptr,
+                                     const int64_t *__restrict__ idx,
+                                     const double *__restrict__ val, double *__restrict__ diag) {
+    const int lane = threadIdx.x & 31;
+    const int64_t stride = (int64_t(gridDim.x) * blockDim.x) >> 5;
+    for (int64_t q = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; q < nlong; q += stride) {
+        const int64_t i = long_rows[q], e = ptr[i + 1];
+        double d = 0, big = 0;
+        for (int64_t k0 = ptr[i]; k0 < e; k0 += 32) {
+            const bool in = k0 + lane < e;
+            const double v = in ? val[k0 + lane] : 0., a = fabs(v);
+            big = big < a ? a : big;
+            for (unsigned hits = __ballot_sync(0xffffffffu, in && idx[k0 + lane] == i); hits;
+                 hits &= hits - 1)
+                d += __shfl_sync(0xffffffffu, v, __ffs(int(hits)) - 1);
+        }
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) {
+            const double a = __shfl_xor_sync(0xffffffffu, big, off);
+            big = big < a ? a : big;
+        }
+        if (lane == 0)
+            diag[i] = carrying(d, big);
     }
 }
 __global__ void newton_scales(int64_t n, const int64_t *__restrict__ ptr,
@@ -316,20 +414,45 @@ __global__ void newton_scales(int64_t n, const int64_t *__restrict__ ptr,
                               const double *__restrict__ diag, double *__restrict__ dinv) {
     const int64_t stride = int64_t(gridDim.x) * blockDim.x;
     for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
-        double out = 1;
-        if (diag[i] != 0)
-            out = 1 / fabs(diag[i]);
-        else {
-            double schur = 0;
-            for (int64_t k = ptr[i]; k < ptr[i + 1]; ++k) {
-                const int64_t j = idx[k];
-                if (j != i && diag[j] != 0)
-                    schur += val[k] * val[k] / fabs(diag[j]);
-            }
-            if (schur > 0 && isfinite(schur))
-                out = 1 / schur;
+        const int64_t b = ptr[i], e = ptr[i + 1];
+        double schur = 0;
+        if (diag[i] == 0) {
+            if (e - b > kNewtonLong)
+                continue;
+            for (int64_t k = b; k < e; ++k)
+                schur += schur_term(val[k], i, idx[k], diag);
         }
-        dinv[i] = out;
+        dinv[i] = newton_scale(diag[i], schur);
+    }
+}
+__global__ void newton_long_scales(int64_t nlong, const int64_t *__restrict__ long_rows,
+                                   const int64_t *__restrict__ ptr,
+                                   const int64_t *__restrict__ idx,
+                                   const double *__restrict__ val,
+                                   const double *__restrict__ diag, double *__restrict__ dinv) {
+    const int lane = threadIdx.x & 31;
+    const int64_t stride = (int64_t(gridDim.x) * blockDim.x) >> 5;
+    for (int64_t q = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; q < nlong; q += stride) {
+        const int64_t i = long_rows[q], e = ptr[i + 1];
+        if (diag[i] != 0) // newton_scales has it
+            continue;
+        constexpr int U = 4;
+        double schur = 0;
+        for (int64_t k0 = ptr[i]; k0 < e; k0 += 32 * U) {
+            double term[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int64_t k = k0 + 32 * u + lane;
+                term[u] = k < e ? schur_term(val[k], i, idx[k], diag) : 0.;
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int l = 0; l < 32; ++l)
+                    schur += __shfl_sync(0xffffffffu, term[u], l);
+        }
+        if (lane == 0)
+            dinv[i] = newton_scale(0., schur);
     }
 }
 __global__ void newton_ones(int64_t n, double *dinv) {
@@ -367,13 +490,24 @@ inline bool newton_solve_t(const nk_csr &K, const double *rhs, bool precondition
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, newton_kernel<V>, kThreads, 0),
                "Newton occupancy");
+    int64_t all_short = -1; // negative while every row is
+    for (int64_t i = 0; i < n; ++i)
+        all_short &= K.ptr[i + 1] - K.ptr[i] - (kNewtonLong + 1);
+    std::vector<int64_t> long_rows;
+    for (int64_t i = 0; all_short >= 0 && i < n; ++i)
+        if (K.ptr[i + 1] - K.ptr[i] > kNewtonLong)
+            long_rows.push_back(i);
+    const int64_t nlong = int64_t(long_rows.size()), resident = int64_t(sms) * std::min(4, per);
+    // the dots' grouping, and their bits, are those of the CTAs that own elements
+    const int element_ctas =
+        int(std::max<int64_t>(1, std::min<int64_t>((n + kThreads - 1) / kThreads, resident)));
     const int grid = int(std::max<int64_t>(
-        1, std::min<int64_t>((n + kThreads - 1) / kThreads, int64_t(sms) * std::min(4, per))));
+        element_ctas, std::min<int64_t>((nlong + kWarps - 1) / kWarps, resident)));
     constexpr int kTurns = 5;
     DevParts mem;
     const size_t optr = mem.add<int64_t>(nn + 1), oidx = mem.add<int64_t>(nz),
                  oval = mem.add<double>(nz), oval32 = mem.add<float>(fp32 ? nz : 0),
-                 orhs = mem.add<double>(nn), ovec = mem.add<double>(10 * nn),
+                 olong = mem.add<int64_t>(size_t(nlong)), orhs = mem.add<double>(nn), ovec = mem.add<double>(10 * nn),
                  opart = mem.add<double>(size_t(kTurns) * 2 * size_t(grid)),
                  ostate = mem.add<NewtonState>(1), osync = mem.add<unsigned>(2);
     mem.alloc();
@@ -387,6 +521,8 @@ inline bool newton_solve_t(const nk_csr &K, const double *rhs, bool precondition
     up(didx, K.index, size_t(nnz) * 8);
     up(dval, K.value, size_t(nnz) * 8);
     up(mem.at<double>(orhs), rhs, nn * 8);
+    int64_t *dlong = mem.at<int64_t>(olong);
+    up(dlong, long_rows.data(), size_t(nlong) * 8);
     cuda_check(cudaMemsetAsync(mem.at<unsigned>(osync), 0, 8, s), "Newton counters");
     cuda_check(cudaMemsetAsync(mem.at<NewtonState>(ostate), 0, sizeof(NewtonState), s),
                "Newton state");
@@ -401,6 +537,9 @@ inline bool newton_solve_t(const nk_csr &K, const double *rhs, bool precondition
         v.val = dval32;
     } else
         v.val = dval;
+    v.long_rows = dlong;
+    v.nlong = nlong;
+    v.element_ctas = element_ctas;
     v.rhs = mem.at<double>(orhs);
     double *dinv = vec, *diag = vec + nn;
     v.dinv = dinv;
@@ -413,7 +552,13 @@ inline bool newton_solve_t(const nk_csr &K, const double *rhs, bool precondition
     v.tolerance = fp32 ? 1e-6 : 1e-10;
     if (precondition) {
         newton_diagonal<<<grid_for(n), kThreads, 0, s>>>(n, dptr, didx, dval, diag);
+        if (nlong)
+            newton_long_diagonal<<<grid_for(32 * nlong), kThreads, 0, s>>>(nlong, dlong, dptr, didx,
+                                                                          dval, diag);
         newton_scales<<<grid_for(n), kThreads, 0, s>>>(n, dptr, didx, dval, diag, dinv);
+        if (nlong)
+            newton_long_scales<<<grid_for(32 * nlong), kThreads, 0, s>>>(nlong, dlong, dptr, didx,
+                                                                        dval, diag, dinv);
     } else
         newton_ones<<<grid_for(n), kThreads, 0, s>>>(n, dinv);
     cuda_check(cudaGetLastError(), "Newton preconditioner");

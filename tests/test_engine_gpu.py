@@ -879,3 +879,62 @@ def test_adaptive_panel_engines_of_different_widths_coexist(gpu):
     assert not (info[0]["resident"] or info[1]["resident"])
     for g, m in zip((wide, narrow), models):
         assert g.advance(20, *step_sizes(m)) > 0
+
+
+def long_row_system(kind):
+    """Newton systems with rows of many entries, as (rows, cols, values, n): dense; 40
+    full rows and columns at the end of short ones (two warps' rows); rows of 31 to
+    65 and of 257 entries; and a saddle point whose zero block's rows hold 40 entries
+    and no diagonal."""
+    rng = np.random.default_rng(14)
+    if kind == "saddle":
+        m, per = 150, 40
+        n = m * per
+        h = rng.uniform(0.1, 10, n)
+        # rows without a common column, of scales from 1e-3 to 1e3: the Schur
+        # complement is diagonal, and with it exact BiCGSTAB needs a few steps
+        a = rng.uniform(0.5, 2, n) * np.repeat(10.0 ** rng.uniform(-3, 3, m), per)
+        i, j = n + np.repeat(np.arange(m), per), np.arange(n)
+        return np.r_[j, i, j], np.r_[j, j, i], np.r_[h, a, a], n + m
+    if kind == "dense":
+        n = 300
+        r, c = np.divmod(np.arange(n * n), n)
+    elif kind == "arrow":
+        n, full = 5000, 40
+        r, c = np.repeat(np.arange(n), 3), rng.integers(0, n, 3 * n)
+        i, j = np.repeat(np.arange(n - full, n), n), np.tile(np.arange(n), full)
+        r, c = np.r_[r, i, j], np.r_[c, j, i]
+    else:
+        n = 2000
+        lens = np.r_[np.arange(30, 65), 256, np.full(n - 36, 4)]
+        r = np.repeat(np.arange(n), lens)
+        c = np.concatenate([rng.choice(n, k, replace=False) for k in lens])
+    key = np.unique((r * n + c)[r != c])
+    r, c = key // n, key % n
+    off = rng.uniform(-1, 1, r.size) * 0.5 / np.maximum(1, np.bincount(r, minlength=n))[r]
+    return np.r_[r, np.arange(n)], np.r_[c, np.arange(n)], np.r_[off, np.full(n, 4.0)], n
+
+
+@pytest.mark.parametrize("fp32", [False, True])
+@pytest.mark.parametrize("kind", ["dense", "arrow", "edges", "saddle"])
+def test_linear_solve_long_rows(gpu, kind, fp32):
+    """Rows of more than 32 entries are products of a warp each, and their scales are
+    summed by one in the rows' order.  Held to the stopping target, twice for the
+    drift of the recurrence's residual over a few dozen steps; the saddle point's rows
+    differ in scale by six orders, so it converges only with the right scales."""
+    rows, cols, vals, n = long_row_system(kind)
+    order = np.lexsort((cols, rows))
+    ptr = np.r_[0, np.cumsum(np.bincount(rows, minlength=n))].astype(np.int64)
+    idx, val = cols[order].astype(np.int64), vals[order]
+    rhs = np.random.default_rng(15).standard_normal(n)
+    x, ok = gpu.linear_solve(ptr, idx, val, rhs, fp32_matrix=fp32)
+    assert ok
+    if fp32:
+        val = val.astype(np.float32).astype(np.float64)
+    residual = rhs - np.add.reduceat(val * x[idx], ptr[:-1])
+    assert np.linalg.norm(residual) <= 2 * (1e-6 if fp32 else 1e-10) * (1 + np.linalg.norm(rhs))
+    if kind != "saddle":
+        y, ok = gpu.linear_solve(ptr, idx, val, rhs, fp32_matrix=fp32, precondition=False)
+        assert ok
+        # two answers within the target, of a matrix with ||K^-1|| <= 1/3.5
+        assert np.max(np.abs(x - y)) <= (1e-6 if fp32 else 1e-10) * (1 + np.linalg.norm(rhs))
