@@ -39,7 +39,7 @@ namespace nk {
 
 struct NewtonState {
     double rho, previous, alpha, omega, target;
-    int stop;      // 0 running, 1 converged, 2 breakdown
+    int stop;      // 0 running, 1 converged, 2 breakdown, 3 out of time
     int converged; // 1 once a residual met the target
     int fault;     // a wait was given up
 };
@@ -60,9 +60,17 @@ template <class V> struct NewtonView {
     double *part;   // two sums per CTA, for each of the iteration's barriers in turn
     unsigned *sync; // [0] arrivals, [1] CTAs done; zero between launches
     NewtonState *st;
+    double *late;     // nonzero once the launch has run for `budget`
+    long long budget; // nanoseconds
     double tolerance;
     int iterations, first; // of this launch; first: form r, rho and the target
 };
+
+__device__ __forceinline__ long long clock_ns() {
+    long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
+}
 
 // Row `base + lane`'s product with x, for the warp's 32 rows: 8, 16 or 32 lanes a
 // row (the warp's longest row decides), lane-strided, then a fixed shuffle tree.
@@ -163,7 +171,8 @@ __device__ __forceinline__ bool newton_barrier(const NewtonView<V> &K, unsigned 
 }
 
 // Grid-wide sums of (a, b) in every thread: CTA trees, a barrier, and the CTAs'
-// sums added by every CTA in one order.  `turn` picks the partials' place.
+// sums added by every CTA in one order.  `turn` picks the partials' place.  In
+// turn 4, what CTA 0 left at K.late before the barrier comes along in out[2].
 template <class V>
 __device__ __forceinline__ bool newton_sum(const NewtonView<V> &K, int turn, unsigned *barrier,
                                            double (&ab)[2], double *red, double *out, int *ok) {
@@ -175,6 +184,7 @@ __device__ __forceinline__ bool newton_sum(const NewtonView<V> &K, int turn, uns
     }
     if (!newton_barrier(K, barrier, ok))
         return false;
+    const double late = turn == 4 && threadIdx.x == 0 ? __ldcg(K.late) : 0.;
     ab[0] = ab[1] = 0;
     for (unsigned b = threadIdx.x; b < gridDim.x; b += kThreads) {
         ab[0] += __ldcg(part + 2 * b);
@@ -184,6 +194,7 @@ __device__ __forceinline__ bool newton_sum(const NewtonView<V> &K, int turn, uns
     if (threadIdx.x == 0) {
         out[0] = ab[0];
         out[1] = ab[1];
+        out[2] = late;
     }
     __syncthreads();
     ab[0] = out[0];
@@ -193,7 +204,7 @@ __device__ __forceinline__ bool newton_sum(const NewtonView<V> &K, int turn, uns
 
 template <class V>
 __global__ void __launch_bounds__(kThreads, 4) newton_kernel(NewtonView<V> K) {
-    __shared__ double red[kWarps * 2], sums[2];
+    __shared__ double red[kWarps * 2], sums[3];
     __shared__ unsigned barrier; // thread 0's count
     __shared__ int ok;
     // the CTAs past element_ctas only walk long rows
@@ -212,6 +223,7 @@ __global__ void __launch_bounds__(kThreads, 4) newton_kernel(NewtonView<V> K) {
         ok = 1;
     }
     __syncthreads();
+    const long long start = clock_ns();
     double rho, previous = 1, alpha = 1, omega = 1, target;
     int stop = 0, converged = 0, it = 0;
     auto leave = [&] {
@@ -338,10 +350,15 @@ __global__ void __launch_bounds__(kThreads, 4) newton_kernel(NewtonView<V> K) {
             ab[0] += r * r;
             ab[1] += K.rhs[e] * r;
         }
+        // CTA 0 looks at the clock for all, since all must stop after the same iteration
+        if (blockIdx.x == 0 && threadIdx.x == 0)
+            __stcg(K.late, clock_ns() - start >= K.budget ? 1. : 0.);
         if (!newton_sum(K, 4, &barrier, ab, red, sums, &ok))
             return;
         converged = sqrt(ab[0]) <= target;
         stop = converged;
+        if (!stop && it + 1 < K.iterations && sums[2] != 0)
+            stop = 3;
         previous = rho;
         rho = ab[1];
     }
@@ -466,9 +483,10 @@ __global__ void newton_ones(int64_t n, double *dinv) {
 // reference's one exactly: every scaling is by 1).  The residual r stays the
 // unpreconditioned one, so the stopping test is the reference's.  Returns true
 // when a residual met the target ((fp32 ? 1e-6 : 1e-10) (1 + |rhs|)) before
-// breakdown, the iteration cap (min(20000, 10 n + 100)) or the time limit
-// (looked at before every launch of kNewtonChunk iterations); x gets the last
-// iterate either way.  The arguments are checked by the caller.
+// breakdown, the iteration cap (min(20000, 10 n + 100)) or the time limit (looked
+// at before every iteration: by the host between launches of kNewtonChunk, by the
+// kernel within one); x gets the last iterate either way.  The arguments are
+// checked by the caller.
 template <class V>
 inline bool newton_solve_t(const nk_csr &K, const double *rhs, bool precondition, double time_limit,
                            double *x_out, bool *timed_out) {
@@ -503,12 +521,13 @@ inline bool newton_solve_t(const nk_csr &K, const double *rhs, bool precondition
         int(std::max<int64_t>(1, std::min<int64_t>((n + kThreads - 1) / kThreads, resident)));
     const int grid = int(std::max<int64_t>(
         element_ctas, std::min<int64_t>((nlong + kWarps - 1) / kWarps, resident)));
-    constexpr int kTurns = 5;
+    constexpr size_t kTurns = 5;
     DevParts mem;
     const size_t optr = mem.add<int64_t>(nn + 1), oidx = mem.add<int64_t>(nz),
                  oval = mem.add<double>(nz), oval32 = mem.add<float>(fp32 ? nz : 0),
-                 olong = mem.add<int64_t>(size_t(nlong)), orhs = mem.add<double>(nn), ovec = mem.add<double>(10 * nn),
-                 opart = mem.add<double>(size_t(kTurns) * 2 * size_t(grid)),
+                 olong = mem.add<int64_t>(size_t(nlong)), orhs = mem.add<double>(nn),
+                 ovec = mem.add<double>(10 * nn),
+                 opart = mem.add<double>(kTurns * 2 * size_t(grid) + 1),
                  ostate = mem.add<NewtonState>(1), osync = mem.add<unsigned>(2);
     mem.alloc();
     int64_t *dptr = mem.at<int64_t>(optr), *didx = mem.at<int64_t>(oidx);
@@ -547,6 +566,8 @@ inline bool newton_solve_t(const nk_csr &K, const double *rhs, bool precondition
     for (size_t k = 0; k < 8; ++k)
         *dst[k] = vec + (2 + k) * nn;
     v.part = mem.at<double>(opart);
+    v.late = v.part + kTurns * 2 * size_t(grid);
+    cuda_check(cudaMemsetAsync(v.late, 0, sizeof(double), s), "Newton state");
     v.sync = mem.at<unsigned>(osync);
     v.st = mem.at<NewtonState>(ostate);
     v.tolerance = fp32 ? 1e-6 : 1e-10;
@@ -568,8 +589,11 @@ inline bool newton_solve_t(const nk_csr &K, const double *rhs, bool precondition
     for (int64_t it = 0; !h.stop && (it < cap || it == 0); it += v.iterations) {
         // a first launch without time forms the target only, and a residual that
         // already meets it still counts
-        const bool late = std::chrono::duration<double>(std::chrono::steady_clock::now() - start)
-                              .count() >= time_limit;
+        const double left =
+            time_limit -
+            std::chrono::duration<double>(std::chrono::steady_clock::now() - start).count();
+        const bool late = left <= 0;
+        v.budget = left < 1e9 ? (long long)(1e9 * left) : INT64_MAX;
         if (late && it > 0) {
             *timed_out = true;
             break;
@@ -584,8 +608,8 @@ inline bool newton_solve_t(const nk_csr &K, const double *rhs, bool precondition
         cuda_check(cudaStreamSynchronize(s), "Newton state");
         if (h.fault)
             throw Error(NK_ERR_CUDA, "a wait inside the Newton kernel was given up");
-        if (late) {
-            *timed_out = !h.stop;
+        if (late || h.stop == 3) {
+            *timed_out = !h.stop || h.stop == 3;
             break;
         }
     }

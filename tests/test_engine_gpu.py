@@ -938,3 +938,30 @@ def test_linear_solve_long_rows(gpu, kind, fp32):
         assert ok
         # two answers within the target, of a matrix with ||K^-1|| <= 1/3.5
         assert np.max(np.abs(x - y)) <= (1e-6 if fp32 else 1e-10) * (1 + np.linalg.norm(rhs))
+
+
+def test_linear_solve_time_limit_within_a_launch(gpu):
+    """The time limit is looked at before every iteration.  8 M unknowns on a periodic
+    grid whose matrix is singular, so that no residual meets the target: 64 iterations
+    take tens of milliseconds, one takes less than one, so a limit of 10 ms ends the
+    call no more than 15 ms (several times the spread of its uploads) later than a
+    limit of 0 does, the limit itself aside."""
+    import time
+    n = 8_000_000
+    i = np.arange(n)
+    idx = np.concatenate([(i + d) % n for d in (0, 1, -1, 200, -200, 40_000, -40_000)])
+    idx = np.ascontiguousarray(idx.reshape(7, n).T).reshape(-1)
+    val = np.tile([6.0, -1, -1, -1, -1, -1, -1], n)
+    ptr = 7 * np.arange(n + 1, dtype=np.int64)
+    rhs = np.random.default_rng(16).standard_normal(n)
+
+    def seconds(limit):
+        best = np.inf
+        for _ in range(5):
+            start = time.perf_counter()
+            with pytest.raises(TimeoutError):
+                gpu.linear_solve(ptr, idx, val, rhs, time_limit=limit)
+            best = min(best, time.perf_counter() - start)
+        return best
+
+    assert seconds(0.01) - seconds(0.0) <= 0.01 + 0.015
