@@ -30,6 +30,7 @@
 #pragma once
 #include "nk_common.cuh"
 #include "nk_kernels.cuh"
+#include <algorithm>
 #include <chrono>
 #include <cmath>
 #include <cstdint>
@@ -47,6 +48,7 @@ struct NewtonState {
 constexpr int kNewtonLong = 32;          // rows of more entries have a warp each
 constexpr int kNewtonChunk = 64;         // iterations of one launch
 constexpr int kNewtonMaxPolls = 4 << 20; // seconds: the barrier's bound
+constexpr int64_t kNewtonStage = int64_t(1) << 24; // FP64 entries held at a time for FP32 ones
 
 template <class V> struct NewtonView {
     int64_t n;
@@ -370,7 +372,8 @@ __global__ void __launch_bounds__(kThreads, 4) newton_kernel(NewtonView<V> K) {
 // point's regularised zero block, |K_ii| < 1e-8 max_j |K_ij|), the diagonal of
 // the row's Schur complement, sum_j K_ij^2 / |K_jj| over the other entries.
 // Rows with neither keep 1.  Two passes: the diagonals and whether they carry
-// their rows (diag: 0 where not), then the scales.  A thread takes a row; a long
+// their rows (diag: 0 where not), then the scales; each over rows [first, last) or
+// a part of the long rows, whose entries val holds.  A thread takes a row; a long
 // row (newton_long_*) a warp, which loads 32 entries at a time and adds them in
 // the same order, entry by entry.
 __device__ __forceinline__ double carrying(double d, double big) {
@@ -382,11 +385,11 @@ __device__ __forceinline__ double schur_term(double a, int64_t i, int64_t j, con
 __device__ __forceinline__ double newton_scale(double d, double schur) {
     return d != 0 ? 1 / fabs(d) : schur > 0 && isfinite(schur) ? 1 / schur : 1.;
 }
-__global__ void newton_diagonal(int64_t n, const int64_t *__restrict__ ptr,
+__global__ void newton_diagonal(int64_t first, int64_t last, const int64_t *__restrict__ ptr,
                                 const int64_t *__restrict__ idx, const double *__restrict__ val,
                                 double *__restrict__ diag) {
     const int64_t stride = int64_t(gridDim.x) * blockDim.x;
-    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
+    for (int64_t i = first + int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < last; i += stride) {
         const int64_t b = ptr[i], e = ptr[i + 1];
         if (e - b > kNewtonLong)
             continue;
@@ -426,11 +429,11 @@ __global__ void newton_long_diagonal(int64_t nlong, const int64_t *__restrict__ 
             diag[i] = carrying(d, big);
     }
 }
-__global__ void newton_scales(int64_t n, const int64_t *__restrict__ ptr,
+__global__ void newton_scales(int64_t first, int64_t last, const int64_t *__restrict__ ptr,
                               const int64_t *__restrict__ idx, const double *__restrict__ val,
                               const double *__restrict__ diag, double *__restrict__ dinv) {
     const int64_t stride = int64_t(gridDim.x) * blockDim.x;
-    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
+    for (int64_t i = first + int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < last; i += stride) {
         const int64_t b = ptr[i], e = ptr[i + 1];
         double schur = 0;
         if (diag[i] == 0) {
@@ -522,9 +525,20 @@ inline bool newton_solve_t(const nk_csr &K, const double *rhs, bool precondition
     const int grid = int(std::max<int64_t>(
         element_ctas, std::min<int64_t>((nlong + kWarps - 1) / kWarps, resident)));
     constexpr size_t kTurns = 5;
+    // the FP64 values: all of them, or for FP32 ones as many whole rows at a time as
+    // hold kNewtonStage entries (one row at least), to be converted
+    std::vector<int64_t> cuts{0};
+    int64_t staged = 1;
+    while (cuts.back() < n) {
+        const int64_t r = cuts.back(), from = K.ptr[r],
+                      to = fp32 ? from + std::min(nnz - from, kNewtonStage) : nnz;
+        const int64_t fit = std::upper_bound(K.ptr + r, K.ptr + n + 1, to) - K.ptr - 1;
+        cuts.push_back(std::max(fit, r + 1));
+        staged = std::max(staged, K.ptr[cuts.back()] - from);
+    }
     DevParts mem;
     const size_t optr = mem.add<int64_t>(nn + 1), oidx = mem.add<int64_t>(nz),
-                 oval = mem.add<double>(nz), oval32 = mem.add<float>(fp32 ? nz : 0),
+                 oval = mem.add<double>(size_t(staged)), oval32 = mem.add<float>(fp32 ? nz : 0),
                  olong = mem.add<int64_t>(size_t(nlong)), orhs = mem.add<double>(nn),
                  ovec = mem.add<double>(10 * nn),
                  opart = mem.add<double>(kTurns * 2 * size_t(grid) + 1),
@@ -538,7 +552,6 @@ inline bool newton_solve_t(const nk_csr &K, const double *rhs, bool precondition
     };
     up(dptr, K.ptr, (nn + 1) * 8);
     up(didx, K.index, size_t(nnz) * 8);
-    up(dval, K.value, size_t(nnz) * 8);
     up(mem.at<double>(orhs), rhs, nn * 8);
     int64_t *dlong = mem.at<int64_t>(olong);
     up(dlong, long_rows.data(), size_t(nlong) * 8);
@@ -549,12 +562,9 @@ inline bool newton_solve_t(const nk_csr &K, const double *rhs, bool precondition
     v.n = n;
     v.ptr = dptr;
     v.idx = didx;
-    if constexpr (fp32) {
-        float *dval32 = mem.at<float>(oval32);
-        if (nnz)
-            to_float<<<grid_for(nnz), kThreads, 0, s>>>(nnz, dval, dval32);
-        v.val = dval32;
-    } else
+    if constexpr (fp32)
+        v.val = mem.at<float>(oval32);
+    else
         v.val = dval;
     v.long_rows = dlong;
     v.nlong = nlong;
@@ -571,16 +581,43 @@ inline bool newton_solve_t(const nk_csr &K, const double *rhs, bool precondition
     v.sync = mem.at<unsigned>(osync);
     v.st = mem.at<NewtonState>(ostate);
     v.tolerance = fp32 ? 1e-6 : 1e-10;
-    if (precondition) {
-        newton_diagonal<<<grid_for(n), kThreads, 0, s>>>(n, dptr, didx, dval, diag);
-        if (nlong)
-            newton_long_diagonal<<<grid_for(32 * nlong), kThreads, 0, s>>>(nlong, dlong, dptr, didx,
-                                                                          dval, diag);
-        newton_scales<<<grid_for(n), kThreads, 0, s>>>(n, dptr, didx, dval, diag, dinv);
-        if (nlong)
-            newton_long_scales<<<grid_for(32 * nlong), kThreads, 0, s>>>(nlong, dlong, dptr, didx,
-                                                                        dval, diag, dinv);
-    } else
+    // Rows [cuts[q], cuts[q + 1]): their FP64 values to the device (unless they are
+    // there, being all), then rows(first, last, long rows, their number, values by
+    // the entries' own offsets).
+    bool uploaded = false;
+    auto for_values = [&](auto rows) {
+        for (size_t q = 0; q + 1 < cuts.size(); ++q) {
+            const int64_t r0 = cuts[q], r1 = cuts[q + 1], k0 = K.ptr[r0], count = K.ptr[r1] - k0;
+            if (!uploaded)
+                up(dval, K.value + k0, size_t(count) * 8);
+            const auto l0 = std::lower_bound(long_rows.begin(), long_rows.end(), r0),
+                       l1 = std::lower_bound(l0, long_rows.end(), r1);
+            rows(r0, r1, dlong + (l0 - long_rows.begin()), int64_t(l1 - l0), dval - k0);
+        }
+        uploaded = cuts.size() == 2;
+    };
+    for_values([&](int64_t r0, int64_t r1, const int64_t *rows, int64_t count, const double *val) {
+        if constexpr (fp32)
+            if (const int64_t k0 = K.ptr[r0], k1 = K.ptr[r1]; k1 > k0)
+                to_float<<<grid_for(k1 - k0), kThreads, 0, s>>>(k1 - k0, val + k0,
+                                                               mem.at<float>(oval32) + k0);
+        if (!precondition)
+            return;
+        newton_diagonal<<<grid_for(r1 - r0), kThreads, 0, s>>>(r0, r1, dptr, didx, val, diag);
+        if (count)
+            newton_long_diagonal<<<grid_for(32 * count), kThreads, 0, s>>>(count, rows, dptr, didx,
+                                                                          val, diag);
+    });
+    if (precondition)
+        for_values([&](int64_t r0, int64_t r1, const int64_t *rows, int64_t count,
+                       const double *val) {
+            newton_scales<<<grid_for(r1 - r0), kThreads, 0, s>>>(r0, r1, dptr, didx, val, diag,
+                                                                dinv);
+            if (count)
+                newton_long_scales<<<grid_for(32 * count), kThreads, 0, s>>>(count, rows, dptr, didx,
+                                                                            val, diag, dinv);
+        });
+    else
         newton_ones<<<grid_for(n), kThreads, 0, s>>>(n, dinv);
     cuda_check(cudaGetLastError(), "Newton preconditioner");
     const int64_t cap = std::min<int64_t>(20000, 10 * n + 100);

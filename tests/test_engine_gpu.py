@@ -965,3 +965,51 @@ def test_linear_solve_time_limit_within_a_launch(gpu):
         return best
 
     assert seconds(0.01) - seconds(0.0) <= 0.01 + 0.015
+
+
+def test_linear_solve_fp32_memory(gpu):
+    """FP32 values take 4 bytes an entry on the device beside 8 for the index; the FP64
+    ones they and the scales are formed from pass through 128 MB at a time.  40 M
+    entries, three such parts, in rows of 41 and 601.  Columns differ in scale by six
+    orders, so the solve converges only with every column's scale right."""
+    import threading
+    import torch
+    n = 125_000
+    rng = np.random.default_rng(17)
+    lens = np.where(np.arange(n) % 2 == 0, 600, 40)
+    row = np.repeat(np.arange(n), lens)
+    col = (row + 1 + rng.integers(0, n - 1, row.size)) % n
+    scale = (10.0 ** rng.uniform(-3, 3, n)).astype(np.float32).astype(np.float64)
+    off = rng.uniform(-0.5, 0.5, row.size) / np.repeat(lens, lens)
+    ptr = np.r_[0, np.cumsum(lens + 1)].astype(np.int64)
+    idx = np.empty(ptr[-1], dtype=np.int64)
+    val = np.empty(ptr[-1])
+    first = np.zeros(ptr[-1], dtype=bool)
+    first[ptr[:-1]] = True
+    idx[first], idx[~first] = np.arange(n), col
+    val[first], val[~first] = 4 * scale, off * scale[col]
+    rhs = rng.standard_normal(n)
+    gpu.linear_solve(ptr[:2], np.zeros(601, dtype=np.int64), np.ones(601), rhs[:1],
+                     fp32_matrix=True)  # context and kernels
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    least, done = [before], threading.Event()
+
+    def watch():
+        while not done.wait(0.001):
+            least[0] = min(least[0], torch.cuda.mem_get_info()[0])
+    watcher = threading.Thread(target=watch)
+    watcher.start()
+    try:
+        x, ok = gpu.linear_solve(ptr, idx, val, rhs, fp32_matrix=True)
+    finally:
+        done.set()
+        watcher.join()
+    assert ok
+    val = val.astype(np.float32).astype(np.float64)
+    residual = rhs - np.add.reduceat(val * x[idx], ptr[:-1])
+    assert np.linalg.norm(residual) <= 2e-6 * (1 + np.linalg.norm(rhs))
+    used = before - least[0]
+    # entries, the 128 MB, a dozen vectors, and 48 MB for what else the driver takes
+    bound = 12 * ptr[-1] + (128 << 20) + 12 * 8 * n + (48 << 20)
+    assert 12 * ptr[-1] < used <= bound, (used, bound)
