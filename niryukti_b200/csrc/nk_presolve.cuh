@@ -95,15 +95,18 @@ inline int64_t compact_csr(const nk_csr &M, int64_t rows, const int64_t *kept, c
     cuda_check(cub::DeviceScan::ExclusiveSum(nullptr, temp, static_cast<int64_t *>(nullptr),
                                              static_cast<int64_t *>(nullptr), rows + 1, s),
                "compaction scan size");
-    // one allocation; the output holds at most `capacity` entries and the source's
-    const size_t most = size_t(std::max<int64_t>(1, std::min(nnz, capacity)));
+    // one allocation; the output too (at most `capacity` entries and the source's)
+    // where that is 16 MB at most, else in memory of its own once its size is known
+    const int64_t most = std::min(nnz, capacity);
+    const bool together = most <= int64_t(1) << 20;
+    const size_t reserved = together ? size_t(std::max<int64_t>(1, most)) : 0;
     DevParts mem;
     const size_t optr_ = mem.add<int64_t>(size_t(M.rows + 1)), oidx_ = mem.add<int64_t>(size_t(nnz)),
                  oval_ = mem.add<double>(size_t(nnz)), okept_ = mem.add<int64_t>(size_t(rows)),
                  omap_ = mem.add<int64_t>(size_t(M.cols)),
                  ocounts_ = mem.add<int64_t>(size_t(rows + 1)),
                  oout_ = mem.add<int64_t>(size_t(rows + 1)), owork_ = mem.add<unsigned char>(temp),
-                 ooidx_ = mem.add<int64_t>(most), ooval_ = mem.add<double>(most);
+                 ooidx_ = mem.add<int64_t>(reserved), ooval_ = mem.add<double>(reserved);
     mem.alloc();
     int64_t *dptr = mem.at<int64_t>(optr_), *didx = mem.at<int64_t>(oidx_),
             *dkept = mem.at<int64_t>(okept_), *dmap = mem.at<int64_t>(omap_),
@@ -136,6 +139,12 @@ inline int64_t compact_csr(const nk_csr &M, int64_t rows, const int64_t *kept, c
     if (total > capacity)
         throw Error(NK_ERR_INVALID, "compaction output capacity is too small");
     if (total) {
+        DevBuf<int64_t> own_idx(together ? 0 : size_t(total));
+        DevBuf<double> own_val(together ? 0 : size_t(total));
+        if (!together) {
+            oidx = own_idx.p;
+            oval = own_val.p;
+        }
         compact_scatter<<<grid, kThreads, 0, s>>>(rows, dkept, dptr, didx, dval, dmap, optr, oidx,
                                                   oval);
         cuda_check(cudaGetLastError(), "compaction scatter");

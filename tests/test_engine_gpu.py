@@ -967,13 +967,32 @@ def test_linear_solve_time_limit_within_a_launch(gpu):
     assert seconds(0.01) - seconds(0.0) <= 0.01 + 0.015
 
 
+def device_bytes_during(call):
+    """call()'s result and the most device memory that was taken while it ran."""
+    import threading
+    import torch
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    least, done = [before], threading.Event()
+
+    def watch():
+        while not done.wait(0.001):
+            least[0] = min(least[0], torch.cuda.mem_get_info()[0])
+    watcher = threading.Thread(target=watch)
+    watcher.start()
+    try:
+        result = call()
+    finally:
+        done.set()
+        watcher.join()
+    return result, before - least[0]
+
+
 def test_linear_solve_fp32_memory(gpu):
     """FP32 values take 4 bytes an entry on the device beside 8 for the index; the FP64
     ones they and the scales are formed from pass through 128 MB at a time.  40 M
     entries, three such parts, in rows of 41 and 601.  Columns differ in scale by six
     orders, so the solve converges only with every column's scale right."""
-    import threading
-    import torch
     n = 125_000
     rng = np.random.default_rng(17)
     lens = np.where(np.arange(n) % 2 == 0, 600, 40)
@@ -991,25 +1010,35 @@ def test_linear_solve_fp32_memory(gpu):
     rhs = rng.standard_normal(n)
     gpu.linear_solve(ptr[:2], np.zeros(601, dtype=np.int64), np.ones(601), rhs[:1],
                      fp32_matrix=True)  # context and kernels
-    torch.cuda.synchronize()
-    before = torch.cuda.mem_get_info()[0]
-    least, done = [before], threading.Event()
-
-    def watch():
-        while not done.wait(0.001):
-            least[0] = min(least[0], torch.cuda.mem_get_info()[0])
-    watcher = threading.Thread(target=watch)
-    watcher.start()
-    try:
-        x, ok = gpu.linear_solve(ptr, idx, val, rhs, fp32_matrix=True)
-    finally:
-        done.set()
-        watcher.join()
+    (x, ok), used = device_bytes_during(
+        lambda: gpu.linear_solve(ptr, idx, val, rhs, fp32_matrix=True))
     assert ok
     val = val.astype(np.float32).astype(np.float64)
     residual = rhs - np.add.reduceat(val * x[idx], ptr[:-1])
     assert np.linalg.norm(residual) <= 2e-6 * (1 + np.linalg.norm(rhs))
-    used = before - least[0]
     # entries, the 128 MB, a dozen vectors, and 48 MB for what else the driver takes
     bound = 12 * ptr[-1] + (128 << 20) + 12 * 8 * n + (48 << 20)
     assert 12 * ptr[-1] < used <= bound, (used, bound)
+
+
+@pytest.mark.parametrize("kept", [1, 3])
+def test_compaction_memory(gpu, kept):
+    """The device holds the source and the entries that are kept, not room for all that
+    could be: 40 M entries, of which a few columns keep 1 in 1,000 (an output inside
+    the call's one allocation would take 640 MB more) or 3 in 4."""
+    rows, per, n = 400_000, 100, 1000
+    rng = np.random.default_rng(18)
+    idx = np.sort(rng.integers(0, n, (rows, per)), axis=1).reshape(-1)
+    val = rng.standard_normal(idx.size)
+    ptr = per * np.arange(rows + 1, dtype=np.int64)
+    stay = np.zeros(n, dtype=bool)
+    stay[500 if kept == 1 else np.arange(n) % 4 != 0] = True
+    cmap = np.where(stay, np.cumsum(stay) - 1, -1)
+    gpu.compact_csr(ptr[:2], idx[:per], val[:per], n, [0], cmap, int(stay.sum()))
+    (p, i, v), used = device_bytes_during(
+        lambda: gpu.compact_csr(ptr, idx, val, n, np.arange(rows), cmap, int(stay.sum())))
+    take = stay[idx]
+    assert np.array_equal(i, cmap[idx[take]]) and np.array_equal(v, val[take])
+    assert np.array_equal(p, np.r_[0, np.cumsum(take.reshape(rows, per).sum(axis=1))])
+    bound = 16 * (idx.size + i.size) + 8 * (5 * rows + n) + (48 << 20)
+    assert 16 * idx.size < used <= bound, (used, bound)
