@@ -623,7 +623,6 @@ class Batch {
     int ncols_ = 0, nrows_ = 0;
     int64_t trial_bytes_ = 0;
     bool dirty_ = true, tuned_ = false;
-    bool deal_p_ = false, deal_d_ = false; // items dealt although there are many instances
     int vp_ = 13, vd_ = 13; // kernel variants (autotuned, see launch_half)
     float ms_primal_ = 0, ms_dual_ = 0; // their best times when tuned
     // wall seconds per part of a check interval: control upload, trials,
@@ -846,12 +845,14 @@ class Batch {
         // the items are sorted by cost, costliest first (a stable counting
         // sort), and dealt one per CTA per round, alternating direction (round
         // k to CTAs 0..G-1 when k is even, G-1..0 when odd).
-        // Which of the two wins at 64 instances and more depends on their sizes (96
-        // instances up to m = 50,000: a check interval of 18.2 ms with segments, 17.2
-        // dealt; 128 up to 30,000: 15.4 and 15.5), so the tuner times both there.
-        constexpr int kSegments = 4;
+        // The line lies where the two meet.  Check intervals in ms, segments / dealt:
+        // 64 instances up to m = 50,000 12.7 / 11.9, 96 17.9 / 16.9 (FP32 values 17.8 /
+        // 16.4), 128 up to 8,000 6.6 / 5.9, 128 up to 30,000 15.2 / 15.2, 192 up to
+        // 20,000 16.4 / 16.4, 256 up to 20,000 21.0 / 21.6.
+        constexpr int kSegments = 4, kSegmentInstances = 192;
+        const bool segmented = int(order_.size()) >= kSegmentInstances;
         auto place = [&](WorkList &W, const std::vector<BWork> &items,
-                         const std::vector<int64_t> &icost, int t, bool segmented) {
+                         const std::vector<int64_t> &icost, int t) {
             const int ncta = std::max(1, std::min<int>(int(items.size()), sms_ * resident_[t]));
             std::vector<int> owner(items.size());
             std::vector<int> coff(size_t(ncta + 1), 0);
@@ -913,13 +914,13 @@ class Batch {
                 auto wc = runs(cols, ccost, cf, cc, kRunLength[r], icost);
                 for (int t = 0; t < kCtaSizes; ++t)
                     if (!tuned_ || t == vp_ % 3)
-                        place(wcols_[r][t], wc, icost, t, many_instances() && !deal_p_);
+                        place(wcols_[r][t], wc, icost, t);
             }
             if (!tuned_ || r == vd_ / 9) {
                 auto wr = runs(rows, rcost, rf, rc, kRunLength[r], icost);
                 for (int t = 0; t < kCtaSizes; ++t)
                     if (!tuned_ || t == vd_ % 3)
-                        place(wrows_[r][t], wr, icost, t, many_instances() && !deal_d_);
+                        place(wrows_[r][t], wr, icost, t);
             }
         }
         ncols_ = int(cols.size());
@@ -956,14 +957,9 @@ class Batch {
         dirty_ = false;
         // tuned once, on the first work list: later tuning would insert trials
         // into running instances' check intervals and change their trajectories
-        if (o_.autotune && !tuned_) {
+        if (o_.autotune && !tuned_)
             autotune();
-            if (many_instances())
-                tune_placement();
-        }
     }
-    static constexpr int kSegmentInstances = 64;
-    bool many_instances() const { return int(order_.size()) >= kSegmentInstances; }
 
     // ---------------------------------------------------------------- launches
     // kernel variant v (autotuned): run length {1, 4, 16}[v / 9], unroll
@@ -998,14 +994,14 @@ class Batch {
         cuda_check(cudaGetLastError(), "batch trial");
     }
 
-    // Best time of a variant's probe launch, of `reps`; a timed dual launch follows
-    // a probe primal launch (it reads that dx).
-    float time_half(int v, bool primal, int reps = 3) {
+    // Best time of a variant's probe launch, of three; a timed dual launch follows a
+    // probe primal launch (it reads that dx).
+    float time_half(int v, bool primal) {
         cudaEvent_t e0, e1;
         cuda_check(cudaEventCreate(&e0), "event");
         cuda_check(cudaEventCreate(&e1), "event");
         float best = 1e30f;
-        for (int rep = 0; rep < reps; ++rep) {
+        for (int rep = 0; rep < 3; ++rep) {
             if (!primal)
                 launch_half(vp_, true, true);
             cuda_check(cudaEventRecord(e0, stream_), "event");
@@ -1019,27 +1015,6 @@ class Batch {
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
         return best;
-    }
-    // With many instances: the chosen variants with their items dealt instead of
-    // in segments, kept where that is faster (where an item runs changes no result).
-    // Both placements are timed anew: the tuner's best of all variants is the
-    // luckiest of many samples.
-    void tune_placement() {
-        constexpr int kReps = 8;
-        ms_primal_ = time_half(vp_, true, kReps);
-        ms_dual_ = time_half(vd_, false, kReps);
-        deal_p_ = deal_d_ = true;
-        dirty_ = true;
-        rebuild_lists();
-        const float tp = time_half(vp_, true, kReps), td = time_half(vd_, false, kReps);
-        deal_p_ = tp < ms_primal_;
-        deal_d_ = td < ms_dual_;
-        ms_primal_ = std::min(ms_primal_, tp);
-        ms_dual_ = std::min(ms_dual_, td);
-        if (!deal_p_ || !deal_d_) {
-            dirty_ = true;
-            rebuild_lists();
-        }
     }
 
     // Autotuner: times every kernel variant on the batch as it stands and
