@@ -250,10 +250,12 @@ __device__ __forceinline__ void propose_entry(double v, int64_t j, const RowActi
 // One pass over the rows.  Reads the bounds of the previous pass (lb, ub) and
 // proposes into new_lb / new_ub; flags a row whose activity range misses
 // [rl, ru].  A thread per row walking its entries twice is two chains of
-// dependent, uncoalesced loads (78 us for 20,000 rows of 16 entries); so a warp
-// takes 32 rows together: the terms are formed flat, entry by entry, into shared
-// memory, a lane adds up its row's in order, and the proposals are formed flat
-// again (48 us).  32 rows of more than kPropEntries entries keep the walk.
+// dependent, uncoalesced loads; so a warp takes 32 rows together, kPropEntries
+// entries at a time: the terms are formed flat, entry by entry, into shared memory,
+// a lane adds up its row's in order, and when all are added the proposals are
+// formed flat again.  us a pass with a thread per row / so: 20,000 rows of 16
+// entries 79 / 47, of 24 entries 103 / 68, 1,000,000 of 24 2,340 / 1,600, 400,000 of
+// 60 1,270 / 1,150, 2,000 of 7,250 26,000 / 23,300 (a long row's sum is one chain).
 constexpr int kPropWarps = 4, kPropEntries = 640;
 __global__ void __launch_bounds__(kPropWarps * 32)
     propagate_rows(int64_t rows, const int64_t *__restrict__ ptr,
@@ -272,53 +274,55 @@ __global__ void __launch_bounds__(kPropWarps * 32)
         const int64_t row = 32 * g + lane, base = ptr[32 * g];
         const int64_t b = ptr[row < rows ? row : rows], e = ptr[row < rows ? row + 1 : rows];
         const double rlo = row < rows ? rl[row] : 0., rhi = row < rows ? ru[row] : 0.;
-        const int64_t total = __shfl_sync(0xffffffffu, e, 31) - base;
+        const int64_t end = __shfl_sync(0xffffffffu, e, 31);
         RowActivity r;
-        if (total > kPropEntries) {
-            for (int64_t k = b; k < e; ++k) {
-                const double v = a[k];
-                if (v != 0)
-                    r.add(term_low(v, lb[index[k]], ub[index[k]]),
-                          term_high(v, lb[index[k]], ub[index[k]]));
+        // the lane's own entries among the n from k0 on, each marked as its row's
+        int first = 0, last = 0;
+        auto own = [&](int64_t k0, int n) {
+            first = int(b < k0 ? 0 : b - k0 < n ? b - k0 : n);
+            last = int(e < k0 ? 0 : e - k0 < n ? e - k0 : n);
+            for (int k = first; k < last; ++k)
+                owner[w][k] = static_cast<unsigned char>(lane);
+            __syncwarp();
+        };
+        for (int64_t k0 = base; k0 < end; k0 += kPropEntries) {
+            const int n = int(end - k0 < kPropEntries ? end - k0 : kPropEntries);
+            own(k0, n);
+            for (int k = lane; k < n; k += 32) {
+                const double v = a[k0 + k];
+                const int64_t j = index[k0 + k];
+                const double l = lb[j], u = ub[j];
+                const int at = k + owner[w][k];
+                // a zero coefficient has no term, whatever its column's bounds
+                lows[w][at] = v != 0 ? term_low(v, l, u) : 0.;
+                highs[w][at] = v != 0 ? term_high(v, l, u) : 0.;
             }
-            if (row < rows && r.misses(rlo, rhi))
-                atomicExch(failed, 1);
-            for (int64_t k = b; k < e; ++k)
-                if (a[k] != 0)
-                    propose_entry(a[k], index[k], r, rlo, rhi, integer, lb[index[k]], ub[index[k]],
-                                  new_lb, new_ub);
-            continue;
+            __syncwarp();
+#pragma unroll 4
+            for (int k = first; k < last; ++k)
+                r.add(lows[w][k + lane], highs[w][k + lane]);
+            __syncwarp();
         }
-        const int first = int(b - base), last = int(e - base), n = int(total);
-        for (int k = first; k < last; ++k)
-            owner[w][k] = static_cast<unsigned char>(lane);
-        __syncwarp();
-        for (int k = lane; k < n; k += 32) {
-            const double v = a[base + k];
-            const int64_t j = index[base + k];
-            const double l = lb[j], u = ub[j];
-            const int at = k + owner[w][k];
-            // a zero coefficient has no term, whatever its column's bounds
-            lows[w][at] = v != 0 ? term_low(v, l, u) : 0.;
-            highs[w][at] = v != 0 ? term_high(v, l, u) : 0.;
-        }
-        __syncwarp();
-        for (int k = first; k < last; ++k)
-            r.add(lows[w][k + lane], highs[w][k + lane]);
         if (row < rows && r.misses(rlo, rhi))
             atomicExch(failed, 1);
         activity[w][lane] = r;
         __syncwarp();
-        for (int k0 = 0; k0 < n; k0 += 32) { // whole warps: the bounds come by shuffle
-            const int k = k0 + lane, q = k < n ? owner[w][k] : 0;
-            const double lo = __shfl_sync(0xffffffffu, rlo, q), hi = __shfl_sync(0xffffffffu, rhi, q);
-            if (k < n && a[base + k] != 0) {
-                const int64_t j = index[base + k];
-                propose_entry(a[base + k], j, activity[w][q], lo, hi, integer, lb[j], ub[j], new_lb,
-                              new_ub);
+        for (int64_t k0 = base; k0 < end; k0 += kPropEntries) {
+            const int n = int(end - k0 < kPropEntries ? end - k0 : kPropEntries);
+            if (end - base > kPropEntries) // else the marks still stand
+                own(k0, n);
+            for (int q0 = 0; q0 < n; q0 += 32) { // whole warps: the bounds come by shuffle
+                const int k = q0 + lane, q = k < n ? owner[w][k] : 0;
+                const double lo = __shfl_sync(0xffffffffu, rlo, q),
+                             hi = __shfl_sync(0xffffffffu, rhi, q);
+                if (k < n && a[k0 + k] != 0) {
+                    const int64_t j = index[k0 + k];
+                    propose_entry(a[k0 + k], j, activity[w][q], lo, hi, integer, lb[j], ub[j],
+                                  new_lb, new_ub);
+                }
             }
+            __syncwarp();
         }
-        __syncwarp();
     }
 }
 

@@ -1042,3 +1042,32 @@ def test_compaction_memory(gpu, kept):
     assert np.array_equal(p, np.r_[0, np.cumsum(take.reshape(rows, per).sum(axis=1))])
     bound = 16 * (idx.size + i.size) + 8 * (5 * rows + n) + (48 << 20)
     assert 16 * idx.size < used <= bound, (used, bound)
+
+
+@pytest.mark.parametrize("lens", [[5000], [0] * 31 + [1281], [640, 0, 1, 639, 3], [20] * 31 + [21],
+                                  [700] * 33, [1] * 32 + [640] * 2 + [5] * 40])
+def test_propagate_bounds_long_groups(gpu, oracle, lens):
+    """Groups of 32 rows with more than the 640 entries that a warp holds at a time: one
+    long row, rows that end at and cross its edges, a single entry more; bit-identical
+    to the sequential restatement."""
+    rng = np.random.default_rng(19)
+    n = sum(lens)
+    cols = np.split(rng.permutation(n), np.cumsum(lens)[:-1])
+    m = tiny(n, len(lens), [(i, int(j), float(v)) for i, js in enumerate(cols)
+                            for j, v in zip(np.sort(js), np.round(rng.standard_normal(js.size), 1))])
+    lb, ub = rng.uniform(-5, 0, n), rng.uniform(0, 40, n)
+    # rows held near their greatest activity, so that most columns are tightened; where
+    # there are several rows, one column of the last without an upper bound
+    row = np.repeat(np.arange(m.m), np.diff(m.ptr))
+    high = np.bincount(row, weights=np.maximum(m.val * lb[m.idx], m.val * ub[m.idx]),
+                       minlength=m.m)
+    m.rl, m.ru = high - rng.uniform(0.5, 3, m.m), np.full(m.m, np.inf)
+    if np.count_nonzero(lens) > 1:
+        ub[m.idx[-1]] = np.inf
+    integer = (np.arange(n) % 3 == 0).astype(np.int32)
+    got = gpu.propagate_bounds(m, integer, lb, ub, 4)
+    want = oracle.propagate_bounds(m, integer, lb, ub, 4)
+    assert got[0] == want[0]
+    assert np.sum((want[1] != lb) | (want[2] != ub)) >= n // 3
+    for u, w in zip(got[1:], want[1:]):
+        assert np.array_equal(u.view(np.int64), w.view(np.int64))
