@@ -1765,6 +1765,12 @@ void plan_resident(Engine &E, const CtaLists &lists_t, const CtaLists &lists_a,
     if (!coop || std::max(R.lists_p, R.lists_d) > kResMaxLists)
         return;
     P.grid = std::min(sms, 1 + int(std::max(E.At.chunk_len.size(), E.A.chunk_len.size())));
+    const size_t value = size_t(E.vbits() / 8), budget = smem_budget(k, 1);
+    // an equal share of the products alone is more than a CTA holds
+    for (const SellMatrix *M : {&E.At, &E.A})
+        if (size_t(std::accumulate(M->chunk_len.begin(), M->chunk_len.end(), int64_t(0))) * 32 * 8 >
+            budget * size_t(P.grid - 1))
+            return;
     std::vector<int> ot = own_ranges(E.At.chunk_len, P.grid - 1),
                      oa = own_ranges(E.A.chunk_len, P.grid - 1);
     ot.push_back(ot.back());
@@ -1785,7 +1791,6 @@ void plan_resident(Engine &E, const CtaLists &lists_t, const CtaLists &lists_a,
     R.entries_t = most(ot, E.At.chunk_len, R.cols);
     R.entries_a = most(oa, E.A.chunk_len, R.rows);
     R.products = std::max(R.entries_t, R.entries_a);
-    const size_t value = size_t(E.vbits() / 8), budget = smem_budget(k, 1);
     int per_sm = 0;
     cuda_check(cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev),
                "shared memory per SM");
@@ -2124,8 +2129,14 @@ Engine *create_engine(const nk_csr *Ah, const nk_csr *Qh, const double *hc, cons
         E->wide ? configure<double, float, int64_t>(*E) : configure<double, float, int32_t>(*E);
     else
         E->wide ? configure<float, float, int64_t>(*E) : configure<float, float, int32_t>(*E);
+    // Adaptive steps amplify a difference of rounding about tenfold every few
+    // trials, so a model whose long rows the panels sum keeps its panels, and their
+    // order of addition, under them.  (4 x 4,000 rows of a block-angular LP with 372
+    // linking rows: the sequential sums' iterates, as accurate, were 5e-8 away after
+    // 40 trials.)  Fixed and Halpern steps don't amplify it.
+    const bool panel_order = E->panels && E->adaptive;
     const CtaLists lists_t = chunk_schedule(E->At, E->grid_p),
-                   lists_a = chunk_schedule(E->A, E->grid_d);
+                   lists_a = panel_order ? CtaLists{} : chunk_schedule(E->A, E->grid_d);
     use_schedule(E->At, lists_t, s);
     use_schedule(E->A, E->panels ? dual_panel_schedule(E->A, E->pan.rows, E->pan.hroff, E->grid_d)
                                  : lists_a, s);
@@ -2135,12 +2146,6 @@ Engine *create_engine(const nk_csr *Ah, const nk_csr *Qh, const double *hc, cons
         E->wide ? attach_slots<double, float, int64_t>(*E) : attach_slots<double, float, int32_t>(*E);
     else
         E->wide ? attach_slots<float, float, int64_t>(*E) : attach_slots<float, float, int32_t>(*E);
-    // Adaptive steps amplify a difference of rounding about tenfold every few
-    // trials, so a model whose long rows the panels sum keeps its panels, and their
-    // order of addition, under them.  (4 x 4,000 rows of a block-angular LP with 372
-    // linking rows: the sequential sums' iterates, as accurate, were 5e-8 away after
-    // 40 trials.)  Fixed and Halpern steps don't amplify it.
-    const bool panel_order = E->panels && E->adaptive;
     if (!panel_order) {
         std::vector<int64_t> engine_rlen(static_cast<size_t>(m)); // longest first
         for (int64_t i = 0; i < m; ++i)
