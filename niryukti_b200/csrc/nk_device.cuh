@@ -271,9 +271,13 @@ __device__ __forceinline__ void ordered_slots(const double *slots, int count, do
 // chunks is finished by whichever warp adds its last segment; its dx^2 goes
 // to that row's own slot (split_p[counter]), added by the decision in row
 // order, so it too lands in the sums the same way every time.
-template <class Acc, class V, class I, bool SPARSE_Q, bool FP32G, bool SPLIT>
+// QX: a sparse Q's part of the gradient, from q_rows_kernel or, for short rows
+// (Q.lanes 1), walked by the column's own lane.
+enum class QX { none, formed, walked };
+template <class Acc, class V, class I, QX Q_X, bool FP32G, bool SPLIT>
 __global__ void __launch_bounds__(kFusedThreads, kFusedMinBlocks)
-    primal_kernel(Sell<V, I> At, Vecs v) {
+    primal_kernel(Sell<V, I> At, QCsr<V, I> Q, Vecs v) {
+    constexpr bool SPARSE_Q = Q_X != QX::none;
     __shared__ double wpart[SPLIT ? kFusedWarps : 1][32];
     __shared__ unsigned claim;
     extern __shared__ __align__(16) unsigned char dyn_smem[];
@@ -300,8 +304,10 @@ __global__ void __launch_bounds__(kFusedThreads, kFusedMinBlocks)
                           double aj) -> double {
             if (pending)
                 v.xa[j] = aj + (xj - aj) * pw;
-            if constexpr (SPARSE_Q)
+            if constexpr (Q_X == QX::formed)
                 g = g + (qx[j] + qj * xj);
+            if constexpr (Q_X == QX::walked)
+                g = g + (q_walk(Q, j, x) + qj * xj);
             double t = (xj - tau * g) / (1 + tau * (SPARSE_Q ? 0. : qj));
             t = clampd(t, lj, uj);
             xt[j] = t;

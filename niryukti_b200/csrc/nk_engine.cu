@@ -456,15 +456,26 @@ void upload_raw(const nk_csr *H, int vbits, cudaStream_t stream, DevBuf<int64_t>
     cuda_check(cudaStreamSynchronize(stream), "matrix upload");
 }
 
-// The primal kernel instance for a model: sparse Q or not, split rows of A^T
-// or not (each leaves unused paths out of the build).
-template <class V, class I> using PrimalFn = void (*)(Sell<V, I>, Vecs);
-template <class Acc, class V, class I> PrimalFn<V, I> primal_kernel_for(bool sparse_q, bool split) {
+// Rows of a sparse Q with up to this many entries on average are walked by the
+// column's own lane; longer ones are shared by lanes in a launch before the primal
+// kernel.  us a trial, walked / shared: banded Q of 1 M columns, 7 entries a row 84 /
+// 102, 15 109 / 127, 21 134 / 148, 31 177 / 171; 200,000 columns 26 / 30, 32 / 36, 37 /
+// 38, 45 / 46; 4 M entries in rows of hundreds 257 / 108.
+constexpr int64_t kQWalk = 24;
+
+// The primal kernel instance for a model: how it gets a sparse Q's part, and split
+// rows of A^T or not (each leaves unused paths out of the build).
+template <class V, class I> using PrimalFn = void (*)(Sell<V, I>, QCsr<V, I>, Vecs);
+template <class Acc, class V, class I> PrimalFn<V, I> primal_kernel_for(QX qx, bool split) {
     constexpr bool F = sizeof(Acc) == 4;
-    if (sparse_q)
-        return split ? primal_kernel<Acc, V, I, true, F, true>
-                     : primal_kernel<Acc, V, I, true, F, false>;
-    return split ? primal_kernel<Acc, V, I, false, F, true> : primal_kernel<Acc, V, I, false, F, false>;
+    if (qx == QX::walked)
+        return split ? primal_kernel<Acc, V, I, QX::walked, F, true>
+                     : primal_kernel<Acc, V, I, QX::walked, F, false>;
+    if (qx == QX::formed)
+        return split ? primal_kernel<Acc, V, I, QX::formed, F, true>
+                     : primal_kernel<Acc, V, I, QX::formed, F, false>;
+    return split ? primal_kernel<Acc, V, I, QX::none, F, true>
+                 : primal_kernel<Acc, V, I, QX::none, F, false>;
 }
 // The dual kernel instance.  With long rows a lane loads 8 entries ahead where a
 // warp's walk through a split chunk, up to 256 steps, shows in the kernel's time,
@@ -602,10 +613,10 @@ struct Engine {
         auto a = A.fused_view<V, I>();
         if (ev[0])
             mark(0);
-        if (sparse_q)
+        if (qx_form() == QX::formed)
             q_rows(x[0].p, x[1].p, qx[0].p, qx[1].p, ctl.p);
-        primal_kernel_for<Acc, V, I>(sparse_q, At.nsv > 0)<<<grid_p, kFusedThreads, smem_p(),
-                                                              stream>>>(at, v);
+        primal_kernel_for<Acc, V, I>(qx_form(), At.nsv > 0)<<<grid_p, kFusedThreads, smem_p(),
+                                                               stream>>>(at, Q.view<V, I>(), v);
         if (ev[1])
             mark(1);
         if (panels) {
@@ -717,6 +728,10 @@ struct Engine {
         config.attrs = attr;
         config.numAttrs = 2;
         cuda_check(cudaLaunchKernelExC(&config, resident_function(), args), "trial launch");
+    }
+    // how a trial that runs as kernels of its own gets Q x
+    QX qx_form() const {
+        return !sparse_q ? QX::none : Q.lanes > 1 ? QX::formed : QX::walked;
     }
     int vbits() const { return precision == NK_PRECISION_FP64 ? 64 : 32; }
 
@@ -1676,7 +1691,7 @@ void build_panels(PanelMatrix &P, int64_t rows, int64_t cols, const std::vector<
 // grids hold exactly the CTAs that fit on the device at once; their slot
 // memory is sized after the schedules are built (attach_slots).
 template <class Acc, class V, class I> void configure(Engine &E) {
-    const void *pk = (const void *)primal_kernel_for<Acc, V, I>(E.sparse_q, E.At.nsv > 0);
+    const void *pk = (const void *)primal_kernel_for<Acc, V, I>(E.qx_form(), E.At.nsv > 0);
     const void *dk = (const void *)dual_kernel_for<Acc, V, I>(E.A, E.panels);
     // the grids are sized without the slot arrays (they pass 48 KB from about 14.5 M
     // rows on), which the occupancy check after the schedules confirms
@@ -1685,7 +1700,7 @@ template <class Acc, class V, class I> void configure(Engine &E) {
     E.grid_s = occupancy_grid((const void *)spmv_kernel<V, I>, int64_t(1) << 40);
 }
 template <class Acc, class V, class I> void attach_slots(Engine &E) {
-    const void *pk = (const void *)primal_kernel_for<Acc, V, I>(E.sparse_q, E.At.nsv > 0);
+    const void *pk = (const void *)primal_kernel_for<Acc, V, I>(E.qx_form(), E.At.nsv > 0);
     const void *dk = (const void *)dual_kernel_for<Acc, V, I>(E.A, E.panels);
     for (auto [k, bytes, grid] : {std::tuple<const void *, size_t, int>{pk, E.smem_p(), E.grid_p},
                                   {dk, E.smem_d(), E.grid_d}}) {
@@ -2040,7 +2055,7 @@ Engine *create_engine(const nk_csr *Ah, const nk_csr *Qh, const double *hc, cons
             }
         E->Q.nrows = int(qrows.size());
         const int64_t mean = qnnz / std::max(1, E->Q.nrows);
-        while (E->Q.lanes < 32 && 4 * E->Q.lanes < mean)
+        while (E->Q.lanes < 32 && mean > kQWalk && 4 * E->Q.lanes < mean)
             E->Q.lanes *= 2;
         upload_vector(E->Q.rows, qrows, s);
         for (auto &d : E->qx) {
@@ -2483,7 +2498,7 @@ nk_status nk_pdhg_layout_info(nk_pdhg *h, int64_t *long_rows, int64_t *panel_wid
         if (runs)
             *runs = e.panels ? e.pan.slots : 0;
         if (kernels_per_trial)
-            *kernels_per_trial = 2 + (e.sparse_q ? 1 : 0) + (e.panels ? 1 : 0) + (e.halpern ? 1 : 0);
+            *kernels_per_trial = 2 + (e.qx_form() == nk::QX::formed ? 1 : 0) + (e.panels ? 1 : 0) + (e.halpern ? 1 : 0);
     });
 }
 nk_status nk_pdhg_trial_path(nk_pdhg *h, int *resident, int *stage) {

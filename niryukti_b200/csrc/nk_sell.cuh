@@ -118,11 +118,11 @@ __device__ __forceinline__ Acc sell_dot_pipelined(const Sell<V, I> &M, int64_t v
 }
 
 // Sparse symmetric Q in CSR (engine order on both sides), with its rows that
-// have entries.  `lanes` lanes (a power of two, about a quarter of the mean
-// row) share a row: a convex QP's Q = D + L L^T has few rows, of hundreds of
-// entries each, which one lane a row would walk alone.  On a 10,000 x 20,000 QP
-// with 80 k entries in 568 rows of Q that walk was 16 of a trial's 34 us; with
-// its rows shared, inside the resident kernel, a trial takes 8.7 us.
+// have entries.  `lanes` lanes (a power of two, about a quarter of the mean row;
+// 1 up to a mean of 24 entries) share a row: a convex QP's Q = D + L L^T has few rows,
+// of hundreds of entries each, which one lane a row would walk alone.  On a 10,000 x
+// 20,000 QP with 80 k entries in 568 rows of Q that walk was 16 of a trial's 34 us;
+// with its rows shared, inside the resident kernel, a trial takes 9.3 us.
 template <class V, class I> struct QCsr {
     const int64_t *ptr;
     const I *idx;
@@ -130,6 +130,15 @@ template <class V, class I> struct QCsr {
     const int32_t *rows;
     int nrows, lanes;
 };
+
+// Row r of Q times x by one lane, entry by entry (q_row's order with one lane).
+template <class V, class I>
+__device__ __forceinline__ double q_walk(const QCsr<V, I> &Q, int64_t r, const double *x) {
+    double acc = 0;
+    for (int64_t k = Q.ptr[r]; k < Q.ptr[r + 1]; ++k)
+        acc = acc + double(Q.val[k]) * x[Q.idx[k]];
+    return acc;
+}
 
 // The product of x with entry r of Q.rows (none past the list's end `end`), by
 // the calling group of Q.lanes lanes: lane-strided sums, then a fixed shuffle

@@ -828,10 +828,13 @@ def test_slot_limits_of_large_engines_coexist(gpu):
 
 def test_kernels_of_a_trial_are_counted(gpu):
     """The launches of a trial that runs as kernels of its own: the primal and the
-    dual one, Q x of a sparse Q, and Halpern's commit."""
-    m = sparse_qp_model()
+    dual one, Q x of a sparse Q with long rows, and Halpern's commit."""
+    m = synth.random_lp(m=300, n=600, per_col=4, seed=10)
+    m.qptr, m.qidx, m.qval = sparse_q(m.n, "low rank")
+    assert m.qptr[-1] > 24 * np.count_nonzero(np.diff(m.qptr))
     assert gpu.PdhgBackend(m).layout_info()["kernels_per_trial"] == 3
     assert gpu.PdhgBackend(m, halpern=True).layout_info()["kernels_per_trial"] == 4
+    assert gpu.PdhgBackend(sparse_qp_model()).layout_info()["kernels_per_trial"] == 2
     m = synth.random_lp(m=70, n=131, per_col=2, seed=5)
     assert gpu.PdhgBackend(m).layout_info()["kernels_per_trial"] == 2
     assert gpu.PdhgBackend(m, halpern=True).layout_info()["kernels_per_trial"] == 3
@@ -1071,3 +1074,40 @@ def test_propagate_bounds_long_groups(gpu, oracle, lens):
     assert np.sum((want[1] != lb) | (want[2] != ub)) >= n // 3
     for u, w in zip(got[1:], want[1:]):
         assert np.array_equal(u.view(np.int64), w.view(np.int64))
+
+
+@pytest.mark.parametrize("n,band,resident", [(600, 23, True), (600, 25, True), (2001, 2001, True),
+                                             (400_001, 3, False), (400_001, 27, False)])
+def test_sparse_q_paths(gpu, oracle, n, band, resident):
+    """A sparse Q's rows walked in the primal kernel (24 entries or fewer on average) and
+    shared by lanes (more), in models whose trials run in one launch and, with a large A,
+    as kernels of their own: the same bits either way, and the oracle's
+    sequential row sums to rounding (rows of up to 3,001 terms of one size, 7e-13 a
+    trial)."""
+    m = synth.random_lp(m=n // 2, n=n, per_col=5, seed=20)
+    i, half = np.arange(n), band // 2
+    rows = np.repeat(i, 2 * half + 1)
+    cols = (rows + np.tile(np.arange(-half, half + 1), n)) % n
+    vals = np.where(rows == cols, 1.0, -0.5 / band)
+    order = np.lexsort((cols, rows))
+    m.qptr = (2 * half + 1) * np.arange(n + 1, dtype=np.int64)
+    m.qidx, m.qval = cols[order].astype(np.int64), vals[order]
+    tau, sigma = (0.3 * v for v in step_sizes(m))
+    a, b = (gpu.PdhgBackend(m, graphs=True) for _ in range(2))
+    info = a.layout_info()
+    assert info["resident"] == resident, info
+    assert info["kernels_per_trial"] == (2 if band <= 24 else 3), info
+    cpu = oracle.model(m).backend(np.zeros(m.n), np.zeros(m.m))
+    # the step sizes that advance() reduces a QP's own to
+    ptr = np.r_[0, np.cumsum(np.abs(m.val))]
+    norm = math.sqrt(np.max(ptr[m.ptr[1:]] - ptr[m.ptr[:-1]])) * math.sqrt(
+        np.bincount(m.idx, weights=np.abs(m.val), minlength=n).max())
+    scale = min(1.0, 0.9 / (math.sqrt(tau * sigma) * norm + tau * 1.6))
+    assert scale == 1.0
+    for count in (1, 9):
+        a.advance(count, tau, sigma)
+        b.profile_kernels(count, tau, sigma)
+        cpu.advance(count, tau, sigma)
+        for u, w, z in zip(a.candidates(), b.candidates(), cpu.candidates()):
+            assert np.array_equal(u, w)
+            near(u, z)
