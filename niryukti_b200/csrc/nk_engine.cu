@@ -1770,6 +1770,14 @@ void plan_resident(Engine &E, const CtaLists &lists_t, const CtaLists &lists_a,
     if (E.wide || E.precision == NK_PRECISION_FP32 || E.A.ncounters || E.At.ncounters ||
         E.A.nv == 0 || E.At.nv == 0)
         return;
+    // A sparse Q's rows share the resident grid's 16 warps an SM, so its entries weigh
+    // more here than in kernels of their own, and the more the larger A is.  us a
+    // trial, resident / not: A 0.3 M, Q 1.9 M entries 20 / 27, 0.6 M and 1.8 M 19 / 24,
+    // 1.0 M and 0.6 M 27 / 24, 1.0 M and 3.0 M 48 / 32; in rows of hundreds 0.3 M and
+    // 3.8 M 32 / 47, 0.6 M and 1.9 M 30 / 37, 1.0 M and 0.8 M 34 / 33, and 3.2 M 51 / 47.
+    const int64_t room = 1'150'000 - E.A.nnz;
+    if (E.sparse_q && (E.Q.lanes > 1 ? E.Q.nnz : 2 * E.Q.nnz) > 7 * room)
+        return;
     const void *k = E.resident_function();
     int dev = 0, sms = 148, coop = 0, per = 0;
     cuda_check(cudaGetDevice(&dev), "device");

@@ -1077,11 +1077,12 @@ def test_propagate_bounds_long_groups(gpu, oracle, lens):
 
 
 @pytest.mark.parametrize("n,band,resident", [(600, 23, True), (600, 25, True), (2001, 2001, True),
-                                             (400_001, 3, False), (400_001, 27, False)])
+                                             (240_001, 3, False), (240_001, 27, False),
+                                             (3001, 3001, False)])
 def test_sparse_q_paths(gpu, oracle, n, band, resident):
     """A sparse Q's rows walked in the primal kernel (24 entries or fewer on average) and
-    shared by lanes (more), in models whose trials run in one launch and, with a large A,
-    as kernels of their own: the same bits either way, and the oracle's
+    shared by lanes (more), in models whose trials run in one launch and, with a large Q
+    or a large A, as kernels of their own: the same bits either way, and the oracle's
     sequential row sums to rounding (rows of up to 3,001 terms of one size, 7e-13 a
     trial)."""
     m = synth.random_lp(m=n // 2, n=n, per_col=5, seed=20)
