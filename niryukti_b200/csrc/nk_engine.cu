@@ -180,12 +180,40 @@ struct PanelMatrix {
 struct ResidentPlan {
     bool on = false;
     int grid = 0, carveout = 100; // carveout: percent of the SM's shared memory
+    int device = 0, sms = 148;
     unsigned tag = 1;
     size_t smem = 0;
     ResidentView view{};
     DevBuf<int> lists;   // own_t, own_a, slot_t, slot_a, own_q, sync of the view
     DevBuf<double> work; // sum_p, sum_d, word, last_x, last_y
     size_t device_bytes() const { return lists.bytes() + work.bytes(); }
+};
+
+// The trials that advance() calls have in flight on a device, as the CTAs that they
+// take as resident launches (or would).  Such launches run one after the other
+// where together they need more than the SMs, while trials that run as kernels of a
+// few CTAs overlap; so a call runs resident while those in flight fit twice over,
+// and else, where that changes no bit, as kernels.  us an interval of 40 trials per
+// engine with 2, 4 and 8 threads: always resident 323, 296, 282, as kernels 472, 245,
+// 211, by this rule 325, 226, 172 (2,000 x 5,000 LP); 437, 398, 377, then 595, 320,
+// 304, then 430, 345, 242 (30,011 x 60,037).
+struct TrialsInFlight {
+    static constexpr int kDevices = 64;
+    std::atomic<int> &ctas;
+    const int mine;
+    bool resident;
+    explicit TrialsInFlight(const ResidentPlan &P)
+        : ctas(in_flight(P.device)), mine(P.on ? P.grid : 0) {
+        const int others = ctas.fetch_add(mine);
+        resident = P.on && (others == 0 || others + mine <= 2 * P.sms);
+    }
+    ~TrialsInFlight() { ctas.fetch_sub(mine); }
+    TrialsInFlight(const TrialsInFlight &) = delete;
+    TrialsInFlight &operator=(const TrialsInFlight &) = delete;
+    static std::atomic<int> &in_flight(int device) {
+        static std::atomic<int> all[kDevices];
+        return all[size_t(device) % kDevices];
+    }
 };
 
 // Stable order of items by decreasing length (counting sort): result[k] is the
@@ -876,7 +904,9 @@ struct Engine {
         }
         int left = count;
         ctl_known = false;
-        if (resident.on) {
+        const TrialsInFlight flight(resident);
+        // (with panels a resident model's two paths round their long rows differently)
+        if (resident.on && (flight.resident || panels)) {
             run_resident(left);
         } else if (graphs) {
             for (int k = 7; k >= 0 && left > 0; --k)
@@ -1783,6 +1813,8 @@ void plan_resident(Engine &E, const CtaLists &lists_t, const CtaLists &lists_a,
     cuda_check(cudaGetDevice(&dev), "device");
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+    P.device = dev;
+    P.sms = sms;
     R.lists_p = E.grid_p;
     R.lists_d = E.grid_d;
     if (!coop || std::max(R.lists_p, R.lists_d) > kResMaxLists)

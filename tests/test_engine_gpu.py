@@ -1112,3 +1112,56 @@ def test_sparse_q_paths(gpu, oracle, n, band, resident):
         for u, w, z in zip(a.candidates(), b.candidates(), cpu.candidates()):
             assert np.array_equal(u, w)
             near(u, z)
+
+
+@pytest.mark.parametrize("method", ["adaptive", "halpern", "sparse q"])
+def test_resident_and_kernel_trials_alternate(gpu, method):
+    """With several engines in flight a call's trials may run as kernels of their own
+    and the next call's in one launch: an engine that alternates ends, bit for bit,
+    where one that never runs resident does."""
+    m = synth.random_lp(m=900, n=2001, per_col=5, seed=21)
+    if method == "sparse q":
+        m.qptr, m.qidx, m.qval = sparse_q(m.n, "low rank")
+    # the step sizes that advance() would reduce a QP's own to are below its limit
+    tau, sigma = (v * (0.01 if method == "sparse q" else 1) for v in step_sizes(m))
+    options = dict(adaptive=method == "adaptive", halpern=method == "halpern", graphs=True)
+    if method == "halpern":
+        options.update(reflection=0.5, residual_restarts=True)
+    a, b = gpu.PdhgBackend(m, **options), gpu.PdhgBackend(m, **options)
+    assert a.layout_info()["resident"]
+    for k, count in enumerate((3, 7, 30, 2, 1, 40, 5)):
+        (a.profile_kernels if k % 2 else a.advance)(count, tau, sigma)
+        b.profile_kernels(count, tau, sigma)
+        for u, w in zip(a.candidates(), b.candidates()):
+            assert np.array_equal(u, w)
+        if a.restart_requested():
+            for g in (a, b):
+                g.reset_candidate(True)
+    assert a.rejected_steps() == b.rejected_steps()
+
+
+def test_many_engines_in_flight(gpu):
+    """Eight engines from eight threads, more than run resident at once: each ends where
+    it ends alone, bit for bit."""
+    import threading
+    models = [synth.random_lp(m=m, n=2 * m + 1, per_col=4, seed=m) for m in
+              (400, 9000, 2000, 20000, 500, 3000, 12000, 5000)]
+    steps = [step_sizes(m) for m in models]
+
+    def run(k, out):
+        g = gpu.PdhgBackend(models[k], adaptive=k % 2 == 0, halpern=k % 2 == 1, graphs=True)
+        for _ in range(25):
+            g.advance(40, *steps[k])
+        out[k] = g.candidates()
+
+    alone, together = {}, {}
+    for k in range(8):
+        run(k, alone)
+    threads = [threading.Thread(target=run, args=(k, together)) for k in range(8)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for k in range(8):
+        for u, w in zip(alone[k], together[k]):
+            assert np.array_equal(u, w)
