@@ -2098,10 +2098,6 @@ Engine *create_engine(const nk_csr *Ah, const nk_csr *Qh, const double *hc, cons
         while (E->Q.lanes < 32 && mean > kQWalk && 4 * E->Q.lanes < mean)
             E->Q.lanes *= 2;
         upload_vector(E->Q.rows, qrows, s);
-        for (auto &d : E->qx) {
-            d.alloc(size_t(n));
-            cuda_check(cudaMemsetAsync(d.p, 0, d.bytes(), s), "Q product");
-        }
         cuda_check(cudaStreamSynchronize(s), "Q build");
         // norms for the QP step safety (src/cpu.cpp:25-42, src/model.cpp:257-267)
         std::vector<double> cols(static_cast<size_t>(n), 0.0);
@@ -2207,6 +2203,11 @@ Engine *create_engine(const nk_csr *Ah, const nk_csr *Qh, const double *hc, cons
             engine_rlen[size_t(i)] = rlen[size_t(rperm[size_t(i)])];
         plan_resident(*E, lists_t, lists_a, engine_rlen, s);
     }
+    if (E->resident.on ? sparse_q : E->qx_form() == QX::formed)
+        for (auto &d : E->qx) { // (rows without entries stay zero)
+            d.alloc(size_t(n));
+            cuda_check(cudaMemsetAsync(d.p, 0, d.bytes(), s), "Q product");
+        }
     // Column panels cost a launch and a pass over the run sums, about 25 us
     // together, and pay for that from about 4 M entries in the long rows on.  us a
     // trial with and without: 1.2 M of them (power-law, 2 M entries in all) 62 / 41,

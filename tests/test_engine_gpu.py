@@ -1165,3 +1165,16 @@ def test_many_engines_in_flight(gpu):
     for k in range(8):
         for u, w in zip(alone[k], together[k]):
             assert np.array_equal(u, w)
+
+
+def test_walked_sparse_q_memory(gpu):
+    """A sparse Q walked in the primal kernel takes its own storage and nothing else."""
+    m = synth.random_lp(m=20_000, n=40_001, per_col=5, seed=22)
+    lp = gpu.PdhgBackend(m, indices="64").stats()["device_bytes"]
+    i = np.arange(m.n)
+    rows = np.repeat(i, 3)
+    cols = np.sort(np.stack([(i - 1) % m.n, i, (i + 1) % m.n], axis=1), axis=1).reshape(-1)
+    m.qptr, m.qidx = 3 * np.arange(m.n + 1, dtype=np.int64), cols.astype(np.int64)
+    m.qval = np.where(rows == cols, 2.0, -1.0)
+    qp = gpu.PdhgBackend(m, indices="64").stats()["device_bytes"]
+    assert 16 * cols.size < qp - lp <= 16 * cols.size + 8 * (m.n + 1) + 4 * m.n + 4096
