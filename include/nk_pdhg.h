@@ -124,7 +124,9 @@ nk_status nk_pdhg_stats(nk_pdhg *h, int64_t *trials, int64_t *device_bytes);
  * + decision) steps in milliseconds; the dual step includes the panel kernel
  * when A's long rows are stored by column panel.  With graphs on, each trial
  * replays one captured trial whose events are graph nodes, as the graph path
- * runs it.  The trials advance the iterate as nk_pdhg_advance's do, bit for bit. */
+ * runs it.  The trials advance the iterate as nk_pdhg_advance's do, bit for bit.
+ * Where nk_pdhg_advance runs its trials in one launch (nk_pdhg_trial_path), these are
+ * not the kernels that it spends its time in. */
 nk_status nk_pdhg_profile(nk_pdhg *h, int count, double tau, double sigma, double *ms_primal,
                           double *ms_dual);
 /* The same, kernel by kernel: ms[0] the primal kernel, ms[1] the panel kernel

@@ -1787,12 +1787,12 @@ std::vector<int> own_ranges(const std::vector<int32_t> &chunk_len, int parts) {
 
 // Turns the resident kernel on (nk_resident.cuh) for a model that it can run as the
 // kernel path does, bit for bit (with column panels, which only fixed and Halpern
-// steps reach here, up to the rounding of the long rows' sums): 32-bit indices, FP64 sums, no row split across chunks; and
-// that fits: a CTA's products of either matrix and its rows' state in shared
-// memory (up to about 1.5 M entries).  Up to there it is the faster path,
-// measured in us a trial on LPs with 6 entries per column (FP64, adaptive),
-// resident against two kernels: 5.5 / 14.6 at 4 k entries, 6.6 / 16.6 at 54 k,
-// 8.0 / 20.6 at 360 k, 12.6 / 22.6 at 720 k, 18.7 / 26.7 at 1.2 M.
+// steps reach here, up to the rounding of the long rows' sums): 32-bit indices, FP64
+// sums, no row split across chunks; and that fits: a CTA's products of either matrix
+// and its rows' state in shared memory (up to about 1.5 M entries).  Up to there it is
+// the faster path, measured in us a trial on LPs with 6 entries per column (FP64,
+// adaptive), resident against two kernels: 6.1 / 14.6 at 4 k entries, 6.7 / 16.6 at 54
+// k, 8.4 / 20.6 at 360 k, 12.4 / 22.6 at 720 k, 18.3 / 26.7 at 1.2 M.
 void plan_resident(Engine &E, const CtaLists &lists_t, const CtaLists &lists_a,
                    const std::vector<int64_t> &rlen, cudaStream_t s) {
     ResidentPlan &P = E.resident;
@@ -2208,12 +2208,15 @@ Engine *create_engine(const nk_csr *Ah, const nk_csr *Qh, const double *hc, cons
             d.alloc(size_t(n));
             cuda_check(cudaMemsetAsync(d.p, 0, d.bytes(), s), "Q product");
         }
-    // Column panels cost a launch and a pass over the run sums, about 25 us
-    // together, and pay for that from about 4 M entries in the long rows on.  us a
-    // trial with and without: 1.2 M of them (power-law, 2 M entries in all) 62 / 41,
-    // 2.4 M (power-law, 4 M) 75 / 52, 2.4 M (block-angular) 59 / 49, 3 M 63 / 56,
-    // 9 M 81 / 91.  (FP32 sums keep them: their rounding is the panels'.  So do
-    // resident models, whose profiled kernels use them.)
+    // Column panels cost a launch and a pass over the run sums, about 25 us together,
+    // so under fixed and Halpern steps (adaptive ones keep them for their order) long
+    // rows of few entries do without.  us a trial of fixed steps with and without, by
+    // the entries in the long rows: power-law 0.8 M 54 / 36, 1.0 M 62 / 38, 2.0 M 72 /
+    // 50; block-angular 1.8 M 57 / 48, 2.3 M 59 / 50, 3.5 M 65 / 57, 4.7 M 68 / 62, 5.9
+    // M 72 / 69, 8.8 M 81 / 83.  The two meet near 8 M; between the line and there
+    // models keep the panels' sums, which they have always had.  (FP32 sums keep them
+    // at any size: their rounding is the panels'.  So do resident models: at most 24 MB,
+    // for nk_pdhg_profile_kernels, which times the panel kernel.)
     if (E->panels && !panel_order && !E->resident.on && !E->wide &&
         o->precision != NK_PRECISION_FP32 && E->pan.entries < NK_PANEL_MIN_ENTRIES) {
         E->panels = false;

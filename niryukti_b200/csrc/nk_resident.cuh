@@ -27,7 +27,10 @@
 //     trial is rejected.  One reader of the terms, because 147 of them at once
 //     queue up in L2: every CTA deciding for itself took 3.4 us of a 9.1 us trial
 //     of a 30,011 x 60,037 LP.
-// So a trajectory is the same, bit for bit, whichever path runs it.
+// So a trajectory is the same, bit for bit, whichever path runs it -- except with
+// column panels (nk_panel.cuh), whose runs of a long row are added in another order:
+// those models run resident under fixed and Halpern steps only, which don't amplify
+// the rounding.
 //
 // What is left of a trial is mostly the two barriers (1.2 to 1.4 us each), the
 // decision (about 2 us, less what the gathers beside it take) and the gathers,
